@@ -507,50 +507,6 @@ void *compat_workspace(size_t bytes)
     return c.ptr;
 }
 
-// Largest degree of a CSR into *out (zeroed by the caller); grid-stride,
-// warp max, one atomic per warp.
-template <typename OffT>
-__global__ void max_degree_kernel(const OffT *__restrict__ off, long long n,
-                                  unsigned long long *out)
-{
-    unsigned long long best = 0;
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += stride) {
-        const long long d = (long long)off[v + 1] - (long long)off[v];
-        if (d > 0 && (unsigned long long)d > best) best = (unsigned long long)d;
-    }
-    best = cg::reduce(cg::tiled_partition<32>(cg::this_thread_block()), best,
-                      cg::greater<unsigned long long>());
-    if ((threadIdx.x & 31) == 0 && best) atomicMax(out, best);
-}
-
-// Skew above which the compat shims switch a low-mean-degree graph from
-// vertex-id to degree-rank labels: R-MAT scale 20-22 at edge factor 6-8 (skew
-// in the thousands) count 15-25% faster with ranks, while meshes and ER
-// graphs (skew below 4) are faster with ids.
-constexpr long long kCompatSkewRanks = 64;
-
-// The compat shims' launch shape: the mean-degree rule, then -- since these
-// calls synchronise anyway -- one read of the largest degree, and rank labels
-// for a skewed graph.  scratch: 8 bytes of device memory.
-template <typename OffT>
-RowConfig compat_row_config(const OffT *d_off, long long n, long long nnz, void *scratch)
-{
-    RowConfig cfg = pick_row_config(n, nnz);
-    if (cfg.rank_labels || n <= 0 || nnz <= 0) return cfg;
-    unsigned long long *dmax = static_cast<unsigned long long *>(scratch);
-    unsigned long long h = 0;
-    if (cudaMemsetAsync(dmax, 0, sizeof(*dmax), 0) != cudaSuccess) return cfg;
-    const long long want = div_up<long long>(n, 256);
-    max_degree_kernel<OffT><<<(unsigned)(want < 1184 ? want : 1184), 256>>>(d_off, n, dmax);
-    if (cudaMemcpy(&h, dmax, sizeof(h), cudaMemcpyDeviceToHost) != cudaSuccess) return cfg;
-    if ((long long)h * n > kCompatSkewRanks * nnz) {
-        cfg.rank_labels = true;
-        cfg.merge_rows = false;
-    }
-    return cfg;
-}
-
 bool compat_block_size_ok(unsigned int bs)
 {
     switch (bs) {
@@ -617,7 +573,7 @@ gtc_status gtc_count_launches(int64_t n, int64_t nnz, gtc_mode mode,
     const gtc_status st = apply_tuning(cfg, tuning);
     if (st != GTC_OK) return st;
     *launches = launches_per_count(cfg, mode == GTC_MODE_PLAIN, n);
-    *labels = cfg.rank_labels ? GTC_LABELS_DEGREE_RANK : GTC_LABELS_VERTEX_ID;
+    *labels = cfg.split ? GTC_LABELS_DEGREE_RANK : GTC_LABELS_VERTEX_ID;
     return GTC_OK;
 }
 
@@ -632,8 +588,8 @@ gtc_status gtc_count_tuned(const void *d_off, int off_bits, const int32_t *d_ind
     if (!d_off || (nnz > 0 && !d_ind) || !d_workspace) return GTC_ERR_INVALID_ARGUMENT;
     if (mode == GTC_MODE_ORIENTED && (d_r || d_t || d_lcc)) return GTC_ERR_INVALID_ARGUMENT;
     if (reinterpret_cast<uintptr_t>(d_workspace) & 255) return GTC_ERR_INVALID_ARGUMENT;
-    if (ws_bytes < need) return GTC_ERR_WORKSPACE_TOO_SMALL;
     const bool pv = mode == GTC_MODE_PLAIN;
+    if (ws_bytes < make_plan(n, nnz, off_bits, pv).need) return GTC_ERR_WORKSPACE_TOO_SMALL;
     RowConfig cfg = pick_row_config(n, nnz);
     st = apply_tuning(cfg, tuning);
     if (st != GTC_OK) return st;
@@ -663,7 +619,7 @@ gtc_status gtc_count_phase_times(const void *d_off, int off_bits, const int32_t 
     gtc_status st = gtc_workspace_size(n, nnz, off_bits, GTC_MODE_PLAIN, &need);
     if (st != GTC_OK) return st;
     if (!d_off || (nnz > 0 && !d_ind) || !d_workspace || !h_ms) return GTC_ERR_INVALID_ARGUMENT;
-    if (ws_bytes < need) return GTC_ERR_WORKSPACE_TOO_SMALL;
+    if (ws_bytes < make_plan(n, nnz, off_bits, true).need) return GTC_ERR_WORKSPACE_TOO_SMALL;
     RowConfig cfg = pick_row_config(n, nnz);
     st = apply_tuning(cfg, tuning);
     if (st != GTC_OK) return st;
@@ -788,14 +744,13 @@ void gtc_kernelCall_i64(unsigned int numberBlocks, unsigned int numberThreads, i
     if (nnz < 0 || nv > 0x7fffffffll) { g_compat_status = GTC_ERR_INVALID_ARGUMENT; return; }
     size_t need = make_plan(nv, nnz, 64, true).bytes;
     size_t ind_bytes = (((size_t)nnz * sizeof(int)) + 255) & ~(size_t)255;
-    char *ws = static_cast<char *>(compat_workspace(need + ind_bytes + 256));
+    char *ws = static_cast<char *>(compat_workspace(need + ind_bytes));
     if (!ws) { g_compat_status = GTC_ERR_OUT_OF_MEMORY; return; }
     int *ind32 = reinterpret_cast<int *>(ws + need);
     if (nnz > 0)
         narrow_kernel<<<(unsigned)div_up<long long>(nnz, 256), 256>>>(
             reinterpret_cast<const long long *>(d_ind), ind32, nnz, nv);
-    RowConfig cfg = compat_row_config(reinterpret_cast<const long long *>(d_off), nv, nnz,
-                                      ws + need + ind_bytes);
+    const RowConfig cfg = pick_row_config(nv, nnz);
     g_compat_status = run_count<long long>(reinterpret_cast<const long long *>(d_off), ind32, nv,
                                            nnz, true, reinterpret_cast<long long *>(out), nullptr,
                                            nullptr, nullptr, ws, need, 0, cfg, nullptr);
@@ -819,10 +774,10 @@ void gtc_kernelCall_i32(unsigned int numberBlocks, unsigned int numberThreads, i
     if (nnz < 0) { g_compat_status = GTC_ERR_INVALID_ARGUMENT; return; }
     size_t need = make_plan(nv, nnz, 32, true).bytes;
     size_t r_bytes = (((size_t)nv * sizeof(long long)) + 255) & ~(size_t)255;
-    char *ws = static_cast<char *>(compat_workspace(need + r_bytes + 256));
+    char *ws = static_cast<char *>(compat_workspace(need + r_bytes));
     if (!ws) { g_compat_status = GTC_ERR_OUT_OF_MEMORY; return; }
     long long *r64 = reinterpret_cast<long long *>(ws + need);
-    RowConfig cfg = compat_row_config(d_off, nv, nnz, ws + need + r_bytes);
+    const RowConfig cfg = pick_row_config(nv, nnz);
     g_compat_status = run_count<int>(d_off, d_ind, nv, nnz, true, r64, nullptr, nullptr, nullptr,
                                      ws, need, 0, cfg, nullptr);
     if (g_compat_status == GTC_OK) {

@@ -27,15 +27,6 @@ namespace {
 
 constexpr int kChunk = 4096;     // entries (or vertices) per block
 
-// estart[g] = off[vstart[g]] for g in [0, G]
-__global__ void graph_entry_starts(const long long *__restrict__ off,
-                                   const long long *__restrict__ vstart, long long G,
-                                   long long *__restrict__ estart)
-{
-    long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (g <= G) estart[g] = off[vstart[g]];
-}
-
 // Largest g in [0, G) with start[g] <= x (start non-decreasing, start[0] <= x).
 __device__ __forceinline__ long long owner(const long long *__restrict__ start, long long G,
                                            long long x)
@@ -46,78 +37,6 @@ __device__ __forceinline__ long long owner(const long long *__restrict__ start, 
         if (start[mid] <= x) lo = mid; else hi = mid;
     }
     return lo;
-}
-
-// ind_g[e] = ind[e] + vstart[graph of e]; a block covers kChunk entries, each
-// thread four consecutive ones at a time (one 16-byte load and store when
-// both arrays are 16-byte aligned), walking forward from the block's first
-// graph with the current graph's bounds in registers (2.8 TB/s with one
-// entry per thread and the bounds reloaded per entry; 5 ms instead of 9 on
-// the 3.1 G-entry batch).  A local id outside its graph's [0, n_g) becomes
-// -1, which the counting kernels flag (kErrIndexRange) and skip instead of
-// crediting another graph's vertex.
-template <bool VEC>
-__global__ void globalize_kernel(const long long *__restrict__ estart,
-                                 const long long *__restrict__ vstart, long long G,
-                                 const int *__restrict__ ind, int *__restrict__ ind_g,
-                                 long long nnz)
-{
-    __shared__ long long s_g0;
-    const long long e_begin = (long long)blockIdx.x * kChunk;
-    if (threadIdx.x == 0) s_g0 = owner(estart, G, e_begin);
-    __syncthreads();
-    long long g = s_g0;
-    long long g_end = g + 1 < G ? estart[g + 1] : nnz;      // first entry past graph g
-    long long v0 = vstart[g], nv = vstart[g + 1] - v0;
-    const long long e_stop = e_begin + kChunk < nnz ? e_begin + kChunk : nnz;
-    for (long long e4 = e_begin + 4ll * threadIdx.x; e4 < e_stop; e4 += 4ll * blockDim.x) {
-        int x[4];
-        if (VEC && e4 + 4 <= e_stop) {
-            const int4 q = *reinterpret_cast<const int4 *>(ind + e4);
-            x[0] = q.x; x[1] = q.y; x[2] = q.z; x[3] = q.w;
-        } else {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) x[j] = e4 + j < e_stop ? ind[e4 + j] : 0;
-        }
-        int y[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            while (e4 + j >= g_end && g + 1 < G) {
-                ++g;
-                g_end = g + 1 < G ? estart[g + 1] : nnz;
-                v0 = vstart[g];
-                nv = vstart[g + 1] - v0;
-            }
-            y[j] = (x[j] >= 0 && x[j] < nv) ? x[j] + (int)v0 : -1;
-        }
-        if (VEC && e4 + 4 <= e_stop) {
-            *reinterpret_cast<int4 *>(ind_g + e4) = make_int4(y[0], y[1], y[2], y[3]);
-        } else {
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (e4 + j < e_stop) ind_g[e4 + j] = y[j];
-        }
-    }
-}
-
-// graph_T[g] = (sum of t over graph g's vertices) / 3
-__global__ void graph_triangles_kernel(const unsigned long long *__restrict__ tacc,
-                                       const long long *__restrict__ vstart,
-                                       long long *__restrict__ graph_T)
-{
-    const long long g = blockIdx.x;
-    unsigned long long s = 0;
-    for (long long v = vstart[g] + threadIdx.x; v < vstart[g + 1]; v += blockDim.x) s += tacc[v];
-    auto warp = cg::tiled_partition<32>(cg::this_thread_block());
-    s = cg::reduce(warp, s, cg::plus<unsigned long long>());
-    __shared__ unsigned long long ws[32];
-    if (warp.thread_rank() == 0) ws[warp.meta_group_rank()] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned long long t = 0;
-        for (int i = 0; i < (int)(blockDim.x / 32); ++i) t += ws[i];
-        graph_T[g] = (long long)(t / 3);
-    }
 }
 
 struct PackRef {
@@ -161,31 +80,7 @@ __global__ void pack_entries_kernel(const PackRef *__restrict__ refs,
     }
 }
 
-struct BatchPlan {
-    Plan inner;               // the union graph's pipeline workspace
-    size_t o_estart = 0, o_indg = 0, o_inner = 0, o_ghist = 0, o_scan = 0, o_rend = 0,
-           bytes = 0;
-};
-
 inline size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
-
-// The union graph's pipeline workspace comes first, so that the batch
-// workspace starts with its status word (gtc_count_status reads offset 0).
-BatchPlan make_batch_plan(long long G, long long total_n, long long total_nnz)
-{
-    BatchPlan b;
-    b.inner = make_plan(total_n, total_nnz, 64, true);
-    size_t o = 0;
-    b.o_inner = o;  o = align256(o + b.inner.bytes);
-    b.o_estart = o; o = align256(o + sizeof(long long) * (size_t)(G + 1));
-    b.o_indg = o;   o = align256(o + sizeof(int) * (size_t)(total_nnz + 1));
-    // graph-major degree ranks: per-graph bucket histogram and its scan
-    b.o_ghist = o;  o = align256(o + sizeof(long long) * (size_t)(G * kSegBuckets + 1));
-    b.o_scan = o;   o = align256(o + scan_tmp_bytes(G * kSegBuckets));
-    b.o_rend = o;   o = align256(o + sizeof(int) * (size_t)(total_n + 1));
-    b.bytes = o;
-    return b;
-}
 
 }  // namespace
 }  // namespace gtc
@@ -199,7 +94,7 @@ gtc_status gtc_batch_workspace_size(int64_t num_graphs, int64_t total_n, int64_t
 {
     if (!bytes || num_graphs < 0 || total_n < 0 || total_nnz < 0) return GTC_ERR_INVALID_ARGUMENT;
     if (total_n > 0x7fffffffll) return GTC_ERR_UNSUPPORTED;      // union ids are int32
-    *bytes = make_batch_plan(num_graphs, total_n, total_nnz).bytes;
+    *bytes = make_plan(total_n, total_nnz, 64, true, num_graphs).bytes;
     return GTC_OK;
 }
 
@@ -216,55 +111,20 @@ gtc_status gtc_count_batch(int64_t num_graphs, const int64_t *d_vstart, const in
     if (!d_vstart || !d_off || (total_nnz > 0 && !d_ind) || !d_workspace)
         return GTC_ERR_INVALID_ARGUMENT;
     if (reinterpret_cast<uintptr_t>(d_workspace) & 255) return GTC_ERR_INVALID_ARGUMENT;
-    if (ws_bytes < need) return GTC_ERR_WORKSPACE_TOO_SMALL;
-    const BatchPlan b = make_batch_plan(num_graphs, total_n, total_nnz);
-    char *base = static_cast<char *>(d_workspace);
-    long long *estart = reinterpret_cast<long long *>(base + b.o_estart);
-    int *ind_g = reinterpret_cast<int *>(base + b.o_indg);
-    void *inner = base + b.o_inner;
-    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    const long long *vstart = reinterpret_cast<const long long *>(d_vstart);
-    const long long *off = reinterpret_cast<const long long *>(d_off);
-
+    if (ws_bytes < make_plan(total_n, total_nnz, 64, true, num_graphs).need)
+        return GTC_ERR_WORKSPACE_TOO_SMALL;
     RowConfig cfg = pick_row_config(total_n, total_nnz);
-    // a batch mixes degree profiles: the warp-per-item kernel unless asked
-    // (per-row merges were 24% slower on the 4,096-graph mix)
-    cfg.merge_rows = false;
     st = apply_tuning(cfg, tuning);
     if (st != GTC_OK) return st;
-
-    graph_entry_starts<<<(unsigned)div_up<long long>(num_graphs + 1, 256), 256, 0, s>>>(
-        off, vstart, num_graphs, estart);
-    if (total_nnz > 0)
-    {
-        const unsigned gb = (unsigned)div_up<long long>(total_nnz, kChunk);
-        if ((reinterpret_cast<uintptr_t>(d_ind) & 15) == 0 &&
-            (reinterpret_cast<uintptr_t>(ind_g) & 15) == 0)
-            globalize_kernel<true><<<gb, 256, 0, s>>>(estart, vstart, num_graphs, d_ind, ind_g,
-                                                      total_nnz);
-        else
-            globalize_kernel<false><<<gb, 256, 0, s>>>(estart, vstart, num_graphs, d_ind, ind_g,
-                                                       total_nnz);
-    }
-    if (cudaGetLastError() != cudaSuccess) return GTC_ERR_CUDA;
-    SegRanks seg;
-    seg.vstart = vstart;
-    seg.num_graphs = num_graphs;
-    seg.ghist = reinterpret_cast<long long *>(base + b.o_ghist);
-    seg.scan_tmp = base + b.o_scan;
-    seg.rank_end = reinterpret_cast<int *>(base + b.o_rend);
-    st = run_count<long long>(off, ind_g, total_n, total_nnz, true,
-                              reinterpret_cast<long long *>(d_r),
-                              reinterpret_cast<long long *>(d_t), d_lcc, nullptr, inner,
-                              b.inner.bytes, s, cfg, nullptr, &seg);
-    if (st != GTC_OK) return st;
-    if (d_graph_T) {
-        const unsigned long long *tacc =
-            reinterpret_cast<const unsigned long long *>(static_cast<char *>(inner) + b.inner.o_tacc);
-        graph_triangles_kernel<<<(unsigned)num_graphs, 256, 0, s>>>(
-            tacc, vstart, reinterpret_cast<long long *>(d_graph_T));
-    }
-    return cudaGetLastError() == cudaSuccess ? GTC_OK : GTC_ERR_CUDA;
+    Batch batch;
+    batch.vstart = reinterpret_cast<const long long *>(d_vstart);
+    batch.num_graphs = num_graphs;
+    batch.graph_T = reinterpret_cast<long long *>(d_graph_T);
+    return run_count<long long>(reinterpret_cast<const long long *>(d_off), d_ind, total_n,
+                                total_nnz, true, reinterpret_cast<long long *>(d_r),
+                                reinterpret_cast<long long *>(d_t), d_lcc, nullptr, d_workspace,
+                                ws_bytes, reinterpret_cast<cudaStream_t>(stream), cfg, nullptr,
+                                &batch);
 }
 
 size_t gtc_batch_pack_scratch_bytes(int64_t num_graphs)

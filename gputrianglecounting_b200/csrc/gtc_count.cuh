@@ -1,0 +1,1156 @@
+// gtc_count.cuh -- kernels that find the triangles: pairs of core members in
+// the bit matrix, forward lists of the other members in hash tables; and the
+// epilogue.
+#pragma once
+
+#include <type_traits>
+
+#include "gtc_build.cuh"
+
+namespace gtc {
+
+__device__ __forceinline__ void add64(unsigned long long *p, unsigned int x)
+{
+    atomicAdd(p, (unsigned long long)x);
+}
+
+__device__ __forceinline__ unsigned int warp_sum(unsigned int x)
+{
+    return __reduce_add_sync(0xffffffffu, x);
+}
+
+// 32 x 32 bit transpose: bit c of lane r's result is bit r of lane c's x.  At
+// distance k the lanes swap the halves of every 2k-bit field; a rotation by k
+// (back for the upper lanes) aligns the partner's bits.
+__device__ __forceinline__ unsigned int transpose32(unsigned int x, int lane)
+{
+    unsigned int y = __shfl_xor_sync(0xffffffffu, x, 16);
+    x = __byte_perm(x, y, lane & 16 ? 0x3276 : 0x5410);
+    y = __shfl_xor_sync(0xffffffffu, x, 8);
+    x = __byte_perm(x, y, lane & 8 ? 0x3715 : 0x6240);
+#pragma unroll
+    for (int k = 4; k >= 1; k >>= 1) {
+        const unsigned int low = k == 4 ? 0x0f0f0f0fu : (k == 2 ? 0x33333333u : 0x55555555u);
+        const unsigned int keep = lane & k ? ~low : low;
+        y = __shfl_xor_sync(0xffffffffu, x, k);
+        y = __funnelshift_l(y, y, lane & k ? 32 - k : k);
+        x = (x & keep) | (y & ~keep);
+    }
+    return x;
+}
+
+// Credit of a list element: vertices in tacc, core positions in tcore.
+__device__ __forceinline__ void credit(const Data &w, long long v0, int m, unsigned int c)
+{
+    add64(m >= 0 ? &w.tacc[m] : &w.tcore[v0 + ~m], c);
+}
+
+// ============================================== pairs of core members (bits)
+
+// base[i], the address in one multiply-add: the integer pipe that adds and
+// shifts is the busy one here, and a multiplier `word` (4) that the compiler
+// cannot see keeps the address off it.
+__device__ __forceinline__ unsigned int load_word(const unsigned int *base, int i, int word)
+{
+    unsigned long long p;
+    asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(p) : "r"(i), "r"(word), "l"(base));
+    return __ldg(reinterpret_cast<const unsigned int *>(p));
+}
+
+// A core member s as a lane sees it: its word in row 0, and the factor that
+// moves its bit to the top.
+struct CoreBit {
+    const unsigned int *up;
+    unsigned int mul;
+};
+
+__device__ __forceinline__ CoreBit core_bit(const unsigned int *U, int pos)
+{
+    return {U + (pos >> 5), 0x80000000u >> (pos & 31)};
+}
+
+// Bit k of the result: whether s is in core row k of qb[0 .. nq) (word
+// offsets; entries up to the next multiple of 16 must be readable).  Per row
+// an address, a load, a multiplication that brings the bit to the top, a shift
+// that takes it in and a quarter of a shared load; 16 loads in flight.
+__device__ __forceinline__ unsigned int row_bits(const CoreBit &s, const int *qb, int nq, int word)
+{
+    unsigned int hb = 0;
+    int i = 0;
+    for (; i < nq; i += 16) {
+        unsigned int x[16];
+#pragma unroll
+        for (int j = 0; j < 16; j += 4) {
+            const int4 a = *reinterpret_cast<const int4 *>(qb + i + j);
+            x[j] = load_word(s.up, a.x, word);
+            x[j + 1] = load_word(s.up, a.y, word);
+            x[j + 2] = load_word(s.up, a.z, word);
+            x[j + 3] = load_word(s.up, a.w, word);
+        }
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            unsigned int t;
+            asm("mul.lo.u32 %0, %1, %2;" : "=r"(t) : "r"(x[j]), "r"(s.mul));
+            hb = __funnelshift_l(t, hb, 1);
+        }
+    }
+    hb = __brev(hb) >> (32 - i);                  // i >= 16; row k at bit k
+    return nq < 32 ? hb & ((1u << nq) - 1u) : hb;
+}
+
+// Ascending sort of 32 E integers by a warp in registers (bitonic network):
+// lane l ends with elements l E .. l E + E - 1.
+template <int E>
+__device__ __forceinline__ void warp_sort(int (&v)[E], int lane)
+{
+#pragma unroll
+    for (int k = 2; k <= 32 * E; k <<= 1) {
+#pragma unroll
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            if (j >= E) {
+                const bool lower = (lane & (j / E)) == 0;
+#pragma unroll
+                for (int e = 0; e < E; ++e) {
+                    const bool asc = k >= E ? (lane & (k / E)) == 0 : (e & k) == 0;
+                    const int y = __shfl_xor_sync(0xffffffffu, v[e], j / E);
+                    v[e] = lower == asc ? min(v[e], y) : max(v[e], y);
+                }
+            } else {
+#pragma unroll
+                for (int e = 0; e < E; ++e) {
+                    if ((e & j) == 0) {
+                        const bool asc = k >= E ? (lane & (k / E)) == 0 : (e & k) == 0;
+                        const int a = v[e], b = v[e + j];
+                        v[e] = asc ? min(a, b) : max(a, b);
+                        v[e + j] = asc ? max(a, b) : min(a, b);
+                    }
+                }
+            }
+        }
+    }
+}
+
+// Longest list of a wide row that a warp takes: bit matrix, tables.
+constexpr int kWarpList = 256, kWarpTable = 128;
+constexpr int kWideRows = 16;                     // wide rows a block claims at a time
+
+// A block's claim of kWideRows rows of the wide list, parted by list length.
+struct WideClaim {
+    int row[2][kWideRows];                        // [0] a warp each, [1] the block together
+    int count[2];
+    int next;
+    long long item;
+};
+
+// Claim the next wide rows that `want` (of the row's record); false when the
+// list is used up.  A block's first claim is its own share, the next ones come
+// from a queue.  A claim's rows are spread over the list, whose neighbours
+// tend to be alike (generators give hubs the lowest ids).
+template <class Want>
+__device__ __forceinline__ bool claim_rows(const Data &w, WideClaim &cl, unsigned long long *queue,
+                                           long long rows, int most, bool first, const Want &want)
+{
+    const long long claims = div_up<long long>(rows, kWideRows);
+    if (!first && gridDim.x >= claims) return false;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        long long item = blockIdx.x;
+        if (!first) {
+            if (threadIdx.x == 0) item = gridDim.x + (long long)atomicAdd(queue, 1ull);
+            item = __shfl_sync(0xffffffffu, item, 0);
+        }
+        const long long at = item < claims && threadIdx.x < kWideRows
+                                 ? item + claims * threadIdx.x : rows;
+        int v = 0;
+        VInfo vi{0, 0, 0};
+        if (at < rows) {
+            v = w.wide[at];
+            vi = w.vinfo[v];
+        }
+        const bool in = at < rows && want(vi);
+        const unsigned int below = (1u << threadIdx.x) - 1u;
+        const unsigned int m0 = __ballot_sync(0xffffffffu, in && vi.fdeg <= most);
+        const unsigned int m1 = __ballot_sync(0xffffffffu, in && vi.fdeg > most);
+        if (in) {
+            if (vi.fdeg <= most) cl.row[0][__popc(m0 & below)] = v;
+            else cl.row[1][__popc(m1 & below)] = v;
+        }
+        if (threadIdx.x == 0) {
+            cl.count[0] = __popc(m0);
+            cl.count[1] = __popc(m1);
+            cl.next = 0;
+            cl.item = item;
+        }
+    }
+    __syncthreads();
+    return cl.item < claims;
+}
+
+// The claimed rows that take a warp each, in turn.
+template <class Row>
+__device__ __forceinline__ void claimed_by_warps(WideClaim &cl, const Row &row)
+{
+    while (true) {
+        int k = 0;
+        if ((threadIdx.x & 31) == 0) k = atomicAdd(&cl.next, 1);
+        k = __shfl_sync(0xffffffffu, k, 0);
+        if (k >= cl.count[0]) break;
+        row(cl.row[0][k]);
+    }
+}
+
+struct CoreWarpSmem {
+    int qb[kWarpList];                            // word offset of each member's core row
+    unsigned int cnt[kWarpList];
+    unsigned short pos[kWarpList];
+};
+
+struct CoreBlockSmem {
+    unsigned int bits[kCoreMax / 32];             // the row's core members
+    unsigned short below[kCoreMax / 32];          // members in earlier words
+    int spos[kMemberChunk], qpos[kMemberChunk];   // positions of the s and q members
+    int qb[kMemberChunk];                         // word offset of each q member's row
+    unsigned int scnt[kMemberChunk], qcnt[kMemberChunk];
+    unsigned int wsum[kThreads / 32];
+    unsigned int total;
+};
+
+struct CoreSmem {
+    union {
+        CoreWarpSmem warp[kThreads / 32];
+        CoreBlockSmem block;
+    };
+    WideClaim claim;
+};
+
+// Where a row's core lives.
+struct CoreView {
+    const unsigned int *U;
+    unsigned long long *tcore;
+    unsigned long long *own;      // the row's own credits
+};
+
+template <bool PV, bool BATCH>
+__device__ __forceinline__ CoreView core_view(const Data &w, int v)
+{
+    const GraphRec *rec = &w.recs[BATCH ? w.gid[v] : 0];
+    CoreView c{w.u, w.tcore, nullptr};
+    if (BATCH) {
+        c.U += rec->ubase;
+        c.tcore += rec->v0;
+    }
+    if (PV) {
+        const int kv = w.key[v];
+        c.own = kv > kKeyTop - rec->core ? &c.tcore[kKeyTop - kv] : &w.tacc[v];
+    }
+    return c;
+}
+
+// Pairs (q, s) of core members of one row, q -> s a bit of U: with the members
+// in ascending position (descending order) s has the lower index, so the pairs
+// are a lower triangle of index pairs, in tiles of 32 q by 32 s.  A lane holds
+// a member s and loads its word of 32 rows q.  A tile's hits are a 32 x 32 bit
+// matrix: rows count s, columns (transposed) count q.
+
+// A row of at most kWarpList members (32 E) by a warp, sorted in registers.
+template <int E, bool PV>
+__device__ __forceinline__ void core_warp_row(const Data &w, const VInfo &vi, const CoreView &cv,
+                                              CoreWarpSmem &sm, unsigned long long &tri)
+{
+    const int lane = threadIdx.x & 31;
+    int p[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const int k = e * 32 + lane;
+        const int m = k < vi.fdeg ? w.find[vi.fbeg + k] : 0;
+        p[e] = m < 0 ? ~m : INT32_MAX;
+    }
+    warp_sort<E>(p, lane);
+    const int n = vi.dk & INT32_MAX;
+    __syncwarp();
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const int k = lane * E + e;
+        sm.pos[k] = (unsigned short)p[e];
+        sm.qb[k] = k < n ? u_row(p[e]) : 0;
+        if (PV) sm.cnt[k] = 0;
+    }
+    __syncwarp();
+    unsigned int tot = 0;
+    const int groups = (n + 31) >> 5;
+    for (int ts = 0; ts < groups; ++ts) {
+        const int si = ts * 32 + lane;
+        const CoreBit s = core_bit(cv.U, si < n ? sm.pos[si] : 0);
+        // s is above q only at lower indices
+        unsigned int keep = si < n && lane < 31 ? 0xffffffffu << (lane + 1) : 0u, v = 0;
+        for (int tq = ts; tq < groups; ++tq) {
+            const unsigned int hb = keep & row_bits(s, sm.qb + tq * 32, min(32, n - tq * 32),
+                                                    w.word);
+            keep = 0xffffffffu;
+            v += __popc(hb);
+            // an index modulo 32 belongs to one lane
+            if (PV) sm.cnt[tq * 32 + lane] += __popc(transpose32(hb, lane));
+        }
+        tot += v;
+        if (PV) sm.cnt[si] += v;
+    }
+    tot = warp_sum(tot);
+    if (tot) {
+        if (PV) {
+            for (int k = lane; k < n; k += 32)
+                if (sm.cnt[k]) add64(&cv.tcore[sm.pos[k]], sm.cnt[k]);
+            if (lane == 0) add64(cv.own, tot);
+        }
+        tri += lane == 0 ? tot : 0u;
+    }
+}
+
+// A longer row by the block: a bitmap of the members over the core positions
+// and the members below each of its words give every member its index; rows
+// of more than kMemberChunk members go chunk by chunk.
+template <bool PV>
+__device__ void core_block_row(const Data &w, const VInfo &vi, int core, const CoreView &cv,
+                               CoreBlockSmem &sm, unsigned long long &tri)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int words = (core + 31) >> 5;
+    constexpr int kPer = kCoreMax / 32 / kThreads;
+    __syncthreads();
+    for (int k = threadIdx.x; k < kThreads * kPer; k += kThreads) sm.bits[k] = 0;
+    if (threadIdx.x == 0) sm.total = 0;
+    __syncthreads();
+    for (int k = threadIdx.x; k < vi.fdeg; k += kThreads) {
+        const int m = w.find[vi.fbeg + k];
+        if (m < 0) atomicOr(&sm.bits[~m >> 5], 1u << (~m & 31));
+    }
+    __syncthreads();
+    const int w0 = threadIdx.x * kPer;
+    int cnt[kPer], sum = 0;
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+        cnt[j] = __popc(sm.bits[w0 + j]);
+        sum += cnt[j];
+    }
+    int incl = sum;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int o = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += o;
+    }
+    if (lane == 31) sm.wsum[warp] = (unsigned int)incl;
+    __syncthreads();
+    int first = incl - sum, total = 0;
+    for (int i = 0; i < kThreads / 32; ++i) {
+        if (i < warp) first += (int)sm.wsum[i];
+        total += (int)sm.wsum[i];
+    }
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+        if (w0 + j < words) sm.below[w0 + j] = (unsigned short)first;
+        first += cnt[j];
+    }
+    __syncthreads();
+    auto fill = [&](int base, int *pos, int *qb) {
+        for (int k = threadIdx.x; k < vi.fdeg; k += kThreads) {
+            const int m = w.find[vi.fbeg + k];
+            if (m >= 0) continue;
+            const int x = ~m;
+            const int at = sm.below[x >> 5] +
+                           __popc(sm.bits[x >> 5] & ((1u << (x & 31)) - 1u)) - base;
+            if (at >= 0 && at < kMemberChunk) {
+                pos[at] = x;
+                if (qb) qb[at] = u_row(x);
+            }
+        }
+        if (qb)
+            for (int k = total - base + (int)threadIdx.x;
+                 k < kMemberChunk && k < total - base + 16; k += kThreads)
+                qb[k] = 0;
+    };
+    unsigned int mine = 0;
+    const bool one = total <= kMemberChunk;
+    for (int sb = 0; sb < total; sb += kMemberChunk) {
+        const int ns = min(total - sb, kMemberChunk), sg = (ns + 31) >> 5;
+        fill(sb, sm.spos, one ? sm.qb : nullptr);
+        if (PV)
+            for (int k = threadIdx.x; k < ns; k += kThreads) sm.scnt[k] = 0;
+        for (int qs = sb; qs < total; qs += kMemberChunk) {
+            const int nq = min(total - qs, kMemberChunk), qg = (nq + 31) >> 5;
+            if (!one) fill(qs, sm.qpos, sm.qb);
+            if (PV)
+                for (int k = threadIdx.x; k < nq; k += kThreads) sm.qcnt[k] = 0;
+            __syncthreads();
+            const bool diag = qs == sb;
+            // tiles, the q groups of an s group in turn, parted evenly among
+            // the warps
+            const int tiles = diag ? qg * (qg + 1) / 2 : qg * sg;
+            const int t1 = tiles * (warp + 1) / (kThreads / 32);
+            int t = tiles * warp / (kThreads / 32), ts, tq;
+            if (diag) {                           // from the last tile, a triangle row by row
+                const int r = tiles - 1 - t;
+                int a = (int)((sqrtf(8.0f * (float)r + 1.0f) - 1.0f) * 0.5f);
+                while (a * (a + 1) / 2 > r) --a;
+                while ((a + 1) * (a + 2) / 2 <= r) ++a;
+                ts = qg - 1 - a;
+                tq = qg - 1 - (r - a * (a + 1) / 2);
+            } else {
+                ts = t / qg;
+                tq = t - ts * qg;
+            }
+            while (t < t1) {
+                const int si = ts * 32 + lane;
+                const CoreBit s = core_bit(cv.U, si < ns ? sm.spos[si] : 0);
+                unsigned int v = 0;
+                for (; tq < qg && t < t1; ++tq, ++t) {
+                    unsigned int hb = row_bits(s, sm.qb + tq * 32, min(32, nq - tq * 32), w.word);
+                    if (diag && tq == ts) hb &= lane < 31 ? 0xffffffffu << (lane + 1) : 0u;
+                    if (si >= ns) hb = 0;
+                    v += __popc(hb);
+                    if (PV) {
+                        const unsigned int c = __popc(transpose32(hb, lane));
+                        if (c) atomicAdd(&sm.qcnt[tq * 32 + lane], c);
+                    }
+                }
+                if (PV) {
+                    if (v) atomicAdd(&sm.scnt[si], v);
+                } else {
+                    mine += v;
+                }
+                ++ts;
+                tq = diag ? ts : 0;
+            }
+            __syncthreads();
+            if (PV) {
+                const int *pos = one ? sm.spos : sm.qpos;
+                for (int k = threadIdx.x; k < nq; k += kThreads) {
+                    const unsigned int c = sm.qcnt[k];
+                    mine += c;
+                    const unsigned int both = one ? c + sm.scnt[k] : c;
+                    if (both) add64(&cv.tcore[pos[k]], both);
+                }
+                __syncthreads();
+            }
+        }
+        if (PV && !one) {
+            for (int k = threadIdx.x; k < ns; k += kThreads)
+                if (sm.scnt[k]) add64(&cv.tcore[sm.spos[k]], sm.scnt[k]);
+            __syncthreads();
+        }
+    }
+    const unsigned int ws = warp_sum(mine);
+    if (lane == 0 && ws) atomicAdd(&sm.total, ws);
+    __syncthreads();
+    if (threadIdx.x == 0 && sm.total) {
+        if (PV) add64(cv.own, sm.total);
+        tri += sm.total;
+    }
+}
+
+template <bool PV, bool BATCH>
+__device__ __forceinline__ void core_wide_rows(const Data &w, CoreSmem &sm,
+                                               unsigned long long &tri)
+{
+    const long long rows = (long long)w.ctr->wide_rows;
+    for (bool first = true;
+         claim_rows(w, sm.claim, &w.ctr->core_wide_next, rows, kWarpList, first,
+                    [](const VInfo &vi) { return (vi.dk & INT32_MAX) >= 2; });
+         first = false) {
+        for (int k = 0; k < sm.claim.count[1]; ++k) {
+            const int v = sm.claim.row[1][k];
+            core_block_row<PV>(w, w.vinfo[v], w.recs[BATCH ? w.gid[v] : 0].core,
+                               core_view<PV, BATCH>(w, v), sm.block, tri);
+        }
+        __syncthreads();
+        claimed_by_warps(sm.claim, [&](int v) {
+            const VInfo vi = w.vinfo[v];
+            const CoreView cv = core_view<PV, BATCH>(w, v);
+            CoreWarpSmem &ws = sm.warp[threadIdx.x >> 5];
+            if (vi.fdeg <= 32) core_warp_row<1, PV>(w, vi, cv, ws, tri);
+            else if (vi.fdeg <= 64) core_warp_row<2, PV>(w, vi, cv, ws, tri);
+            else if (vi.fdeg <= 128) core_warp_row<4, PV>(w, vi, cv, ws, tri);
+            else core_warp_row<8, PV>(w, vi, cv, ws, tri);
+        });
+    }
+}
+
+// Up to 32 consecutive rows by a warp, one after another: a lane per member of
+// the row (at most kShortList), every core member q in turn broadcast to the
+// members above it.
+template <bool PV, bool BATCH>
+__device__ __forceinline__ void core_short_rows(const Data &w, long long u0, int batch,
+                                                unsigned long long &tri)
+{
+    const int lane = threadIdx.x & 31;
+    VInfo vi{0, 0, 0};
+    int g = 0;
+    if (lane < batch && u0 + lane < w.n) {
+        vi = w.vinfo[u0 + lane];
+        if (BATCH) g = w.gid[u0 + lane];
+    }
+    unsigned int rows = __ballot_sync(0xffffffffu, vi.dk >= 2);   // not a wide row
+    while (rows) {
+        const int r = __ffs(rows) - 1;
+        rows &= rows - 1;
+        const long long fb = __shfl_sync(0xffffffffu, vi.fbeg, r);
+        const int fd = __shfl_sync(0xffffffffu, vi.fdeg, r);
+        const int m = lane < fd ? w.find[fb + lane] : 0;
+        const bool core = m < 0;
+        const int pos = ~m;
+        const int rb = core ? u_row(pos) : INT32_MAX;   // ascending with the position
+        const unsigned int *up = w.u + (core ? pos >> 5 : 0);
+        long long v0 = 0;
+        if (BATCH) {
+            const GraphRec *rec = &w.recs[__shfl_sync(0xffffffffu, g, r)];
+            up += rec->ubase;
+            v0 = rec->v0;
+        }
+        unsigned int qm = __ballot_sync(0xffffffffu, core);
+        unsigned int cq = 0, cs = 0;
+        while (qm) {
+            int q[4];
+            unsigned int x[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                q[j] = qm ? __ffs(qm) - 1 : -1;
+                qm &= qm - 1;
+                const int rq = __shfl_sync(0xffffffffu, rb, q[j] & 31);
+                x[j] = (q[j] >= 0 && rb < rq) ? __ldg(up + rq) : 0u;
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const bool hit = (x[j] >> (pos & 31)) & 1u;
+                const unsigned int h = __ballot_sync(0xffffffffu, hit);
+                cs += hit;
+                if (lane == q[j]) cq += __popc(h);
+            }
+        }
+        const unsigned int tot = warp_sum(cq);
+        if (tot) {
+            if (PV) {
+                if (core && cq + cs) add64(&w.tcore[v0 + pos], cq + cs);
+                if (lane == 0) add64(&w.tacc[u0 + r], tot);
+            }
+            tri += lane == 0 ? tot : 0u;
+        }
+    }
+}
+
+// ====================================================== other members (lists)
+
+constexpr int kNoProbe = INT32_MIN + 1;           // never a list element nor kNoMember
+
+__device__ __forceinline__ int warp_incl_scan(int v)
+{
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int o = __shfl_up_sync(0xffffffffu, v, d);
+        if (lane >= d) v += o;
+    }
+    return v;
+}
+
+// The lane i whose [incl_i - count_i, incl_i) holds f (incl: this lane's
+// inclusive prefix of a per-lane count).
+__device__ __forceinline__ int warp_corank(int incl, int f)
+{
+    int i = 0;
+#pragma unroll
+    for (int step = 16; step >= 1; step >>= 1) {
+        const int v = __shfl_sync(0xffffffffu, incl, i + step - 1);
+        if (v <= f) i += step;
+    }
+    return i;
+}
+
+// A tile: consecutive short rows with at most kTileEdges members in all, of
+// which at most kTileIds are distinct.
+constexpr int kTileEdges = 192, kTileIds = 96, kTileWords = kTileIds / 32;
+constexpr int kTileSlots = 1024;
+constexpr int kTileLong = 32;                     // longer lists are taken by the whole warp
+constexpr unsigned short kNoEdge = 0xffff;
+
+struct __align__(16) TileSmem {
+    unsigned short slot[kTileSlots];              // first edge whose member hashes here
+    unsigned int adj[kTileWords][kTileIds];       // adjacency among the tile's distinct members
+    unsigned int rowbits[kTileWords][32];         // a row's members
+    unsigned int credit[kTileIds];
+    int member[kTileEdges];                       // an edge's member
+    unsigned short hash[kTileEdges];              // ... its slot
+    unsigned char row[kTileEdges];                // ... its row
+    unsigned char num[kTileEdges];                // ... its member's number
+    unsigned char first[kTileIds];                // first edge of a number
+};
+
+// Empties a warp's table; every tile leaves it empty again.
+__device__ __forceinline__ void tile_init(TileSmem &sm)
+{
+    for (int k = threadIdx.x & 31; k < kTileSlots / 2; k += 32)
+        reinterpret_cast<unsigned int *>(sm.slot)[k] = 0xffffffffu;
+    __syncwarp();
+}
+
+// Short rows, a tile at a time by a warp.  The members of all rows of the
+// tile are numbered through a shared hash table (rows near each other share
+// members: on a geometric graph a tile's 160 edges have some 75), every
+// distinct member's forward list is looked up once, and what is found sets
+// the bits of the symmetric adjacency among the numbers.  Then an edge p -> q
+// closes popc(members of p & neighbours of q) triangles: those in which q is
+// the middle and those in which it is the highest vertex, so that is q's
+// credit, and half a row's sum is p's.  The pairs of core members are not
+// among them (their lists are not looked up).  The table is a tenth full, so
+// a look-up that finds nothing mostly ends at its first slot.
+template <bool PV, bool BATCH, typename Pos>
+__device__ __forceinline__ void
+tile_rows(const Data &w, long long u0, const VInfo &vi, int g, bool act, TileSmem &sm,
+          unsigned long long &tri)
+{
+    const int lane = threadIdx.x & 31;
+    const unsigned int below = (1u << lane) - 1u;
+    constexpr unsigned int kMask = kTileSlots - 1;
+    constexpr int kLog = ilog2(kTileSlots);
+    const int fd = act ? vi.fdeg : 0;
+    const int incl = warp_incl_scan(fd);
+    const int total = __shfl_sync(0xffffffffu, incl, 31);
+    const Pos start = (Pos)vi.fbeg - (Pos)(incl - fd);
+    for (int base = 0; base < total;) {
+        // rows that may join: one graph (core members are positions in it)
+        int stop = total;
+        long long v0 = 0;
+        if (BATCH) {
+            const int f0 = __ffs(__ballot_sync(0xffffffffu, incl > base)) - 1;
+            const int gf = __shfl_sync(0xffffffffu, g, f0);
+            const unsigned int other = __ballot_sync(0xffffffffu, fd > 0 && lane > f0 && g != gf);
+            const int o = other ? __ffs(other) - 1 : 0;
+            const int excl = __shfl_sync(0xffffffffu, incl - fd, o);
+            if (other) stop = excl;
+            v0 = w.recs[gf].v0;
+        }
+        stop = min(stop - base, kTileEdges);
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < kTileWords; ++k) {
+#pragma unroll
+            for (int j = 0; j < kTileIds / 32; ++j) sm.adj[k][j * 32 + lane] = 0;
+            sm.rowbits[k][lane] = 0;
+            if (PV) sm.credit[k * 32 + lane] = 0;
+        }
+        // number the members, 32 edges at a time while there is room
+        int n = 0, seen = 0;
+        for (; seen < stop && n <= kTileIds - 32; seen += 32) {
+            const int e = seen + lane;
+            const int i = warp_corank(incl, base + e);
+            const Pos f = __shfl_sync(0xffffffffu, start, i);
+            const bool in = e < stop;
+            int m = 0;
+            if (in) {
+                m = w.find[f + (Pos)(base + e)];
+                sm.member[e] = m;
+                sm.row[e] = (unsigned char)i;
+            }
+            __syncwarp();
+            bool won = false;
+            if (in) {
+                unsigned int h = hash_slot(m, kLog);
+                while (true) {
+                    const unsigned short old = atomicCAS(&sm.slot[h], kNoEdge, (unsigned short)e);
+                    won = old == kNoEdge;
+                    if (won || sm.member[old] == m) break;
+                    h = (h + 1) & kMask;
+                }
+                sm.hash[e] = (unsigned short)h;
+            }
+            const unsigned int wm = __ballot_sync(0xffffffffu, won);
+            if (won) {
+                const int id = n + __popc(wm & below);
+                sm.num[e] = (unsigned char)id;
+                sm.first[id] = (unsigned char)e;
+            }
+            n += __popc(wm);
+        }
+        seen = min(seen, stop);
+        __syncwarp();
+        // whole rows only: the edges of a cut row come again in the next tile
+        const int r1 = __popc(__ballot_sync(0xffffffffu, incl - base <= seen));
+        const int edges = __shfl_sync(0xffffffffu, incl, r1 - 1) - base;
+        for (int e = lane; e < edges; e += 32) {
+            const int id = sm.num[sm.slot[sm.hash[e]]];
+            sm.num[e] = (unsigned char)id;
+            atomicOr(&sm.rowbits[id >> 5][sm.row[e]], 1u << (id & 31));
+        }
+        // look the members' lists up
+        auto look = [&](int id, int y) {
+            unsigned int h = hash_slot(y, kLog);
+            unsigned short e = sm.slot[h];
+            while (e != kNoEdge) {
+                if (sm.member[e] == y) {
+                    const int j = sm.num[e];
+                    atomicOr(&sm.adj[j >> 5][id], 1u << (j & 31));
+                    atomicOr(&sm.adj[id >> 5][j], 1u << (id & 31));
+                    break;
+                }
+                h = (h + 1) & kMask;
+                e = sm.slot[h];
+            }
+        };
+        __syncwarp();
+        for (int x0 = 0; x0 < n; x0 += 32) {
+            const int id = x0 + lane;
+            const int e = id < n ? sm.first[id] : edges;
+            int len = 0;
+            Pos qf = 0;
+            const int x = e < edges ? sm.member[e] : -1;
+            if (x >= 0) {
+                const VInfo q = w.vinfo[x];
+                len = q.fdeg;
+                qf = (Pos)q.fbeg;
+            }
+            unsigned int longs = __ballot_sync(0xffffffffu, len > kTileLong);
+            if (len <= kTileLong) {
+                const int head = (int)(qf & 3);
+                const int4 *q4 = reinterpret_cast<const int4 *>(w.find + (qf - (Pos)head));
+                for (int k = -head; k < len; k += 4, ++q4) {
+                    const int4 y = *q4;
+                    if (k >= 0) look(id, y.x);
+                    if (k + 1 >= 0 && k + 1 < len) look(id, y.y);
+                    if (k + 2 >= 0 && k + 2 < len) look(id, y.z);
+                    if (k + 3 < len) look(id, y.w);
+                }
+            }
+            __syncwarp();
+            while (longs) {
+                const int q = __ffs(longs) - 1;
+                longs &= longs - 1;
+                const Pos f = __shfl_sync(0xffffffffu, qf, q);
+                const int ql = __shfl_sync(0xffffffffu, len, q);
+                for (int j = lane; j < ql; j += 64) {
+                    const int y0 = w.find[f + (Pos)j];
+                    const int y1 = j + 32 < ql ? w.find[f + (Pos)(j + 32)] : kNoProbe;
+                    look(x0 + q, y0);
+                    if (y1 != kNoProbe) look(x0 + q, y1);
+                }
+                __syncwarp();
+            }
+        }
+        __syncwarp();
+        // count
+        unsigned int sum = 0;
+        for (int e0 = 0; e0 < edges; e0 += 32) {
+            const int e = e0 + lane;
+            unsigned int c = 0;
+            if (e < edges) {
+                const int id = sm.num[e], r = sm.row[e];
+#pragma unroll
+                for (int k = 0; k < kTileWords; ++k)
+                    c += __popc(sm.rowbits[k][r] & sm.adj[k][id]);
+                if (PV && c) atomicAdd(&sm.credit[id], c);
+            }
+            if (PV) {
+                // a row's edges are consecutive: its lane takes a difference
+                // of prefix sums
+                const int ps = warp_incl_scan((int)c);
+                const int lo = max(incl - fd - base - e0, 0), hi = min(incl - base - e0, 32);
+                const int top = __shfl_sync(0xffffffffu, ps, (hi - 1) & 31);
+                const int bot = __shfl_sync(0xffffffffu, ps, (lo - 1) & 31);
+                if (hi > lo) sum += (unsigned int)(top - (lo > 0 ? bot : 0));
+            } else {
+                sum += c;
+            }
+        }
+        __syncwarp();
+        if (PV) {
+            sum >>= 1;
+            if (sum) add64(&w.tacc[u0 + lane], sum);
+            tri += sum;
+        } else {
+            sum = warp_sum(sum) >> 1;
+            tri += lane == 0 ? sum : 0u;
+        }
+        for (int id = lane; id < n; id += 32) {
+            const int e = sm.first[id];
+            if (PV) {
+                const unsigned int c = sm.credit[id];
+                if (c) credit(w, v0, sm.member[e], c);
+            }
+            sm.slot[sm.hash[e]] = kNoEdge;
+        }
+        base += edges;
+    }
+}
+
+struct TableWarpSmem {
+    int key[4 * kWarpTable];                      // kNoMember = empty
+    unsigned int cnt[4 * kWarpTable];
+};
+
+struct TableBlockSmem {
+    int key[1 << kTableLog2];
+    unsigned int cnt[1 << kTableLog2];
+    int next;
+    unsigned int total;
+};
+
+struct ListSmem {
+    union {
+        TableWarpSmem warp[kThreads / 32];
+        TableBlockSmem block;
+        TileSmem tile[kThreads / 32];
+    };
+    WideClaim claim;
+};
+
+// Shared-memory table of a row's members: linear probing, a counter per slot.
+struct MemberTable {
+    int *key;
+    unsigned int *cnt;
+    int lg;
+
+    __device__ __forceinline__ void insert(int m) const
+    {
+        const unsigned int mask = (1u << lg) - 1u;
+        unsigned int s = hash_slot(m, lg);
+        while (atomicCAS(&key[s], kNoMember, m) != kNoMember) s = (s + 1) & mask;
+    }
+    __device__ __forceinline__ int find(int x) const
+    {
+        const unsigned int mask = (1u << lg) - 1u;
+        unsigned int s = hash_slot(x, lg);
+        int k = key[s];
+        while (k != x && k != kNoMember) {
+            s = (s + 1) & mask;
+            k = key[s];
+        }
+        return k == x ? (int)s : -1;
+    }
+};
+
+// The lists of the members of list[k .. k + 32) that are not core, looked up
+// by the warp, a list at a time, four loads in flight.  Returns this lane's
+// member's hits.
+template <bool PV>
+__device__ __forceinline__ unsigned int probe_members(const Data &w, const int *list, int k, int n,
+                                                      const MemberTable &tab)
+{
+    const int lane = threadIdx.x & 31;
+    const int m = k + lane < n ? list[k + lane] : kNoMember;
+    VInfo q{0, 0, 0};
+    if (m >= 0) q = w.vinfo[m];
+    unsigned int lists = __ballot_sync(0xffffffffu, q.fdeg > 0);
+    unsigned int cq = 0;
+    while (lists) {
+        const int src = __ffs(lists) - 1;
+        lists &= lists - 1;
+        const int *ql = w.find + __shfl_sync(0xffffffffu, q.fbeg, src);
+        const int len = __shfl_sync(0xffffffffu, q.fdeg, src);
+        unsigned int c = 0;
+        for (int j = lane; j < len; j += 128) {
+            int x[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) x[i] = j + 32 * i < len ? ql[j + 32 * i] : kNoProbe;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                if (x[i] == kNoProbe) break;
+                const int s = tab.find(x[i]);
+                if (s >= 0) {
+                    ++c;
+                    if (PV) atomicAdd(&tab.cnt[s], 1u);
+                }
+            }
+        }
+        c = warp_sum(c);
+        if (lane == src) cq = c;
+    }
+    if (PV && cq) add64(&w.tacc[m], cq);
+    return cq;
+}
+
+// A wide row of at most kWarpTable members by a warp.
+template <bool PV>
+__device__ __forceinline__ void table_warp_row(const Data &w, int v, const VInfo &vi, long long v0,
+                                               TableWarpSmem &sm, unsigned long long &tri)
+{
+    const int lane = threadIdx.x & 31;
+    const int *list = w.find + vi.fbeg;
+    const MemberTable tab{sm.key, sm.cnt, max(ceil_log2(4 * (long long)vi.fdeg), 5)};
+    const int slots = 1 << tab.lg;
+    __syncwarp();
+    for (int k = lane; k < slots; k += 32) {
+        sm.key[k] = kNoMember;
+        if (PV) sm.cnt[k] = 0;
+    }
+    __syncwarp();
+    for (int k = lane; k < vi.fdeg; k += 32) tab.insert(list[k]);
+    __syncwarp();
+    unsigned int mine = 0;
+    for (int k = 0; k < vi.fdeg; k += 32) mine += probe_members<PV>(w, list, k, vi.fdeg, tab);
+    mine = warp_sum(mine);
+    __syncwarp();
+    if (mine) {
+        if (PV) {
+            for (int k = lane; k < slots; k += 32)
+                if (sm.cnt[k]) credit(w, v0, sm.key[k], sm.cnt[k]);
+            if (lane == 0) add64(&w.tacc[v], mine);
+        }
+        tri += lane == 0 ? mine : 0u;
+    }
+}
+
+// A longer one by the block, at most kMemberChunk members in the table at a
+// time (a quarter full at most).
+template <bool PV>
+__device__ void table_block_row(const Data &w, int v, const VInfo &vi, long long v0,
+                                TableBlockSmem &sm, unsigned long long &tri)
+{
+    const int lane = threadIdx.x & 31;
+    const int *list = w.find + vi.fbeg;
+    __syncthreads();
+    if (threadIdx.x == 0) sm.total = 0;
+    for (int c0 = 0; c0 < vi.fdeg; c0 += kMemberChunk) {
+        const int nm = min(vi.fdeg - c0, kMemberChunk);
+        const MemberTable tab{sm.key, sm.cnt,
+                              min(max(ceil_log2(8 * (long long)nm), 6), kTableLog2)};
+        const int slots = 1 << tab.lg;
+        for (int k = threadIdx.x; k < slots; k += kThreads) {
+            sm.key[k] = kNoMember;
+            if (PV) sm.cnt[k] = 0;
+        }
+        if (threadIdx.x == 0) sm.next = 0;
+        __syncthreads();
+        for (int k = threadIdx.x; k < nm; k += kThreads) tab.insert(list[c0 + k]);
+        __syncthreads();
+        unsigned int mine = 0;
+        while (true) {
+            int k = 0;
+            if (lane == 0) k = atomicAdd(&sm.next, 32);
+            k = __shfl_sync(0xffffffffu, k, 0);
+            if (k >= vi.fdeg) break;
+            mine += probe_members<PV>(w, list, k, vi.fdeg, tab);
+        }
+        __syncthreads();
+        if (PV)
+            for (int k = threadIdx.x; k < slots; k += kThreads)
+                if (sm.cnt[k]) credit(w, v0, sm.key[k], sm.cnt[k]);
+        const unsigned int ws = warp_sum(mine);
+        if (lane == 0 && ws) atomicAdd(&sm.total, ws);
+        __syncthreads();
+    }
+    if (threadIdx.x == 0 && sm.total) {
+        if (PV) add64(&w.tacc[v], sm.total);
+        tri += sm.total;
+    }
+}
+
+template <bool PV, bool BATCH>
+__device__ __forceinline__ void table_wide_rows(const Data &w, ListSmem &sm,
+                                                unsigned long long &tri)
+{
+    const long long rows = (long long)w.ctr->wide_rows;
+    // a member outside the core, and one more (core rows have none)
+    for (bool first = true;
+         claim_rows(w, sm.claim, &w.ctr->table_wide_next, rows, kWarpTable, first,
+                    [](const VInfo &vi) {
+                        return vi.fdeg >= 2 && vi.fdeg > (vi.dk & INT32_MAX);
+                    });
+         first = false) {
+        for (int k = 0; k < sm.claim.count[1]; ++k) {
+            const int v = sm.claim.row[1][k];
+            table_block_row<PV>(w, v, w.vinfo[v], BATCH ? w.recs[w.gid[v]].v0 : 0, sm.block, tri);
+        }
+        __syncthreads();
+        claimed_by_warps(sm.claim, [&](int v) {
+            table_warp_row<PV>(w, v, w.vinfo[v], BATCH ? w.recs[w.gid[v]].v0 : 0,
+                               sm.warp[threadIdx.x >> 5], tri);
+        });
+    }
+}
+
+template <bool PV, bool BATCH, typename Pos>
+__device__ __forceinline__ void list_short_rows(const Data &w, long long u0, int batch,
+                                                TileSmem &sm, unsigned long long &tri)
+{
+    const int lane = threadIdx.x & 31;
+    VInfo vi{0, 0, 0};
+    int g = 0;
+    if (lane < batch && u0 + lane < w.n) {
+        vi = w.vinfo[u0 + lane];
+        if (BATCH) g = w.gid[u0 + lane];
+    }
+    // not a wide row, at least one member outside the core and one more
+    const bool act = vi.dk >= 0 && vi.fdeg >= 2 && vi.fdeg > vi.dk;
+    tile_rows<PV, BATCH, Pos>(w, u0, vi, g, act, sm, tri);
+}
+
+// ================================================================== kernels
+
+// Warps take `batch` consecutive rows at a time: their own share first, then
+// from a queue.
+template <class Rows>
+__device__ __forceinline__ void warp_batches(unsigned long long *queue, long long n, int batch,
+                                             const Rows &rows)
+{
+    const long long all = (long long)gridDim.x * (kThreads / 32) * batch;
+    long long u0 = ((long long)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5)) * batch;
+    while (u0 < n) {
+        rows(u0);
+        if (all >= n) break;
+        if ((threadIdx.x & 31) == 0)
+            u0 = all + (long long)atomicAdd(queue, (unsigned long long)batch);
+        u0 = __shfl_sync(0xffffffffu, u0, 0);
+    }
+}
+
+__device__ __forceinline__ void add_triangles(Counters *ctr, unsigned long long tri)
+{
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) tri += __shfl_down_sync(0xffffffffu, tri, d);
+    if ((threadIdx.x & 31) == 0 && tri) atomicAdd(&ctr->tri_total, tri);
+}
+
+template <bool BATCH>
+__device__ __forceinline__ bool has_core(const Data &w)
+{
+    return (BATCH ? (long long)w.ctr->u_words : (long long)w.recs[0].core) != 0;
+}
+
+template <bool PV, bool BATCH>
+__global__ void __launch_bounds__(kThreads, 5)
+core_kernel(const Data w, bool do_wide, bool do_short, int batch)
+{
+    __shared__ CoreSmem sm;
+    if (!has_core<BATCH>(w)) return;
+    unsigned long long tri = 0;
+    if (do_wide) core_wide_rows<PV, BATCH>(w, sm, tri);
+    if (do_short)
+        warp_batches(&w.ctr->core_short_next, w.n, batch, [&](long long u0) {
+            core_short_rows<PV, BATCH>(w, u0, batch, tri);
+        });
+    add_triangles(w.ctr, tri);
+}
+
+template <bool PV, bool BATCH, typename Pos>
+__global__ void __launch_bounds__(kThreads, 5)
+list_kernel(const Data w, bool do_wide, bool do_short, int batch)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    ListSmem &sm = *reinterpret_cast<ListSmem *>(smem);
+    unsigned long long tri = 0;
+    if (do_wide && w.ctr->wide_rows > 0) {
+        table_wide_rows<PV, BATCH>(w, sm, tri);
+        __syncthreads();
+    }
+    if (do_short) {
+        tile_init(sm.tile[threadIdx.x >> 5]);
+        warp_batches(&w.ctr->list_short_next, w.n, batch, [&](long long u0) {
+            list_short_rows<PV, BATCH, Pos>(w, u0, batch, sm.tile[threadIdx.x >> 5], tri);
+        });
+    }
+    add_triangles(w.ctr, tri);
+}
+
+// Both, for small graphs, whose time is launches and latency.
+template <bool PV, bool BATCH, typename Pos>
+__global__ void __launch_bounds__(kThreads, 4)
+count_kernel(const Data w, int batch)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    union Smem {
+        ListSmem list;
+        CoreSmem core;
+    };
+    Smem &sm = *reinterpret_cast<Smem *>(smem);
+    unsigned long long tri = 0;
+    const bool core = has_core<BATCH>(w);
+    if (w.ctr->wide_rows > 0) {
+        if (core) core_wide_rows<PV, BATCH>(w, sm.core, tri);
+        __syncthreads();
+        table_wide_rows<PV, BATCH>(w, sm.list, tri);
+        __syncthreads();
+    }
+    tile_init(sm.list.tile[threadIdx.x >> 5]);
+    warp_batches(&w.ctr->list_short_next, w.n, batch, [&](long long u0) {
+        list_short_rows<PV, BATCH, Pos>(w, u0, batch, sm.list.tile[threadIdx.x >> 5], tri);
+        if (core) core_short_rows<PV, BATCH>(w, u0, batch, tri);
+    });
+    add_triangles(w.ctr, tri);
+}
+
+// ================================================================ epilogue
+
+__device__ __forceinline__ void write_global(const Counters *ctr, long long *global)
+{
+    const long long T = (long long)ctr->tri_total;
+    global[0] = T;
+    global[1] = 3 * T;
+    global[2] = 6 * T;
+}
+
+__global__ void global_kernel(const Counters *ctr, long long *global)
+{
+    write_global(ctr, global);
+}
+
+// Batch in split launches: the core's credits go to their vertices.
+__global__ void core_credits_kernel(const Data w)
+{
+    const long long rows = (long long)w.ctr->wide_rows;
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < rows; i += stride) {
+        const int v = w.wide[i];
+        const GraphRec *rec = &w.recs[w.gid[v]];
+        const int k = w.key[v];
+        if (k > kKeyTop - rec->core) w.tacc[v] += w.tcore[rec->v0 + kKeyTop - k];
+    }
+}
+
+// r, t, lcc of every vertex; a batch's sums of t per graph; thread 0 also
+// writes the global counts (nullable).
+template <typename OffT, bool BATCH>
+__global__ void __launch_bounds__(kThreads)
+finalize_kernel(const View<OffT> w, bool credits, long long *__restrict__ r,
+                long long *__restrict__ t, double *__restrict__ lcc, long long *global)
+{
+    const long long v = (long long)blockIdx.x * kThreads + threadIdx.x;
+    if (v == 0 && global) write_global(w.ctr, global);
+    unsigned long long tv = 0;
+    int g = -1;
+    if (v < w.n) {
+        tv = w.tacc[v];
+        if (BATCH) g = w.gid[v];
+        if (credits) {
+            const GraphRec *rec = &w.recs[BATCH ? g : 0];
+            if (rec->core > 0) {
+                const int k = w.key[v];
+                if (k > kKeyTop - rec->core)
+                    tv += w.tcore[(BATCH ? rec->v0 : 0) + kKeyTop - k];
+            }
+        }
+        if (r) r[v] = (long long)(2 * tv);
+        if (t) t[v] = (long long)tv;
+        if (lcc) {
+            const long long d = row_degree(w, v);
+            // one IEEE division of exactly converted integers (bit-identical
+            // to the host formula)
+            lcc[v] = d < 2 ? 0.0 : __ddiv_rn((double)(2 * tv), (double)(d * (d - 1)));
+        }
+    }
+    if (BATCH && w.gsum) {
+        // a warp within one graph adds once
+        const int g_all = __shfl_sync(0xffffffffu, g, 0);
+        if (__all_sync(0xffffffffu, g == g_all || g < 0) && g_all >= 0) {
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1) tv += __shfl_down_sync(0xffffffffu, tv, d);
+            if ((threadIdx.x & 31) == 0 && tv) atomicAdd(&w.gsum[g_all], tv);
+        } else if (g >= 0 && tv) {
+            atomicAdd(&w.gsum[g], tv);
+        }
+    }
+}
+
+__global__ void graph_triangles_kernel(const unsigned long long *__restrict__ gsum, long long G,
+                                       long long *__restrict__ graph_T)
+{
+    const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (g < G) graph_T[g] = (long long)(gsum[g] / 3);
+}
+
+}  // namespace gtc

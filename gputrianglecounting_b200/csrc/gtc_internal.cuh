@@ -2,26 +2,22 @@
 //
 // Algorithm (same output as the reference's per-vertex kernel,
 // src/clusteringCount.cu:314-359, computed differently):
-//   1. order the vertices by degree -- as (degree, id) with vertex-id labels,
-//      or by a counting sort into ranks with degree-rank labels -- orient
-//      every undirected edge from its lower to its higher end and build the
-//      forward lists N+(v) in one pass, each at the start of v's own CSR
-//      segment (holding ids or ranks); lists a consumer reads in order are
-//      sorted;
-//   2. give every oriented edge one "apex" that intersects for it: the end
-//      with the longer forward list (ties to the source), except that with
-//      rank labels a block-kernel apex owns every edge to a lower-ranked
-//      neighbour.  The apex's N+ is staged in shared memory (hash table, rank
-//      bitmap or per-rank counters) and the partner's N+ is probed into it --
-//      or, for short lists with vertex-id labels, the two id-ordered lists
-//      are merged by one lane -- so each triangle {u,v,w} is found exactly
-//      once, at the edge between its two lowest-ordered vertices;
-//   3. credit the triangle to all three vertices: the apex through a register
-//      or block count, the partner through a warp reduction or a ballot
-//      popcount, the third vertex w through a shared per-member hit counter
-//      flushed to global memory once per (apex, w).
-// All counting is integer and exact; the result does not depend on the
-// order in which blocks run, on the labels or on the order of equal degrees.
+//   1. order the vertices by degree and orient every undirected edge from its
+//      lower to its higher end; N+(v), v's forward list, is written to the
+//      start of v's own CSR segment in one pass.  The vertices of the highest
+//      degrees -- the core, a set closed upwards in the order -- are numbered
+//      by a counting sort of their degrees (position 0 = highest) and named by
+//      position; every other vertex keeps its id;
+//   2. the core's forward lists become the rows of a triangular bit matrix U:
+//      bit s of row q is set iff q -> s;
+//   3. every triangle p < q < s is found at its lowest vertex p, at the edge
+//      p -> q.  If q is a core vertex then so is s, and the pair (q, s) of
+//      N+(p) is tested in U, one bit per pair.  Otherwise q's forward list is
+//      looked up in a shared-memory table of N+(p);
+//   4. the triangle is credited to p, q and s: p by a sum, q by a population
+//      count, s by a per-member counter, each flushed once per (p, member).
+// All counting is integer and exact; the result does not depend on the order
+// in which blocks run nor on the order of equal degrees.
 #pragma once
 
 #include <cstdint>
@@ -32,39 +28,19 @@
 namespace gtc {
 
 // ------------------------------------------------------------------ tuning
-constexpr int kPrepThreads = 256;           // merge-path tile kernels
-constexpr int kPrepItemsPerThread = 8;      // (rows + entries) per thread
-constexpr int kPrepTile = kPrepThreads * kPrepItemsPerThread;
-constexpr long long kRowPlaceThreadMin = 1ll << 18;   // rows from which a thread takes a row
-constexpr int kLongRowMin = 64;             // longest row a placement thread takes
-
-constexpr int kRowThreads = 256;            // warp-per-item count kernel
-constexpr int kRowSlots = 512;              // shared table slots per warp
-constexpr int kRowMinBlocks = 6;            // 48 warps per SM (register budget 42)
-constexpr int kMinItemLen = 32;             // smallest warp work item (entries)
-constexpr int kMaxItemLen = 32768;          // largest: a 16-bit hit counter must not carry
-constexpr int kBigThreads = 256;            // block-per-row count kernel
-constexpr int kBigMinBlocks = 8;            // 8 blocks (64 warps) per SM: 32 registers
-constexpr int kMinBigChunk = 32;            // smallest block-kernel item (entries)
-constexpr int kBigTableLog2 = 12;
-constexpr int kBigTableSlots = 1 << kBigTableLog2;   // shared hash slots (block kernel)
-constexpr int kBigHashMaxFdeg = 2048;       // longest list hashed (load <= 1/2)
-
-// Degree-rank labels (skewed graphs): vertices are ordered by degree (a
-// counting sort over kRankBuckets degree buckets: exact degrees below half of
-// them, then a float-like map with kRankBuckets / 32 buckets per octave) and
-// every forward list holds the ranks of its members, sorted ascending.
-constexpr int kRankBuckets = 1 << 13;
-constexpr int kRankScanThreads = 1024;
-constexpr int kRankThreads = 256;           // histogram / rank kernels
-constexpr int kRankChunk = 4096;            // vertices per histogram / rank block
-constexpr int kSortThreads = 256;           // forward-list sort kernel (warp per 32 rows)
-constexpr int kSortRegMax = 1024;           // longest list sorted in registers
-constexpr int kDirectRanks = 12288;         // block kernel: one 16-bit counter per rank
-constexpr int kTrimLoads = 2;               // block kernel: loads in flight per partner window
-constexpr int kBitWords = 2048;             // block kernel rank bitmap: 65536 ranks
-constexpr int kBitKeys = 2048;              // longest apex list on the bitmap path
-constexpr int kSegBuckets = 1024;           // degree buckets per graph (batched rank labels)
+constexpr int kThreads = 256;               // every pipeline kernel
+constexpr long long kSmallGraph = 1ll << 18;  // vertices from which the core keys get a launch
+constexpr int kShortRow = 64;               // longest row that one placement thread takes
+constexpr int kShortList = 32;              // longest forward list that one warp takes
+constexpr int kRowChunk = 2048;             // entries of a longer row per placement item
+constexpr int kBuckets = 1024;              // degree buckets (counting sort of the core)
+constexpr int kCoreMax = 32768;             // most core vertices of a graph
+constexpr int kCoreMinDegree = kShortRow + 1;   // core rows are never short rows
+constexpr int kCoreDegreeRatio = 4;         // ... and have 4 times the mean degree at least
+constexpr int kMemberChunk = 1024;          // members of a wide row held at a time
+constexpr int kTableLog2 = 12;              // wide rows: shared hash slots
+constexpr int kKeyTop = 0x7fffffff;         // key of core position 0
+constexpr int kNoMember = INT32_MIN;        // never a list element
 
 // Error bits written to the workspace status word (the first 4 bytes of
 // every counting workspace) by device code; gtc_count_status reads them.
@@ -72,22 +48,65 @@ enum : unsigned int {
     kErrIndexRange = 1u,   // a neighbour id outside [0, n) was met (and skipped)
 };
 
-// Per-vertex record built once per count: forward-list start, forward degree
-// and the vertex's order key in one 16-byte load.  The key is the degree
-// (vertex-id labels: order by (degree, id)) or the degree rank (rank labels:
-// every key distinct).
+// Per-vertex record: forward-list start, forward degree and the number of
+// core members, in one 16-byte load.  kWideRow in dk marks rows that a block
+// takes (core rows, rows longer than kShortRow, forward lists longer than
+// kShortList); those are the wide list.
+constexpr int kWideRow = INT32_MIN;
 struct __align__(16) VInfo {
     long long fbeg;
     int fdeg;
-    int key;
+    int dk;
 };
 
-// Order comparison: does x (key kx) come after y (key ky)?  Lexicographic in
-// (key, id), which is the (degree, id) order for degree keys and the rank
-// order for rank keys (distinct keys never reach the id tie-break).
-__device__ __forceinline__ bool rank_above(int kx, int x, int ky, int y)
+// Per-graph record (one for a single graph, one per graph of a batch).
+struct GraphRec {
+    long long v0 = 0;          // first vertex
+    long long ubase = 0;       // first word of the graph's bit matrix
+    int nv = 0;                // vertices
+    int core = 0;              // core vertices K
+    int min_bucket = kBuckets; // lowest degree bucket of the core
+    int dmin = 0;              // lowest degree that may be core
+    int long_min = 0;          // rows longer than this are placed by blocks
+    int kcap = 0;              // most core vertices (bit-matrix space)
+};
+
+// Counters block in the workspace (device, zeroed at the start of a count).
+struct Counters {
+    unsigned long long tri_total;     // triangles found (T)
+    unsigned long long wide_rows;     // entries of the wide list
+    unsigned long long place_items;   // placement items posted for long rows
+    unsigned long long place_next;    // dynamic queues:
+    unsigned long long tile_next;
+    unsigned long long core_wide_next, core_short_next;
+    unsigned long long table_wide_next, list_short_next;
+    unsigned long long u_words;       // bit-matrix words handed out (batch)
+    unsigned int blocks_done;         // degree pass: blocks finished
+};
+
+__host__ __device__ constexpr int ilog2(int v) { return v <= 1 ? 0 : 1 + ilog2(v >> 1); }
+
+// Monotone map of a degree onto kBuckets buckets: exact below half of them,
+// then kBuckets / 32 buckets per octave -- a float with 5 mantissa bits -- for
+// the next 16 octaves, the rest in the last bucket.
+__host__ __device__ __forceinline__ int degree_bucket(int d)
 {
-    return kx > ky || (kx == ky && x > y);
+    constexpr int kExact = kBuckets / 2, kPer = kBuckets / 32;
+    constexpr int kLe = ilog2(kExact), kMb = ilog2(kPer);
+    if (d < kExact) return d < 0 ? 0 : d;
+    int l = kLe;
+    while ((d >> (l + 1)) != 0) ++l;
+    const int b = kExact + (l - kLe) * kPer + ((d >> (l - kMb)) & (kPer - 1));
+    return b < kBuckets ? b : kBuckets - 1;
+}
+
+// First word of core row `pos` in the triangular bit matrix; u_row(K) is the
+// size of a K-row matrix.  Row pos holds bits [0, pos) in whole 32-byte
+// sectors: 8 * (pos / 256 + 1) words.
+__host__ __device__ __forceinline__ int u_row(int pos)
+{
+    const int a = pos >> 8;
+    return 8 * (a + 1) * (128 * a + (pos & 255));
 }
 
 __device__ __forceinline__ unsigned int hash_slot(int key, int log2_slots)
@@ -120,38 +139,5 @@ __device__ __forceinline__ long long row_of_entry(const OffT *__restrict__ off,
     }
     return lo;
 }
-
-// ------------------------------------------------------------ host helpers
-struct Plan {
-    long long n = 0, nnz = 0;
-    int off_bits = 64;
-    long long n_tiles = 0;       // merge-path tiles over rows + entries
-    long long fwd_cap = 0;       // capacity of the forward adjacency
-    // workspace byte offsets
-    size_t o_status = 0, o_counters = 0, o_deg = 0, o_fcnt = 0, o_vinfo = 0, o_find = 0,
-           o_tacc = 0, o_trow = 0, o_irow = 0, o_hist = 0, o_rank = 0, o_order = 0,
-           o_bitem = 0, o_long = 0;
-    size_t bytes = 0;
-};
-
-// Counters block in the workspace (device, zeroed at the start of a count).
-struct Counters {
-    unsigned long long tri_total;     // triangles found (T)
-    unsigned long long row_items;     // dynamic item queue, group kernel
-    unsigned long long big_items;     // dynamic item queue, block kernel
-    unsigned long long big_rows;      // number of rows for the block kernel
-    unsigned long long sort_groups;   // dynamic queue of 32-row groups, list sort
-    unsigned long long big_total;     // block-kernel items posted by the forward build
-    unsigned long long long_rows;     // rows the per-warp row placement leaves to blocks
-    unsigned long long long_next;     // dynamic queue over those rows
-};
-
-
-// out[0..count) = exclusive prefix of in, out[count] = total (in may be out);
-// tmp holds scan_tmp_bytes(count) bytes.
-size_t scan_tmp_bytes(long long count);
-cudaError_t exclusive_scan_i64(const long long *in, long long *out,
-                               long long count, void *tmp,
-                               cudaStream_t stream);
 
 }  // namespace gtc

@@ -75,7 +75,9 @@ extern "C" gtc_status gtc_count_noalloc(const void *d_off, int off_bits, const i
     size_t need = 0;
     gtc_status st = gtc_workspace_size(n, nnz, off_bits, mode, &need);
     if (st != GTC_OK) return st;
-    if (need > kStaticScratchBytes) return GTC_ERR_CAPACITY;
+    // the count's own minimum: with less than `need` the core is smaller
+    if (make_plan(n, nnz, off_bits, mode == GTC_MODE_PLAIN).need > kStaticScratchBytes)
+        return GTC_ERR_CAPACITY;
     if (!d_off || (nnz > 0 && !d_ind)) return GTC_ERR_INVALID_ARGUMENT;
     if (mode == GTC_MODE_ORIENTED && (d_r || d_t || d_lcc)) return GTC_ERR_INVALID_ARGUMENT;
     void *ws = nullptr;
