@@ -123,11 +123,11 @@ __global__ void graph_ids_kernel(const View<OffT> w)
 // Choose a graph's core from its degree histogram (one block of kThreads): the
 // most top buckets that fit kcap.  hist becomes the buckets' first positions.
 __device__ __forceinline__ void choose_core(unsigned int *hist, int dmin, int kcap,
-                                            int &min_bucket, int &core)
+                                            int &min_bucket, int &core, int &uniform)
 {
     constexpr int kPer = kBuckets / kThreads;
     __shared__ unsigned int s_sum[kThreads / 32];
-    __shared__ int s_min, s_core;
+    __shared__ int s_min, s_core, s_any;
     // thread t holds the buckets top - t * kPer - j, j < kPer: a prefix in
     // descending degree
     const int top = kBuckets - 1 - (int)threadIdx.x * kPer;
@@ -137,7 +137,7 @@ __device__ __forceinline__ void choose_core(unsigned int *hist, int dmin, int kc
         h[j] = __ldcg(&hist[top - j]);
         mine += h[j];
     }
-    if (threadIdx.x == 0) { s_min = kBuckets; s_core = 0; }
+    if (threadIdx.x == 0) { s_min = kBuckets; s_core = 0; s_any = 0; }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned int incl = mine;
 #pragma unroll
@@ -154,6 +154,7 @@ __device__ __forceinline__ void choose_core(unsigned int *hist, int dmin, int kc
     for (int j = 0; j < kPer; ++j) {
         hist[top - j] = run;
         run += h[j];
+        if (h[j]) s_any = 1;
         if (top - j >= bmin && run <= (unsigned int)kcap) {
             atomicMin(&s_min, top - j);
             atomicMax(&s_core, (int)run);
@@ -162,6 +163,7 @@ __device__ __forceinline__ void choose_core(unsigned int *hist, int dmin, int kc
     __syncthreads();
     core = s_core;
     min_bucket = core > 0 ? s_min : kBuckets;
+    uniform = !s_any;
 }
 
 // Long row i of the wide list: its record, its placement items and, for a
@@ -173,6 +175,7 @@ __device__ __forceinline__ void key_row(const View<OffT> &w, long long i)
     const long long b = (long long)w.off[v];
     const int d = (int)((long long)w.off[v + 1] - b);
     const int g = w.vstart ? w.gid[v] : 0;
+    if (w.recs[g].uniform) return;
     w.vinfo[v] = VInfo{b, 0, kWideRow};
     const int bk = degree_bucket(d);
     if (bk >= w.recs[g].min_bucket)
@@ -199,38 +202,42 @@ degree_kernel(const View<OffT> w, GraphRec lim, bool ids, bool choose)
 {
     __shared__ int s_g;
     __shared__ bool s_last;
-    const long long v = (long long)blockIdx.x * kThreads + threadIdx.x;
-    if (BATCH && ids) {
-        if (threadIdx.x == 0) s_g = graph_of(w.vstart, w.graphs, v < w.n ? v : w.n - 1);
-        __syncthreads();
-    }
-    bool lng = false;
-    if (v < w.n) {
-        const int d = row_degree(w, v);
-        w.key[v] = d;
-        int g = 0;
-        if (BATCH) {
-            if (ids) {
-                g = walk_graph(w, v, s_g);
-                w.gid[v] = g;
-                lim = batch_limits(w, g);
-            } else {
-                g = w.gid[v];
-                lim = w.recs[g];
-            }
-        }
-        lng = d > lim.long_min;
-        const int bk = degree_bucket(d);
-        if (lng && bk >= degree_bucket(lim.dmin))
-            atomicAdd(&w.hist[(long long)g * kBuckets + bk], 1u);
-    }
-    const unsigned int m = __ballot_sync(0xffffffffu, lng);
     const int lane = threadIdx.x & 31;
-    if (m) {
-        unsigned long long at = 0;
-        if (lane == 0) at = atomicAdd(&w.ctr->wide_rows, (unsigned long long)__popc(m));
-        at = __shfl_sync(0xffffffffu, at, 0);
-        if (lng) w.wide[at + __popc(m & ((1u << lane) - 1u))] = (int)v;
+    const long long stride = (long long)gridDim.x * kThreads;
+    for (long long v0 = (long long)blockIdx.x * kThreads; v0 < w.n; v0 += stride) {
+        const long long v = v0 + threadIdx.x;
+        if (BATCH && ids) {
+            __syncthreads();
+            if (threadIdx.x == 0) s_g = graph_of(w.vstart, w.graphs, v0);
+            __syncthreads();
+        }
+        bool lng = false;
+        if (v < w.n) {
+            const int d = row_degree(w, v);
+            w.key[v] = d;
+            int g = 0;
+            if (BATCH) {
+                if (ids) {
+                    g = walk_graph(w, v, s_g);
+                    w.gid[v] = g;
+                    lim = batch_limits(w, g);
+                } else {
+                    g = w.gid[v];
+                    lim = w.recs[g];
+                }
+            }
+            lng = d > lim.long_min;
+            const int bk = degree_bucket(d);
+            if (lng && bk >= degree_bucket(lim.dmin))
+                atomicAdd(&w.hist[(long long)g * kBuckets + bk], 1u);
+        }
+        const unsigned int m = __ballot_sync(0xffffffffu, lng);
+        if (m) {
+            unsigned long long at = 0;
+            if (lane == 0) at = atomicAdd(&w.ctr->wide_rows, (unsigned long long)__popc(m));
+            at = __shfl_sync(0xffffffffu, at, 0);
+            if (lng) w.wide[at + __popc(m & ((1u << lane) - 1u))] = (int)v;
+        }
     }
     if (!choose) return;
     __threadfence();
@@ -239,7 +246,7 @@ degree_kernel(const View<OffT> w, GraphRec lim, bool ids, bool choose)
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    choose_core(w.hist, lim.dmin, lim.kcap, lim.min_bucket, lim.core);
+    choose_core(w.hist, lim.dmin, lim.kcap, lim.min_bucket, lim.core, lim.uniform);
     if (threadIdx.x == 0) w.recs[0] = lim;
 }
 
@@ -250,9 +257,10 @@ choose_core_kernel(const View<OffT> w, GraphRec lim, bool limits)
 {
     const long long g = blockIdx.x;
     if (BATCH) lim = limits ? batch_limits(w, g) : w.recs[g];
-    int min_bucket = 0, core = 0;
-    choose_core(w.hist + g * kBuckets, lim.dmin, lim.kcap, min_bucket, core);
+    int min_bucket = 0, core = 0, uniform = 0;
+    choose_core(w.hist + g * kBuckets, lim.dmin, lim.kcap, min_bucket, core, uniform);
     if (threadIdx.x == 0) {
+        lim.uniform = uniform;
         lim.min_bucket = min_bucket;
         lim.core = core;
         if (BATCH && core > 0) {
@@ -299,45 +307,59 @@ __global__ void key_rows_kernel(const View<OffT> w, bool zero)
         key_row(w, i);
 }
 
+// Where the rows of a graph keep their forward lists, and what turns a list's
+// ids into vertices: a uniform graph's rows are ordered by id, so a forward
+// list is the end of the row itself.
+struct Lists {
+    const int *base;
+    int shift;
+};
+
+template <bool BATCH>
+__device__ __forceinline__ Lists lists_of(const Data &w, const GraphRec *rec)
+{
+    return rec->uniform ? Lists{w.ind, BATCH ? (int)rec->v0 : 0} : Lists{w.find, 0};
+}
+
 // Forward lists, and the core's bit-matrix rows, in one pass over the
 // adjacency.  x is above v when its key is (ties: the larger id).
-//   * long rows, a block per kRowChunk entries, eight per thread with all
-//     gathers of keys in flight; members are appended a warp's at a time, at
-//     positions reserved by one 64-bit add on {fdeg, dk}, and a core row sets
-//     its bits;
-//   * the other rows, a thread each, four entries at a time.  Their lists
-//     start at a multiple of four entries where the row leaves room, for
-//     16-byte loads.
+//   * long rows, kRowChunk entries per warp, eight per lane with all gathers of
+//     keys in flight; members are appended at positions reserved by one 64-bit
+//     add on {fdeg, dk}, and a core row sets its bits;
+//   * the other rows, 32 consecutive ones per warp, their entries as one
+//     stream, 128 at a time;
+//   * rows of a uniform graph (no degree above a few times the mean) are
+//     ordered by id: no keys are gathered and no list is written, only where
+//     the ids above the row's begin.
 // The order within a list is arbitrary.
 template <typename OffT, bool BATCH>
 __device__ __forceinline__ void place_chunk(const View<OffT> &w, int2 it)
 {
-    constexpr int kPer = kRowChunk / kThreads;
+    constexpr int kPer = kRowChunk / 32;
+    const int lane = threadIdx.x & 31;
     const int v = it.x;
     const long long b = (long long)w.off[v], e = (long long)w.off[v + 1];
     const long long s = b + (long long)it.y * kRowChunk;
     const int kv = w.key[v];
-    long long v0 = 0, nv = w.n, ubase = 0;
-    int g = 0;
-    if (BATCH) g = w.gid[v];
-    const GraphRec *rec = &w.recs[g];
-    if (BATCH) { v0 = rec->v0; nv = rec->nv; ubase = rec->ubase; }
+    const GraphRec *rec = &w.recs[BATCH ? w.gid[v] : 0];
+    const int v0 = BATCH ? (int)rec->v0 : 0;
+    const unsigned int nv = BATCH ? (unsigned int)rec->nv : (unsigned int)w.n;
     const int kmin = kKeyTop - rec->core;            // keys above it are core
     int x[kPer], kx[kPer];
     bool bad = false;
 #pragma unroll
     for (int j = 0; j < kPer; ++j) {
-        const long long i = s + j * kThreads + threadIdx.x;
-        x[j] = i < e ? w.ind[i] : -1;
-        const bool ok = (unsigned long long)(long long)x[j] < (unsigned long long)nv;
-        bad |= i < e && !ok;
-        x[j] = ok ? (int)(x[j] + v0) : -1;
+        const long long i = s + j * 32 + lane;
+        x[j] = i < e ? w.ind[i] : 0;
+        const bool ok = (unsigned int)x[j] < nv;
+        bad |= !ok;
+        x[j] = i < e && ok ? x[j] + v0 : -1;
     }
 #pragma unroll
     for (int j = 0; j < kPer; ++j) kx[j] = x[j] >= 0 ? w.key[x[j]] : -1;
     if (bad) atomicOr(w.status, kErrIndexRange);
     if (kv > kmin) {
-        unsigned int *row = w.u + ubase + u_row(kKeyTop - kv);
+        unsigned int *row = w.u + (BATCH ? rec->ubase : 0) + u_row(kKeyTop - kv);
 #pragma unroll
         for (int j = 0; j < kPer; ++j)
             if (kx[j] > kv) {
@@ -345,7 +367,6 @@ __device__ __forceinline__ void place_chunk(const View<OffT> &w, int2 it)
                 atomicOr(&row[pos >> 5], 1u << (pos & 31));
             }
     }
-    const int lane = threadIdx.x & 31;
     unsigned int fwd[kPer];
     int total = 0, dk = 0;
 #pragma unroll
@@ -370,75 +391,200 @@ __device__ __forceinline__ void place_chunk(const View<OffT> &w, int2 it)
     }
 }
 
-template <typename OffT, bool BATCH>
-__device__ __forceinline__ void place_short(const View<OffT> &w, long long v)
+__device__ __forceinline__ int warp_incl_scan(int v)
 {
-    if (v >= w.n) return;
-    const long long b = (long long)w.off[v];
-    const int d = (int)((long long)w.off[v + 1] - b);
-    const GraphRec *rec = &w.recs[BATCH ? w.gid[v] : 0];
-    if (d > rec->long_min) return;
-    const int v0 = BATCH ? (int)rec->v0 : 0;
-    const unsigned int nv = BATCH ? (unsigned int)rec->nv : (unsigned int)w.n;
-    const int kmin = kKeyTop - rec->core;
-    int *list = w.find + b;
-    int start = (int)(-b & 3), wrote = 0, dk = 0;
-    if (start >= d) start = 0;
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int o = __shfl_up_sync(0xffffffffu, v, d);
+        if (lane >= d) v += o;
+    }
+    return v;
+}
+
+// The lane i whose [incl_i - count_i, incl_i) holds f (incl: this lane's
+// inclusive prefix of a per-lane count).
+__device__ __forceinline__ int warp_corank(int incl, int f)
+{
+    int i = 0;
+#pragma unroll
+    for (int step = 16; step >= 1; step >>= 1) {
+        const int v = __shfl_sync(0xffffffffu, incl, i + step - 1);
+        if (v <= f) i += step;
+    }
+    return i;
+}
+
+// Lanes [lo, hi) as a mask; empty for hi <= lo.
+__device__ __forceinline__ unsigned int lane_range(int lo, int hi)
+{
+    lo = max(lo, 0);
+    hi = min(hi, 32);
+    return hi > lo ? (0xffffffffu >> (32 - hi)) & (0xffffffffu << lo) : 0u;
+}
+
+// A placed row's record; a list longer than `most` makes it a wide row.
+__device__ __forceinline__ void row_record(const Data &w, long long v, long long fbeg, int fdeg,
+                                           int dk, int most, bool listed)
+{
+    if (!listed && fdeg > most) w.wide[atomicAdd(&w.ctr->wide_rows, 1ull)] = (int)v;
+    if (listed || fdeg > most) dk |= kWideRow;
+    w.vinfo[v] = VInfo{fbeg, fdeg, dk};
+}
+
+// Those of rows u0 .. u0 + 31 that are of uniform graphs (mine): where the ids
+// above the row's own begin.
+template <typename OffT, bool BATCH>
+__device__ __forceinline__ void split_rows(const View<OffT> &w, long long u0, int g, bool mine)
+{
+    const int lane = threadIdx.x & 31;
+    const long long v = u0 + lane;
+    long long b = 0, e = 0;
+    int vl = 0, long_min = 0;
+    unsigned int nv = 0;
+    if (mine) {
+        const GraphRec *rec = &w.recs[g];
+        b = (long long)w.off[v];
+        e = (long long)w.off[v + 1];
+        nv = BATCH ? (unsigned int)rec->nv : (unsigned int)w.n;
+        vl = (int)(v - (BATCH ? rec->v0 : 0));
+        long_min = rec->long_min;
+    }
+    // ids out of range, looked for in the rows' entries as one stream
     bool bad = false;
-    for (int k = 0; k < d; k += 4) {
-        int x[4], kx[4];
+    const int g0 = __shfl_sync(0xffffffffu, g, 0);
+    if (__all_sync(0xffffffffu, v >= w.n || (mine && g == g0))) {
+        const unsigned int n0 = __shfl_sync(0xffffffffu, nv, 0);
+        const long long b0 = __shfl_sync(0xffffffffu, b, 0);
+        const int last = (int)min(31ll, w.n - 1 - u0);
+        const long long e1 = __shfl_sync(0xffffffffu, e, last);
+        for (long long i = b0 + lane; i < e1; i += 128) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) x[j] = k + j < d ? w.ind[b + k + j] : -1;
+            for (int j = 0; j < 4; ++j)
+                if (i + 32 * j < e1) bad |= (unsigned int)w.ind[i + 32 * j] >= n0;
+        }
+    } else {
+        bad = true;                               // each lane looks at its own row
+    }
+    if (__any_sync(0xffffffffu, bad)) {
+        bad = false;
+        for (long long i = b; i < e; ++i) bad |= (unsigned int)w.ind[i] >= nv;
+        if (bad) atomicOr(w.status, kErrIndexRange);
+    }
+    if (!mine) return;
+    const bool listed = (int)(e - b) > long_min;
+    long long lo = b;
+    int len = (int)(e - b);
+    while (len > 0) {
+        const int half = len >> 1;
+        if (w.ind[lo + half] <= vl) {
+            lo += half + 1;
+            len -= half + 1;
+        } else {
+            len = half;
+        }
+    }
+    // a row with an id out of range has no list
+    row_record(w, v, lo, bad || e <= lo ? 0 : (int)(e - lo), 0, kShortListIds, listed);
+}
+
+// Rows u0 .. u0 + 31 of other graphs that are not long rows.
+template <typename OffT, bool BATCH>
+__device__ __forceinline__ void stream_rows(const View<OffT> &w, long long u0, int g)
+{
+    constexpr int kPer = 4;
+    const int lane = threadIdx.x & 31;
+    const long long v = u0 + lane;
+    long long b = 0;
+    int d = 0, kmin = kKeyTop, v0 = 0, nv = (int)w.n;
+    bool mine = false;
+    if (v < w.n) {
+        const GraphRec *rec = &w.recs[g];
+        b = (long long)w.off[v];
+        d = (int)((long long)w.off[v + 1] - b);
+        mine = !rec->uniform && d <= rec->long_min;
+        kmin = kKeyTop - rec->core;
+        if (BATCH) {
+            v0 = (int)rec->v0;
+            nv = rec->nv;
+        }
+    }
+    const int n = mine && d > 0 ? d : 0;
+    const int incl = warp_incl_scan(n), excl = incl - n;
+    const int total = __shfl_sync(0xffffffffu, incl, 31);
+    const long long start = b - excl;
+    int wrote = 0, dk = 0;
+    bool bad = false;
+    for (int f0 = 0; f0 < total; f0 += 32 * kPer) {
+        int i[kPer], x[kPer], kx[kPer];
+        long long at[kPer];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const bool ok = (unsigned int)x[j] < nv;
-            bad |= !ok && k + j < d;
-            x[j] += v0;
-            kx[j] = ok ? w.key[x[j]] : -1;
+        for (int j = 0; j < kPer; ++j) {
+            const int f = f0 + 32 * j + lane;
+            i[j] = warp_corank(incl, f);
+            at[j] = __shfl_sync(0xffffffffu, start, i[j]);
+            x[j] = f < total ? w.ind[at[j] + f] : 0;
         }
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-            if (kx[j] > d || (kx[j] == d && x[j] > v)) {
-                const bool core = kx[j] > kmin;
-                if (start > 0 && start + wrote == d) {      // no room: to the row's begin
-                    for (int i = 0; i < wrote; ++i) list[i] = list[start + i];
-                    start = 0;
-                }
-                list[start + wrote++] = core ? (int)((unsigned int)kx[j] ^ 0x80000000u) : x[j];
-                dk += core;
+        for (int j = 0; j < kPer; ++j) {
+            const int f = f0 + 32 * j + lane;
+            const int nj = BATCH ? __shfl_sync(0xffffffffu, nv, i[j]) : nv;
+            const int vj = BATCH ? __shfl_sync(0xffffffffu, v0, i[j]) : 0;
+            const bool ok = (unsigned int)x[j] < (unsigned int)nj;
+            bad |= !ok;
+            x[j] = f < total && ok ? x[j] + vj : -1;
+            kx[j] = x[j] >= 0 ? w.key[x[j]] : -1;
+        }
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            const int g0 = f0 + 32 * j;
+            if (g0 >= total) break;
+            const int di = __shfl_sync(0xffffffffu, d, i[j]);
+            const int ki = __shfl_sync(0xffffffffu, kmin, BATCH ? i[j] : 0);
+            const int ei = __shfl_sync(0xffffffffu, excl, i[j]);
+            const int wi = __shfl_sync(0xffffffffu, wrote, i[j]);
+            const bool f = kx[j] > di || (kx[j] == di && x[j] > (int)(u0 + i[j]));
+            const bool core = kx[j] > ki;
+            const unsigned int mf = __ballot_sync(0xffffffffu, f);
+            const unsigned int mk = __ballot_sync(0xffffffffu, f && core);
+            if (f) {
+                // members of this row before this one: earlier steps', and
+                // this step's from the row's first lane on
+                const int p = wi + __popc(mf & lane_range(ei - g0, lane));
+                w.find[at[j] + ei + p] = core ? (int)((unsigned int)kx[j] ^ 0x80000000u) : x[j];
             }
+            const unsigned int own = lane_range(excl - g0, incl - g0);
+            wrote += __popc(mf & own);
+            dk += __popc(mk & own);
+        }
     }
     if (bad) atomicOr(w.status, kErrIndexRange);
-    if (wrote > kShortList) {
-        dk |= kWideRow;
-        w.wide[atomicAdd(&w.ctr->wide_rows, 1ull)] = (int)v;
-    }
-    w.vinfo[v] = VInfo{b + start, wrote, dk};
+    if (mine) row_record(w, v, b, wrote, dk, kShortList, false);
 }
 
 template <typename OffT, bool BATCH>
 __global__ void __launch_bounds__(kThreads)
 place_kernel(const View<OffT> w, bool do_wide, bool do_short)
 {
-    __shared__ long long s_item;
-    // a block's first item is its own index, the next ones come from a queue
-    auto items = [&](unsigned long long *queue, long long n, const auto &item) {
-        long long i = blockIdx.x;
-        while (i < n) {
-            item(i);
-            if (gridDim.x >= n) break;
-            __syncthreads();
-            if (threadIdx.x == 0) s_item = (long long)atomicAdd(queue, 1ull) + gridDim.x;
-            __syncthreads();
-            i = s_item;
-        }
-    };
-    if (do_wide)
-        items(&w.ctr->place_next, (long long)w.ctr->place_items,
-              [&](long long i) { place_chunk<OffT, BATCH>(w, w.litem[i]); });
-    if (do_short)
-        items(&w.ctr->tile_next, div_up<long long>(w.n, kThreads),
-              [&](long long i) { place_short<OffT, BATCH>(w, i * kThreads + threadIdx.x); });
+    const int lane = threadIdx.x & 31;
+    const long long warps = (long long)gridDim.x * (kThreads / 32);
+    const long long warp = (long long)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+    if (do_wide) {
+        // chunks are alike, so a fixed share of them is an even one
+        const long long items = (long long)w.ctr->place_items;
+        for (long long i = warp; i < items; i += warps) place_chunk<OffT, BATCH>(w, w.litem[i]);
+    }
+    if (!do_short) return;
+    long long u0 = warp * 32;
+    while (u0 < w.n) {
+        const int g = BATCH && u0 + lane < w.n ? w.gid[u0 + lane] : 0;
+        const bool in = u0 + lane < w.n, uniform = in && w.recs[g].uniform;
+        if (__any_sync(0xffffffffu, uniform)) split_rows<OffT, BATCH>(w, u0, g, uniform);
+        if (__any_sync(0xffffffffu, in && !uniform)) stream_rows<OffT, BATCH>(w, u0, g);
+        if (warps * 32 >= w.n) break;
+        if (lane == 0) u0 = 32 * (warps + (long long)atomicAdd(&w.ctr->place_next, 1ull));
+        u0 = __shfl_sync(0xffffffffu, u0, 0);
+    }
 }
 
 }  // namespace gtc

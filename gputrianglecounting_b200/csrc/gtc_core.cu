@@ -115,9 +115,12 @@ Plan make_plan(long long n, long long nnz, int off_bits, bool per_vertex, long l
     p.need = required_bytes(n, nnz, per_vertex, graphs);
     if (p.need < o) p.need = o;
     // bit matrix: 64 bytes per vertex (32 sqrt(n) core vertices), or all of a
-    // small dense graph
+    // small dense graph; a batch uses what the required size leaves, some 4
+    // bytes per entry
     long long u = 64 * n;
-    if (graphs == 0) {
+    if (graphs > 0) {
+        u = 0;
+    } else {
         const long long most = n < kCoreMax ? n : kCoreMax;
         const long long full = 4ll * u_row((int)most);
         if (n <= kCoreMax && n * n <= 32 * nnz && u < full) u = full;
@@ -170,11 +173,11 @@ int launches_per_count(const RowConfig &cfg, bool per_vertex, long long n)
 namespace {
 
 // Rows per warp batch of a persistent kernel of `blocks` blocks: 32, fewer
-// where that would leave warps idle.
+// where that would leave warps with less than two batches each.
 int rows_per_batch(unsigned blocks, long long n)
 {
     int batch = 32;
-    while (batch > 4 && n < (long long)blocks * (kThreads / 32) * batch) batch >>= 1;
+    while (batch > 2 && n < 2ll * blocks * (kThreads / 32) * batch) batch >>= 1;
     return batch;
 }
 
@@ -190,7 +193,7 @@ template <bool PV, bool BATCH, typename Pos>
 void launch_lists(const Data &w, int dev, cudaStream_t s, bool wide, bool shrt)
 {
     constexpr auto k = list_kernel<PV, BATCH, Pos>;
-    const size_t smem = sizeof(ListSmem);
+    const size_t smem = sizeof(ListSmem<Pos>);
     const unsigned blocks = grid_for<k>(smem, dev, w.n);
     k<<<blocks, kThreads, smem, s>>>(w, wide, shrt, rows_per_batch(blocks, w.n));
 }
@@ -199,7 +202,7 @@ template <bool PV, bool BATCH, typename Pos>
 void launch_both(const Data &w, int dev, cudaStream_t s)
 {
     constexpr auto k = count_kernel<PV, BATCH, Pos>;
-    const size_t smem = sizeof(ListSmem) > sizeof(CoreSmem) ? sizeof(ListSmem) : sizeof(CoreSmem);
+    const size_t smem = sizeof(ListSmem<Pos>) > sizeof(CoreSmem) ? sizeof(ListSmem<Pos>) : sizeof(CoreSmem);
     const unsigned blocks = grid_for<k>(smem, dev, w.n);
     k<<<blocks, kThreads, smem, s>>>(w, rows_per_batch(blocks, w.n));
 }
@@ -222,8 +225,8 @@ gtc_status launch(const View<OffT> &w, GraphRec lim, long long *r, long long *t,
             graph_limits_kernel<<<gb, kThreads, 0, s>>>(w);
             graph_ids_kernel<<<vb, kThreads, 0, s>>>(w);
         }
-        degree_kernel<OffT, BATCH><<<vb, kThreads, 0, s>>>(w, lim, !cfg.split,
-                                                           !BATCH && !cfg.split);
+        degree_kernel<OffT, BATCH><<<vb < sms * 8 ? vb : sms * 8, kThreads, 0, s>>>(
+            w, lim, !cfg.split, !BATCH && !cfg.split);
         if (BATCH || cfg.split)
             choose_core_kernel<OffT, BATCH><<<BATCH ? (unsigned)w.graphs : 1u, kThreads, 0, s>>>(
                 w, lim, !cfg.split);

@@ -40,9 +40,10 @@ __device__ __forceinline__ unsigned int transpose32(unsigned int x, int lane)
 }
 
 // Credit of a list element: vertices in tacc, core positions in tcore.
-__device__ __forceinline__ void credit(const Data &w, long long v0, int m, unsigned int c)
+__device__ __forceinline__ void credit(const Data &w, long long v0, int shift, int m,
+                                       unsigned int c)
 {
-    add64(m >= 0 ? &w.tacc[m] : &w.tcore[v0 + ~m], c);
+    add64(m >= 0 ? &w.tacc[m + shift] : &w.tcore[v0 + ~m], c);
 }
 
 // ============================================== pairs of core members (bits)
@@ -132,70 +133,79 @@ __device__ __forceinline__ void warp_sort(int (&v)[E], int lane)
 
 // Longest list of a wide row that a warp takes: bit matrix, tables.
 constexpr int kWarpList = 256, kWarpTable = 128;
-constexpr int kWideRows = 16;                     // wide rows a block claims at a time
+constexpr int kClaim = 128;                       // most wide rows a block looks through at a time
+constexpr int kWarpClaim = 8;                     // ... a warp
 
-// A block's claim of kWideRows rows of the wide list, parted by list length.
+// A block's share of the wide list's long rows.
 struct WideClaim {
-    int row[2][kWideRows];                        // [0] a warp each, [1] the block together
-    int count[2];
-    int next;
+    int row[kClaim];
+    int count;
     long long item;
 };
 
-// Claim the next wide rows that `want` (of the row's record); false when the
-// list is used up.  A block's first claim is its own share, the next ones come
-// from a queue.  A claim's rows are spread over the list, whose neighbours
-// tend to be alike (generators give hubs the lowest ids).
-template <class Want>
-__device__ __forceinline__ bool claim_rows(const Data &w, WideClaim &cl, unsigned long long *queue,
-                                           long long rows, int most, bool first, const Want &want)
+// The rows of the wide list that `want` (of the row's record): the blocks take
+// those of more than `most` members, each as a whole (by_block), then the
+// warps take the others (by_warp).  First shares are fixed, the next ones come
+// from queues.  A share's rows are spread over the list, whose neighbours tend
+// to be alike (generators give hubs the lowest ids).
+template <class Want, class ByBlock, class ByWarp>
+__device__ __forceinline__ void wide_rows(const Data &w, WideClaim &cl, unsigned long long *long_next,
+                                          unsigned long long *next, int most, const Want &want,
+                                          const ByBlock &by_block, const ByWarp &by_warp)
 {
-    const long long claims = div_up<long long>(rows, kWideRows);
-    if (!first && gridDim.x >= claims) return false;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        long long item = blockIdx.x;
-        if (!first) {
-            if (threadIdx.x == 0) item = gridDim.x + (long long)atomicAdd(queue, 1ull);
-            item = __shfl_sync(0xffffffffu, item, 0);
+    const long long rows = (long long)w.ctr->wide_rows;
+    const int lane = threadIdx.x & 31;
+    // shares small enough that the last ones leave no long tail
+    const long long warps = (long long)gridDim.x * (kThreads / 32);
+    const int per_block = (int)min((long long)kClaim, max(8ll, rows / (4ll * gridDim.x)));
+    const int per_warp = (int)min((long long)kWarpClaim, max(1ll, rows / (16 * warps)));
+    long long claims = div_up<long long>(rows, per_block);
+    long long item = blockIdx.x;
+    while (item < claims) {
+        __syncthreads();
+        if (threadIdx.x == 0) cl.count = 0;
+        __syncthreads();
+        if (threadIdx.x < per_block && item + claims * threadIdx.x < rows) {
+            const int v = w.wide[item + claims * threadIdx.x];
+            const VInfo vi = w.vinfo[v];
+            if (vi.fdeg > most && want(vi)) cl.row[atomicAdd(&cl.count, 1)] = v;
         }
-        const long long at = item < claims && threadIdx.x < kWideRows
-                                 ? item + claims * threadIdx.x : rows;
-        int v = 0;
-        VInfo vi{0, 0, 0};
-        if (at < rows) {
-            v = w.wide[at];
-            vi = w.vinfo[v];
+        __syncthreads();
+        for (int k = 0; k < cl.count; ++k) {
+            const int v = cl.row[k];
+            by_block(v, w.vinfo[v]);
         }
-        const bool in = at < rows && want(vi);
-        const unsigned int below = (1u << threadIdx.x) - 1u;
-        const unsigned int m0 = __ballot_sync(0xffffffffu, in && vi.fdeg <= most);
-        const unsigned int m1 = __ballot_sync(0xffffffffu, in && vi.fdeg > most);
-        if (in) {
-            if (vi.fdeg <= most) cl.row[0][__popc(m0 & below)] = v;
-            else cl.row[1][__popc(m1 & below)] = v;
-        }
-        if (threadIdx.x == 0) {
-            cl.count[0] = __popc(m0);
-            cl.count[1] = __popc(m1);
-            cl.next = 0;
-            cl.item = item;
-        }
+        if (gridDim.x >= claims) break;
+        __syncthreads();
+        if (threadIdx.x == 0) cl.item = gridDim.x + (long long)atomicAdd(long_next, 1ull);
+        __syncthreads();
+        item = cl.item;
     }
     __syncthreads();
-    return cl.item < claims;
-}
-
-// The claimed rows that take a warp each, in turn.
-template <class Row>
-__device__ __forceinline__ void claimed_by_warps(WideClaim &cl, const Row &row)
-{
-    while (true) {
-        int k = 0;
-        if ((threadIdx.x & 31) == 0) k = atomicAdd(&cl.next, 1);
-        k = __shfl_sync(0xffffffffu, k, 0);
-        if (k >= cl.count[0]) break;
-        row(cl.row[0][k]);
+    claims = div_up<long long>(rows, per_warp);
+    item = (long long)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+    while (item < claims) {
+        const long long at = item + claims * lane;
+        int v = 0;
+        VInfo vi{0, 0, 0};
+        bool in = lane < per_warp && at < rows;
+        if (in) {
+            v = w.wide[at];
+            vi = w.vinfo[v];
+            in = vi.fdeg <= most && want(vi);
+        }
+        unsigned int todo = __ballot_sync(0xffffffffu, in);
+        while (todo) {
+            const int k = __ffs(todo) - 1;
+            todo &= todo - 1;
+            by_warp(__shfl_sync(0xffffffffu, v, k),
+                    VInfo{__shfl_sync(0xffffffffu, vi.fbeg, k),
+                          __shfl_sync(0xffffffffu, vi.fdeg, k),
+                          __shfl_sync(0xffffffffu, vi.dk, k)});
+        }
+        if (warps >= claims) break;
+        if (lane == 0) item = warps + (long long)atomicAdd(next, 1ull);
+        item = __shfl_sync(0xffffffffu, item, 0);
     }
 }
 
@@ -450,19 +460,14 @@ template <bool PV, bool BATCH>
 __device__ __forceinline__ void core_wide_rows(const Data &w, CoreSmem &sm,
                                                unsigned long long &tri)
 {
-    const long long rows = (long long)w.ctr->wide_rows;
-    for (bool first = true;
-         claim_rows(w, sm.claim, &w.ctr->core_wide_next, rows, kWarpList, first,
-                    [](const VInfo &vi) { return (vi.dk & INT32_MAX) >= 2; });
-         first = false) {
-        for (int k = 0; k < sm.claim.count[1]; ++k) {
-            const int v = sm.claim.row[1][k];
-            core_block_row<PV>(w, w.vinfo[v], w.recs[BATCH ? w.gid[v] : 0].core,
+    wide_rows(
+        w, sm.claim, &w.ctr->core_long_next, &w.ctr->core_wide_next, kWarpList,
+        [](const VInfo &vi) { return (vi.dk & INT32_MAX) >= 2; },
+        [&](int v, const VInfo &vi) {
+            core_block_row<PV>(w, vi, w.recs[BATCH ? w.gid[v] : 0].core,
                                core_view<PV, BATCH>(w, v), sm.block, tri);
-        }
-        __syncthreads();
-        claimed_by_warps(sm.claim, [&](int v) {
-            const VInfo vi = w.vinfo[v];
+        },
+        [&](int v, const VInfo &vi) {
             const CoreView cv = core_view<PV, BATCH>(w, v);
             CoreWarpSmem &ws = sm.warp[threadIdx.x >> 5];
             if (vi.fdeg <= 32) core_warp_row<1, PV>(w, vi, cv, ws, tri);
@@ -470,7 +475,6 @@ __device__ __forceinline__ void core_wide_rows(const Data &w, CoreSmem &sm,
             else if (vi.fdeg <= 128) core_warp_row<4, PV>(w, vi, cv, ws, tri);
             else core_warp_row<8, PV>(w, vi, cv, ws, tri);
         });
-    }
 }
 
 // Up to 32 consecutive rows by a warp, one after another: a lane per member of
@@ -539,30 +543,6 @@ __device__ __forceinline__ void core_short_rows(const Data &w, long long u0, int
 
 constexpr int kNoProbe = INT32_MIN + 1;           // never a list element nor kNoMember
 
-__device__ __forceinline__ int warp_incl_scan(int v)
-{
-    const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const int o = __shfl_up_sync(0xffffffffu, v, d);
-        if (lane >= d) v += o;
-    }
-    return v;
-}
-
-// The lane i whose [incl_i - count_i, incl_i) holds f (incl: this lane's
-// inclusive prefix of a per-lane count).
-__device__ __forceinline__ int warp_corank(int incl, int f)
-{
-    int i = 0;
-#pragma unroll
-    for (int step = 16; step >= 1; step >>= 1) {
-        const int v = __shfl_sync(0xffffffffu, incl, i + step - 1);
-        if (v <= f) i += step;
-    }
-    return i;
-}
-
 // A tile: consecutive short rows with at most kTileEdges members in all, of
 // which at most kTileIds are distinct.
 constexpr int kTileEdges = 192, kTileIds = 96, kTileWords = kTileIds / 32;
@@ -570,20 +550,30 @@ constexpr int kTileSlots = 1024;
 constexpr int kTileLong = 32;                     // longer lists are taken by the whole warp
 constexpr unsigned short kNoEdge = 0xffff;
 
+template <typename Pos>
 struct __align__(16) TileSmem {
     unsigned short slot[kTileSlots];              // first edge whose member hashes here
     unsigned int adj[kTileWords][kTileIds];       // adjacency among the tile's distinct members
-    unsigned int rowbits[kTileWords][32];         // a row's members
-    unsigned int credit[kTileIds];
+    union {
+        Pos start[kTileIds];                      // a streamed list's begin, less its elements before
+        unsigned int rowbits[kTileWords][32];     // a row's members
+    };
+    union {
+        unsigned int begins[kTileIds];            // bit f: a list begins at element f of the stream
+        unsigned int credit[kTileIds];
+    };
     int member[kTileEdges];                       // an edge's member
-    unsigned short hash[kTileEdges];              // ... its slot
+    unsigned char same[kTileEdges];               // ... the first edge with that member
     unsigned char row[kTileEdges];                // ... its row
     unsigned char num[kTileEdges];                // ... its member's number
     unsigned char first[kTileIds];                // first edge of a number
+    unsigned char owner[kTileIds];                // number whose list is the k-th of the stream
 };
+static_assert(kTileLong * kTileIds <= 32 * kTileIds, "begins holds a bit per streamed element");
 
 // Empties a warp's table; every tile leaves it empty again.
-__device__ __forceinline__ void tile_init(TileSmem &sm)
+template <typename Pos>
+__device__ __forceinline__ void tile_init(TileSmem<Pos> &sm)
 {
     for (int k = threadIdx.x & 31; k < kTileSlots / 2; k += 32)
         reinterpret_cast<unsigned int *>(sm.slot)[k] = 0xffffffffu;
@@ -593,18 +583,20 @@ __device__ __forceinline__ void tile_init(TileSmem &sm)
 // Short rows, a tile at a time by a warp.  The members of all rows of the
 // tile are numbered through a shared hash table (rows near each other share
 // members: on a geometric graph a tile's 160 edges have some 75), every
-// distinct member's forward list is looked up once, and what is found sets
-// the bits of the symmetric adjacency among the numbers.  Then an edge p -> q
-// closes popc(members of p & neighbours of q) triangles: those in which q is
-// the middle and those in which it is the highest vertex, so that is q's
-// credit, and half a row's sum is p's.  The pairs of core members are not
-// among them (their lists are not looked up).  The table is a tenth full, so
-// a look-up that finds nothing mostly ends at its first slot.
+// distinct member's forward list is looked up once -- all lists as one stream,
+// so that every lane has an element -- and what is found sets the bits of the
+// symmetric adjacency among the numbers.  Then an edge p -> q closes
+// popc(members of p & neighbours of q) triangles: those in which q is the
+// middle and those in which it is the highest vertex, so that is q's credit,
+// and half a row's sum is p's.  The pairs of core members are not among them
+// (their lists are not looked up).  The table is a tenth full, so a look-up
+// that finds nothing mostly ends at its first slot.
 template <bool PV, bool BATCH, typename Pos>
 __device__ __forceinline__ void
-tile_rows(const Data &w, long long u0, const VInfo &vi, int g, bool act, TileSmem &sm,
+tile_rows(const Data &w, long long u0, const VInfo &vi, int g, bool act, TileSmem<Pos> &sm,
           unsigned long long &tri)
 {
+    constexpr int kPer = 4;
     const int lane = threadIdx.x & 31;
     const unsigned int below = (1u << lane) - 1u;
     constexpr unsigned int kMask = kTileSlots - 1;
@@ -617,6 +609,7 @@ tile_rows(const Data &w, long long u0, const VInfo &vi, int g, bool act, TileSme
         // rows that may join: one graph (core members are positions in it)
         int stop = total;
         long long v0 = 0;
+        const GraphRec *rec = w.recs;
         if (BATCH) {
             const int f0 = __ffs(__ballot_sync(0xffffffffu, incl > base)) - 1;
             const int gf = __shfl_sync(0xffffffffu, g, f0);
@@ -624,16 +617,17 @@ tile_rows(const Data &w, long long u0, const VInfo &vi, int g, bool act, TileSme
             const int o = other ? __ffs(other) - 1 : 0;
             const int excl = __shfl_sync(0xffffffffu, incl - fd, o);
             if (other) stop = excl;
-            v0 = w.recs[gf].v0;
+            rec += gf;
+            v0 = rec->v0;
         }
+        const Lists ls = lists_of<BATCH>(w, rec);
         stop = min(stop - base, kTileEdges);
         __syncwarp();
 #pragma unroll
         for (int k = 0; k < kTileWords; ++k) {
 #pragma unroll
             for (int j = 0; j < kTileIds / 32; ++j) sm.adj[k][j * 32 + lane] = 0;
-            sm.rowbits[k][lane] = 0;
-            if (PV) sm.credit[k * 32 + lane] = 0;
+            sm.begins[k * 32 + lane] = 0;
         }
         // number the members, 32 edges at a time while there is room
         int n = 0, seen = 0;
@@ -644,7 +638,7 @@ tile_rows(const Data &w, long long u0, const VInfo &vi, int g, bool act, TileSme
             const bool in = e < stop;
             int m = 0;
             if (in) {
-                m = w.find[f + (Pos)(base + e)];
+                m = ls.base[f + (Pos)(base + e)];
                 sm.member[e] = m;
                 sm.row[e] = (unsigned char)i;
             }
@@ -652,13 +646,14 @@ tile_rows(const Data &w, long long u0, const VInfo &vi, int g, bool act, TileSme
             bool won = false;
             if (in) {
                 unsigned int h = hash_slot(m, kLog);
+                unsigned short old;
                 while (true) {
-                    const unsigned short old = atomicCAS(&sm.slot[h], kNoEdge, (unsigned short)e);
+                    old = atomicCAS(&sm.slot[h], kNoEdge, (unsigned short)e);
                     won = old == kNoEdge;
                     if (won || sm.member[old] == m) break;
                     h = (h + 1) & kMask;
                 }
-                sm.hash[e] = (unsigned short)h;
+                sm.same[e] = (unsigned char)(won ? e : old);
             }
             const unsigned int wm = __ballot_sync(0xffffffffu, won);
             if (won) {
@@ -673,64 +668,108 @@ tile_rows(const Data &w, long long u0, const VInfo &vi, int g, bool act, TileSme
         // whole rows only: the edges of a cut row come again in the next tile
         const int r1 = __popc(__ballot_sync(0xffffffffu, incl - base <= seen));
         const int edges = __shfl_sync(0xffffffffu, incl, r1 - 1) - base;
-        for (int e = lane; e < edges; e += 32) {
-            const int id = sm.num[sm.slot[sm.hash[e]]];
-            sm.num[e] = (unsigned char)id;
-            atomicOr(&sm.rowbits[id >> 5][sm.row[e]], 1u << (id & 31));
-        }
-        // look the members' lists up
-        auto look = [&](int id, int y) {
+        // in[j] collects who points at number j
+        auto look = [&](unsigned int *in, unsigned int bit, int y) {
             unsigned int h = hash_slot(y, kLog);
             unsigned short e = sm.slot[h];
             while (e != kNoEdge) {
                 if (sm.member[e] == y) {
-                    const int j = sm.num[e];
-                    atomicOr(&sm.adj[j >> 5][id], 1u << (j & 31));
-                    atomicOr(&sm.adj[id >> 5][j], 1u << (id & 31));
+                    atomicOr(&in[sm.num[e]], bit);
                     break;
                 }
                 h = (h + 1) & kMask;
                 e = sm.slot[h];
             }
         };
-        __syncwarp();
-        for (int x0 = 0; x0 < n; x0 += 32) {
-            const int id = x0 + lane;
+        // the distinct members' lists: lay out the stream
+        int qlen[kTileIds / 32];
+        Pos qfb[kTileIds / 32];
+#pragma unroll
+        for (int k = 0; k < kTileIds / 32; ++k) {
+            const int id = k * 32 + lane;
             const int e = id < n ? sm.first[id] : edges;
-            int len = 0;
-            Pos qf = 0;
             const int x = e < edges ? sm.member[e] : -1;
+            qlen[k] = 0;
+            qfb[k] = 0;
             if (x >= 0) {
-                const VInfo q = w.vinfo[x];
-                len = q.fdeg;
-                qf = (Pos)q.fbeg;
+                const VInfo q = w.vinfo[x + ls.shift];
+                qlen[k] = q.fdeg;
+                qfb[k] = (Pos)q.fbeg;
             }
-            unsigned int longs = __ballot_sync(0xffffffffu, len > kTileLong);
-            if (len <= kTileLong) {
-                const int head = (int)(qf & 3);
-                const int4 *q4 = reinterpret_cast<const int4 *>(w.find + (qf - (Pos)head));
-                for (int k = -head; k < len; k += 4, ++q4) {
-                    const int4 y = *q4;
-                    if (k >= 0) look(id, y.x);
-                    if (k + 1 >= 0 && k + 1 < len) look(id, y.y);
-                    if (k + 2 >= 0 && k + 2 < len) look(id, y.z);
-                    if (k + 3 < len) look(id, y.w);
-                }
+        }
+        int lists = 0, elements = 0;
+#pragma unroll
+        for (int k = 0; k < kTileIds / 32; ++k) {
+            const int len = qlen[k] <= kTileLong ? qlen[k] : 0;
+            const int li = warp_incl_scan(len), le = elements + li - len;
+            const unsigned int have = __ballot_sync(0xffffffffu, len > 0);
+            if (len > 0) {
+                const int o = lists + __popc(have & below);
+                sm.start[o] = qfb[k] - (Pos)le;
+                sm.owner[o] = (unsigned char)(k * 32 + lane);
+                atomicOr(&sm.begins[le >> 5], 1u << (le & 31));
             }
-            __syncwarp();
+            lists += __popc(have);
+            elements += __shfl_sync(0xffffffffu, li, 31);
+        }
+        __syncwarp();
+        // look its elements up, 128 at a time
+        int o0 = -1;                              // lists begun before this step
+        for (int f0 = 0; f0 < elements; f0 += 32 * kPer) {
+            int y[kPer], o[kPer];
+#pragma unroll
+            for (int j = 0; j < kPer; ++j) {
+                const int f = f0 + 32 * j + lane;
+                const unsigned int word = f0 + 32 * j < elements ? sm.begins[(f0 >> 5) + j] : 0u;
+                o[j] = o0 + __popc(word & (below | (1u << lane)));
+                o0 += __popc(word);
+                y[j] = f < elements ? ls.base[sm.start[o[j]] + (Pos)f] : kNoProbe;
+            }
+#pragma unroll
+            for (int j = 0; j < kPer; ++j) {
+                if (f0 + 32 * j >= elements) break;
+                const int id = sm.owner[o[j]];
+                look(sm.adj[id >> 5], 1u << (id & 31), y[j]);
+            }
+        }
+        // the long lists, one by one
+#pragma unroll
+        for (int k = 0; k < kTileIds / 32; ++k) {
+            unsigned int longs = __ballot_sync(0xffffffffu, qlen[k] > kTileLong);
             while (longs) {
                 const int q = __ffs(longs) - 1;
                 longs &= longs - 1;
-                const Pos f = __shfl_sync(0xffffffffu, qf, q);
-                const int ql = __shfl_sync(0xffffffffu, len, q);
+                const int *list = ls.base + (long long)__shfl_sync(0xffffffffu, qfb[k], q);
+                const int ql = __shfl_sync(0xffffffffu, qlen[k], q);
                 for (int j = lane; j < ql; j += 64) {
-                    const int y0 = w.find[f + (Pos)j];
-                    const int y1 = j + 32 < ql ? w.find[f + (Pos)(j + 32)] : kNoProbe;
-                    look(x0 + q, y0);
-                    if (y1 != kNoProbe) look(x0 + q, y1);
+                    const int y0 = list[j];
+                    const int y1 = j + 32 < ql ? list[j + 32] : kNoProbe;
+                    look(sm.adj[k], 1u << q, y0);
+                    if (y1 != kNoProbe) look(sm.adj[k], 1u << q, y1);
                 }
                 __syncwarp();
             }
+        }
+        __syncwarp();
+        // symmetric: with the transposed blocks
+        unsigned int block[kTileWords][kTileWords];
+#pragma unroll
+        for (int k = 0; k < kTileWords; ++k)
+#pragma unroll
+            for (int j = 0; j < kTileWords; ++j) block[k][j] = sm.adj[k][j * 32 + lane];
+#pragma unroll
+        for (int k = 0; k < kTileWords; ++k) {
+#pragma unroll
+            for (int j = 0; j < kTileWords; ++j)
+                sm.adj[k][j * 32 + lane] = block[k][j] | transpose32(block[j][k], lane);
+            sm.rowbits[k][lane] = 0;
+            if (PV) sm.credit[k * 32 + lane] = 0;
+        }
+        __syncwarp();
+        for (int e = lane; e < edges; e += 32) {
+            const int id = sm.num[sm.same[e]];
+            sm.num[e] = (unsigned char)id;
+            atomicOr(&sm.rowbits[id >> 5][sm.row[e]], 1u << (id & 31));
         }
         __syncwarp();
         // count
@@ -767,12 +806,14 @@ tile_rows(const Data &w, long long u0, const VInfo &vi, int g, bool act, TileSme
             tri += lane == 0 ? sum : 0u;
         }
         for (int id = lane; id < n; id += 32) {
-            const int e = sm.first[id];
+            const int e = sm.first[id], m = sm.member[e];
             if (PV) {
                 const unsigned int c = sm.credit[id];
-                if (c) credit(w, v0, sm.member[e], c);
+                if (c) credit(w, v0, ls.shift, m, c);
             }
-            sm.slot[sm.hash[e]] = kNoEdge;
+            unsigned int h = hash_slot(m, kLog);
+            while (sm.slot[h] != (unsigned short)e) h = (h + 1) & kMask;
+            sm.slot[h] = kNoEdge;
         }
         base += edges;
     }
@@ -790,11 +831,12 @@ struct TableBlockSmem {
     unsigned int total;
 };
 
+template <typename Pos>
 struct ListSmem {
     union {
         TableWarpSmem warp[kThreads / 32];
         TableBlockSmem block;
-        TileSmem tile[kThreads / 32];
+        TileSmem<Pos> tile[kThreads / 32];
     };
     WideClaim claim;
 };
@@ -825,52 +867,88 @@ struct MemberTable {
 };
 
 // The lists of the members of list[k .. k + 32) that are not core, looked up
-// by the warp, a list at a time, four loads in flight.  Returns this lane's
-// member's hits.
-template <bool PV>
-__device__ __forceinline__ unsigned int probe_members(const Data &w, const int *list, int k, int n,
+// by the warp: list by list, 128 elements at a time, where they are long, else
+// as one stream (finding each element's list costs as much as looking it up,
+// but short lists one by one would wait for memory one by one).  Returns this
+// lane's member's hits.
+template <bool PV, typename Pos>
+__device__ __forceinline__ unsigned int probe_members(const Data &w, const Lists &ls,
+                                                      const int *list, int k, int n,
                                                       const MemberTable &tab)
 {
+    constexpr int kPer = 4;
     const int lane = threadIdx.x & 31;
     const int m = k + lane < n ? list[k + lane] : kNoMember;
-    VInfo q{0, 0, 0};
-    if (m >= 0) q = w.vinfo[m];
-    unsigned int lists = __ballot_sync(0xffffffffu, q.fdeg > 0);
+    int len = 0;
+    Pos qf = 0;
+    if (m >= 0) {
+        const VInfo q = w.vinfo[m + ls.shift];
+        len = q.fdeg;
+        qf = (Pos)q.fbeg;
+    }
+    const int incl = warp_incl_scan(len), excl = incl - len;
+    const int total = __shfl_sync(0xffffffffu, incl, 31);
+    unsigned int lists = __ballot_sync(0xffffffffu, len > 0);
     unsigned int cq = 0;
-    while (lists) {
-        const int src = __ffs(lists) - 1;
-        lists &= lists - 1;
-        const int *ql = w.find + __shfl_sync(0xffffffffu, q.fbeg, src);
-        const int len = __shfl_sync(0xffffffffu, q.fdeg, src);
-        unsigned int c = 0;
-        for (int j = lane; j < len; j += 128) {
-            int x[4];
+    if (total >= 64 * __popc(lists)) {
+        while (lists) {
+            const int src = __ffs(lists) - 1;
+            lists &= lists - 1;
+            const int *ql = ls.base + __shfl_sync(0xffffffffu, qf, src);
+            const int n = __shfl_sync(0xffffffffu, len, src);
+            unsigned int c = 0;
+            for (int j0 = 0; j0 < n; j0 += 32 * kPer) {
+                int x[kPer];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) x[i] = j + 32 * i < len ? ql[j + 32 * i] : kNoProbe;
+                for (int j = 0; j < kPer; ++j)
+                    x[j] = j0 + 32 * j + lane < n ? ql[j0 + 32 * j + lane] : kNoProbe;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                if (x[i] == kNoProbe) break;
-                const int s = tab.find(x[i]);
-                if (s >= 0) {
-                    ++c;
-                    if (PV) atomicAdd(&tab.cnt[s], 1u);
+                for (int j = 0; j < kPer; ++j) {
+                    if (j0 + 32 * j >= n) break;
+                    const int s = tab.find(x[j]);
+                    if (s >= 0) {
+                        ++c;
+                        if (PV) atomicAdd(&tab.cnt[s], 1u);
+                    }
                 }
             }
+            c = warp_sum(c);
+            if (lane == src) cq = c;
         }
-        c = warp_sum(c);
-        if (lane == src) cq = c;
+        if (PV && cq) add64(&w.tacc[m + ls.shift], cq);
+        return cq;
     }
-    if (PV && cq) add64(&w.tacc[m], cq);
+    const Pos start = qf - (Pos)excl;
+    for (int f0 = 0; f0 < total; f0 += 32 * kPer) {
+        int x[kPer];
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            const int f = f0 + 32 * j + lane;
+            const Pos at = __shfl_sync(0xffffffffu, start, warp_corank(incl, f));
+            x[j] = f < total ? ls.base[at + (Pos)f] : kNoProbe;
+        }
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            const int s = tab.find(x[j]);
+            const unsigned int hm = __ballot_sync(0xffffffffu, s >= 0);
+            if (PV && s >= 0) atomicAdd(&tab.cnt[s], 1u);
+            cq += __popc(hm & lane_range(excl - f0 - 32 * j, incl - f0 - 32 * j));
+        }
+    }
+    if (PV && cq) add64(&w.tacc[m + ls.shift], cq);
     return cq;
 }
 
 // A wide row of at most kWarpTable members by a warp.
-template <bool PV>
-__device__ __forceinline__ void table_warp_row(const Data &w, int v, const VInfo &vi, long long v0,
-                                               TableWarpSmem &sm, unsigned long long &tri)
+template <bool PV, bool BATCH, typename Pos>
+__device__ __forceinline__ void table_warp_row(const Data &w, int v, const VInfo &vi,
+                                               const GraphRec *rec, TableWarpSmem &sm,
+                                               unsigned long long &tri)
 {
     const int lane = threadIdx.x & 31;
-    const int *list = w.find + vi.fbeg;
+    const Lists ls = lists_of<BATCH>(w, rec);
+    const long long v0 = BATCH ? rec->v0 : 0;
+    const int *list = ls.base + vi.fbeg;
     const MemberTable tab{sm.key, sm.cnt, max(ceil_log2(4 * (long long)vi.fdeg), 5)};
     const int slots = 1 << tab.lg;
     __syncwarp();
@@ -882,13 +960,13 @@ __device__ __forceinline__ void table_warp_row(const Data &w, int v, const VInfo
     for (int k = lane; k < vi.fdeg; k += 32) tab.insert(list[k]);
     __syncwarp();
     unsigned int mine = 0;
-    for (int k = 0; k < vi.fdeg; k += 32) mine += probe_members<PV>(w, list, k, vi.fdeg, tab);
+    for (int k = 0; k < vi.fdeg; k += 32) mine += probe_members<PV, Pos>(w, ls, list, k, vi.fdeg, tab);
     mine = warp_sum(mine);
     __syncwarp();
     if (mine) {
         if (PV) {
             for (int k = lane; k < slots; k += 32)
-                if (sm.cnt[k]) credit(w, v0, sm.key[k], sm.cnt[k]);
+                if (sm.cnt[k]) credit(w, v0, ls.shift, sm.key[k], sm.cnt[k]);
             if (lane == 0) add64(&w.tacc[v], mine);
         }
         tri += lane == 0 ? mine : 0u;
@@ -897,12 +975,14 @@ __device__ __forceinline__ void table_warp_row(const Data &w, int v, const VInfo
 
 // A longer one by the block, at most kMemberChunk members in the table at a
 // time (a quarter full at most).
-template <bool PV>
-__device__ void table_block_row(const Data &w, int v, const VInfo &vi, long long v0,
+template <bool PV, bool BATCH, typename Pos>
+__device__ void table_block_row(const Data &w, int v, const VInfo &vi, const GraphRec *rec,
                                 TableBlockSmem &sm, unsigned long long &tri)
 {
     const int lane = threadIdx.x & 31;
-    const int *list = w.find + vi.fbeg;
+    const Lists ls = lists_of<BATCH>(w, rec);
+    const long long v0 = BATCH ? rec->v0 : 0;
+    const int *list = ls.base + vi.fbeg;
     __syncthreads();
     if (threadIdx.x == 0) sm.total = 0;
     for (int c0 = 0; c0 < vi.fdeg; c0 += kMemberChunk) {
@@ -924,12 +1004,12 @@ __device__ void table_block_row(const Data &w, int v, const VInfo &vi, long long
             if (lane == 0) k = atomicAdd(&sm.next, 32);
             k = __shfl_sync(0xffffffffu, k, 0);
             if (k >= vi.fdeg) break;
-            mine += probe_members<PV>(w, list, k, vi.fdeg, tab);
+            mine += probe_members<PV, Pos>(w, ls, list, k, vi.fdeg, tab);
         }
         __syncthreads();
         if (PV)
             for (int k = threadIdx.x; k < slots; k += kThreads)
-                if (sm.cnt[k]) credit(w, v0, sm.key[k], sm.cnt[k]);
+                if (sm.cnt[k]) credit(w, v0, ls.shift, sm.key[k], sm.cnt[k]);
         const unsigned int ws = warp_sum(mine);
         if (lane == 0 && ws) atomicAdd(&sm.total, ws);
         __syncthreads();
@@ -940,33 +1020,26 @@ __device__ void table_block_row(const Data &w, int v, const VInfo &vi, long long
     }
 }
 
-template <bool PV, bool BATCH>
-__device__ __forceinline__ void table_wide_rows(const Data &w, ListSmem &sm,
+template <bool PV, bool BATCH, typename Pos>
+__device__ __forceinline__ void table_wide_rows(const Data &w, ListSmem<Pos> &sm,
                                                 unsigned long long &tri)
 {
-    const long long rows = (long long)w.ctr->wide_rows;
     // a member outside the core, and one more (core rows have none)
-    for (bool first = true;
-         claim_rows(w, sm.claim, &w.ctr->table_wide_next, rows, kWarpTable, first,
-                    [](const VInfo &vi) {
-                        return vi.fdeg >= 2 && vi.fdeg > (vi.dk & INT32_MAX);
-                    });
-         first = false) {
-        for (int k = 0; k < sm.claim.count[1]; ++k) {
-            const int v = sm.claim.row[1][k];
-            table_block_row<PV>(w, v, w.vinfo[v], BATCH ? w.recs[w.gid[v]].v0 : 0, sm.block, tri);
-        }
-        __syncthreads();
-        claimed_by_warps(sm.claim, [&](int v) {
-            table_warp_row<PV>(w, v, w.vinfo[v], BATCH ? w.recs[w.gid[v]].v0 : 0,
-                               sm.warp[threadIdx.x >> 5], tri);
+    wide_rows(
+        w, sm.claim, &w.ctr->table_long_next, &w.ctr->table_wide_next, kWarpTable,
+        [](const VInfo &vi) { return vi.fdeg >= 2 && vi.fdeg > (vi.dk & INT32_MAX); },
+        [&](int v, const VInfo &vi) {
+            table_block_row<PV, BATCH, Pos>(w, v, vi, &w.recs[BATCH ? w.gid[v] : 0], sm.block, tri);
+        },
+        [&](int v, const VInfo &vi) {
+            table_warp_row<PV, BATCH, Pos>(w, v, vi, &w.recs[BATCH ? w.gid[v] : 0],
+                                      sm.warp[threadIdx.x >> 5], tri);
         });
-    }
 }
 
 template <bool PV, bool BATCH, typename Pos>
 __device__ __forceinline__ void list_short_rows(const Data &w, long long u0, int batch,
-                                                TileSmem &sm, unsigned long long &tri)
+                                                TileSmem<Pos> &sm, unsigned long long &tri)
 {
     const int lane = threadIdx.x & 31;
     VInfo vi{0, 0, 0};
@@ -1032,10 +1105,10 @@ __global__ void __launch_bounds__(kThreads, 5)
 list_kernel(const Data w, bool do_wide, bool do_short, int batch)
 {
     extern __shared__ __align__(16) unsigned char smem[];
-    ListSmem &sm = *reinterpret_cast<ListSmem *>(smem);
+    ListSmem<Pos> &sm = *reinterpret_cast<ListSmem<Pos> *>(smem);
     unsigned long long tri = 0;
     if (do_wide && w.ctr->wide_rows > 0) {
-        table_wide_rows<PV, BATCH>(w, sm, tri);
+        table_wide_rows<PV, BATCH, Pos>(w, sm, tri);
         __syncthreads();
     }
     if (do_short) {
@@ -1054,7 +1127,7 @@ count_kernel(const Data w, int batch)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     union Smem {
-        ListSmem list;
+        ListSmem<Pos> list;
         CoreSmem core;
     };
     Smem &sm = *reinterpret_cast<Smem *>(smem);
@@ -1063,7 +1136,7 @@ count_kernel(const Data w, int batch)
     if (w.ctr->wide_rows > 0) {
         if (core) core_wide_rows<PV, BATCH>(w, sm.core, tri);
         __syncthreads();
-        table_wide_rows<PV, BATCH>(w, sm.list, tri);
+        table_wide_rows<PV, BATCH, Pos>(w, sm.list, tri);
         __syncthreads();
     }
     tile_init(sm.list.tile[threadIdx.x >> 5]);

@@ -30,9 +30,10 @@ namespace gtc {
 // ------------------------------------------------------------------ tuning
 constexpr int kThreads = 256;               // every pipeline kernel
 constexpr long long kSmallGraph = 1ll << 18;  // vertices from which the core keys get a launch
-constexpr int kShortRow = 64;               // longest row that one placement thread takes
-constexpr int kShortList = 32;              // longest forward list that one warp takes
-constexpr int kRowChunk = 2048;             // entries of a longer row per placement item
+constexpr int kShortRow = 64;               // longest row placed with its neighbours
+constexpr int kShortList = 32;              // longest forward list of a short row,
+constexpr int kShortListIds = 64;           // ... of a uniform graph
+constexpr int kRowChunk = 256;              // entries of a longer row per placement item
 constexpr int kBuckets = 1024;              // degree buckets (counting sort of the core)
 constexpr int kCoreMax = 32768;             // most core vertices of a graph
 constexpr int kCoreMinDegree = kShortRow + 1;   // core rows are never short rows
@@ -69,6 +70,7 @@ struct GraphRec {
     int dmin = 0;              // lowest degree that may be core
     int long_min = 0;          // rows longer than this are placed by blocks
     int kcap = 0;              // most core vertices (bit-matrix space)
+    int uniform = 0;           // no vertex of core degree: rows ordered by id
 };
 
 // Counters block in the workspace (device, zeroed at the start of a count).
@@ -77,9 +79,8 @@ struct Counters {
     unsigned long long wide_rows;     // entries of the wide list
     unsigned long long place_items;   // placement items posted for long rows
     unsigned long long place_next;    // dynamic queues:
-    unsigned long long tile_next;
-    unsigned long long core_wide_next, core_short_next;
-    unsigned long long table_wide_next, list_short_next;
+    unsigned long long core_long_next, core_wide_next, core_short_next;
+    unsigned long long table_long_next, table_wide_next, list_short_next;
     unsigned long long u_words;       // bit-matrix words handed out (batch)
     unsigned int blocks_done;         // degree pass: blocks finished
 };
