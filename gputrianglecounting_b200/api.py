@@ -201,9 +201,27 @@ def count_subset(off: torch.Tensor, ind: torch.Tensor, vertices: torch.Tensor,
         raise TypeError("vertices must be an int32 CUDA tensor")
     vertices = vertices.contiguous()
     out = torch.empty(vertices.numel(), dtype=torch.int64, device=off.device)
-    check(_lib.load().gtc_count_subset(off.data_ptr(), off_bits, ind.data_ptr(),
-                                       vertices.data_ptr(), vertices.numel(), out.data_ptr(),
-                                       _stream_handle(stream)), "gtc_count_subset")
+    lib = _lib.load()
+    n, nnz = off.numel() - 1, ind.numel()
+    need = ctypes.c_size_t(0)
+    ws = None
+    if vertices.numel() >= 1024:          # fewer never take a workspace
+        check(lib.gtc_subset_workspace_size(n, nnz, off_bits, vertices.numel(),
+                                            ctypes.byref(need)), "gtc_subset_workspace_size")
+    if need.value:
+        try:
+            ws = _alloc_workspace(need.value, off.device)
+        except GTCError:
+            pass                          # without a workspace: row by row
+    if ws is None:
+        check(lib.gtc_count_subset(off.data_ptr(), off_bits, ind.data_ptr(),
+                                   vertices.data_ptr(), vertices.numel(), out.data_ptr(),
+                                   _stream_handle(stream)), "gtc_count_subset")
+        return out
+    check(lib.gtc_count_subset_ws(off.data_ptr(), off_bits, ind.data_ptr(), n, nnz,
+                                  vertices.data_ptr(), vertices.numel(), out.data_ptr(),
+                                  ws.data_ptr(), ws.numel(), _stream_handle(stream)),
+          "gtc_count_subset")
     return out
 
 

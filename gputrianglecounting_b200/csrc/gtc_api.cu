@@ -10,6 +10,7 @@
 #include <mutex>
 
 #include "gtc_core.cuh"
+#include "gtc_data.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -36,78 +37,107 @@ __global__ void validate_offsets_kernel(const OffT *__restrict__ off, long long 
         atomicMin(reason, GTC_CSR_BAD_OFFSETS);
 }
 
-// Phase 2 (warp per row): ids in range, no self-loop, strictly ascending.
+// The row that holds entry e (off[0] <= e < off[n]), found by the whole warp:
+// 32 probes cut the range at a time.
 template <typename OffT>
-__global__ void validate_rows_kernel(const OffT *__restrict__ off,
-                                     const int *__restrict__ ind, long long n,
-                                     int *reason)
+__device__ __forceinline__ long long warp_row_of_entry(const OffT *__restrict__ off, long long n,
+                                                       long long e)
 {
-    if (*(volatile int *)reason != kNoReason) return;
     const int lane = threadIdx.x & 31;
-    const long long warps = ((long long)gridDim.x * blockDim.x) >> 5;
-    for (long long a = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; a < n; a += warps) {
-        const long long rb = off[a], re = off[a + 1];
-        int bad = GTC_CSR_OK + 100;
-        for (long long e = rb + lane; e < re; e += 32) {
-            const int x = ind[e];
-            if ((unsigned long long)(long long)x >= (unsigned long long)n) bad = min(bad, (int)GTC_CSR_INDEX_RANGE);
-            else if (x == a) bad = min(bad, (int)GTC_CSR_SELF_LOOP);
-            if (e > rb && ind[e - 1] >= x) bad = min(bad, (int)GTC_CSR_UNSORTED_OR_DUPLICATE);
-        }
-        if (bad != GTC_CSR_OK + 100) atomicMin(reason, bad);
+    long long lo = 0, hi = n;                      // off[lo] <= e < off[hi]
+    while (hi - lo > 1) {
+        const long long step = (hi - lo + 32) / 33;
+        const long long at = lo + (lane + 1) * step;
+        const unsigned int below = __ballot_sync(0xffffffffu, at < hi && (long long)off[at] <= e);
+        const long long k = __popc(below);         // off is non-decreasing: a prefix of the lanes
+        hi = min(hi, lo + (k + 1) * step);
+        lo += k * step;
     }
+    return lo;
 }
 
-// Phase 3: every (a, x) has its mirror (x, a).  Warps take 32-entry strides
-// of the adjacency (so a hub row is spread over many warps); each lane finds
-// its entry's row from the stride's first row.
+// Phase 2, every entry (a, x) once: x in range, no self-loop, rows strictly
+// ascending, and the mirror (x, a) of every entry with a < x present.  If the
+// rows are sound, reversal maps the entries with a < x injectively onto those
+// with a > x: the graph is symmetric iff every such upper entry's mirror is
+// present and both kinds are equally many (counts[0] and counts[1]), so only
+// upper entries are searched for, half of all.  The smallest failing reason
+// wins, so an unsound row outweighs what its searches say.  Warps take
+// kCheckChunk consecutive entries at a time, so that a hub row is spread over
+// many; the rows are walked 32 at a time with their ends in the lanes.
+constexpr int kCheckChunk = 512;
+
 template <typename OffT>
-__global__ void validate_symmetry_kernel(const OffT *__restrict__ off,
-                                         const int *__restrict__ ind, long long n,
-                                         long long nnz, int *reason,
-                                         unsigned long long *counts)
+__global__ void __launch_bounds__(256)
+validate_entries_kernel(const OffT *__restrict__ off, const int *__restrict__ ind, long long n,
+                        long long nnz, int *reason, unsigned long long *counts)
 {
-    // Rows are strictly ascending without self-loops (checked before), so
-    // reversal maps the entries (a, x) with a < x injectively onto those with
-    // a > x: the graph is symmetric iff every such upper entry's reverse is
-    // present and both kinds are equally many (counts[0] vs counts[1]).  Only
-    // upper entries are searched for, half of all entries.
-    if (*(volatile int *)reason != kNoReason) return;
+    if (*(volatile int *)reason == GTC_CSR_BAD_OFFSETS) return;
     const int lane = threadIdx.x & 31;
     const long long warps = ((long long)gridDim.x * blockDim.x) >> 5;
-    unsigned long long upper = 0, lower = 0;
-    bool ok = true;
-    for (long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w * 32 < nnz;
-         w += warps) {
-        const long long e = w * 32 + lane;
-        long long a = 0;
-        if (lane == 0) a = row_of_entry(off, n, w * 32);
-        a = __shfl_sync(0xffffffffu, a, 0);
-        if (e < nnz) {
-            while ((long long)off[a + 1] <= e) ++a;
-            const int x = ind[e];
-            if (x < a) {
-                ++lower;
-            } else {
-                ++upper;
-                long long lo = off[x], hi = off[x + 1];
-                while (lo < hi) {
-                    const long long mid = (lo + hi) >> 1;
-                    if (ind[mid] < a) lo = mid + 1; else hi = mid;
+    unsigned int upper = 0, lower = 0;
+    int bad = kNoReason;
+    for (long long c = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+         c * kCheckChunk < nnz; c += warps) {
+        long long e = c * kCheckChunk;
+        const long long e1 = min(e + kCheckChunk, nnz);
+        long long r = warp_row_of_entry(off, n, e);
+        while (e < e1) {
+            // lane i: where row r + i ends
+            const long long begin = (long long)off[r];
+            const long long end = (long long)off[min(r + 1 + lane, n)];
+            const long long stop = min(e1, __shfl_sync(0xffffffffu, end, 31));
+            for (; e < stop; e += 32) {
+                const long long f = e + lane;
+                int i = 0;                         // rows that end at or before f
+#pragma unroll
+                for (int step = 16; step >= 1; step >>= 1) {
+                    const long long at = __shfl_sync(0xffffffffu, end, i + step - 1);
+                    if (at <= f) i += step;
                 }
-                if (lo >= (long long)off[x + 1] || ind[lo] != a) ok = false;
+                const long long rb = __shfl_sync(0xffffffffu, end, (i - 1) & 31);
+                if (f < stop) {
+                    const long long a = r + i;
+                    const int x = ind[f];
+                    const bool in = (unsigned long long)(long long)x < (unsigned long long)n;
+                    if (!in) bad = min(bad, (int)GTC_CSR_INDEX_RANGE);
+                    else if (x == a) bad = min(bad, (int)GTC_CSR_SELF_LOOP);
+                    if (f > (i > 0 ? rb : begin) && ind[f - 1] >= x)
+                        bad = min(bad, (int)GTC_CSR_UNSORTED_OR_DUPLICATE);
+                    if (x < a) {
+                        ++lower;
+                    } else {
+                        ++upper;
+                        if (in) {
+                            long long lo = off[x];
+                            const long long hi = off[x + 1];
+                            int len = (int)(hi - lo);
+                            while (len > 0) {
+                                const int half = len >> 1;
+                                if (ind[lo + half] < a) {
+                                    lo += half + 1;
+                                    len -= half + 1;
+                                } else {
+                                    len = half;
+                                }
+                            }
+                            if (lo >= hi || ind[lo] != a)
+                                bad = min(bad, (int)GTC_CSR_ASYMMETRIC);
+                        }
+                    }
+                }
             }
+            e = stop;
+            r = min(r + 32, n - 1);
         }
     }
-    if (!__all_sync(0xffffffffu, ok) && lane == 0) atomicMin(reason, GTC_CSR_ASYMMETRIC);
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) {
-        upper += __shfl_down_sync(0xffffffffu, upper, d);
-        lower += __shfl_down_sync(0xffffffffu, lower, d);
-    }
+    bad = __reduce_min_sync(0xffffffffu, bad);
+    upper = __reduce_add_sync(0xffffffffu, upper);
+    lower = __reduce_add_sync(0xffffffffu, lower);
     if (lane == 0) {
-        if (upper) atomicAdd(&counts[0], upper);
-        if (lower) atomicAdd(&counts[1], lower);
+        if (bad != kNoReason) atomicMin(reason, bad);
+        if (upper) atomicAdd(&counts[0], (unsigned long long)upper);
+        if (lower) atomicAdd(&counts[1], (unsigned long long)lower);
     }
 }
 
@@ -128,15 +158,12 @@ gtc_status run_validate(const OffT *off, const int *ind, long long n, long long 
         int dev = 0, sms = 148;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        long long want = div_up<long long>(n, 8);
-        unsigned blocks = (unsigned)(want < (long long)sms * 16 ? want : (long long)sms * 16);
-        validate_rows_kernel<<<blocks, 256, 0, stream>>>(off, ind, n, reason);
         if (nnz > 0) {
-            const long long swant = div_up<long long>(nnz, 32 * 8);
-            const unsigned sblocks =
-                (unsigned)(swant < (long long)sms * 16 ? swant : (long long)sms * 16);
-            validate_symmetry_kernel<<<sblocks, 256, 0, stream>>>(off, ind, n, nnz, reason,
-                                                                  counts);
+            const long long want = div_up<long long>(nnz, 8ll * kCheckChunk);
+            const unsigned blocks =
+                (unsigned)(want < (long long)sms * 8 ? want : (long long)sms * 8);
+            validate_entries_kernel<OffT><<<blocks, 256, 0, stream>>>(off, ind, n, nnz, reason,
+                                                                      counts);
         }
     }
     // reason word and the two entry counts in one read
@@ -157,8 +184,11 @@ gtc_status run_validate(const OffT *off, const int *ind, long long n, long long 
 // ============================================================ vertex subset
 
 constexpr int kSubThreads = 256;
+constexpr int kSubWarpRow = 128;                  // longest listed row that a warp takes
 constexpr int kSubSlots = 4096;
 constexpr long long kSubHubMin = kSubSlots / 2;   // longer listed rows go to the hub kernel
+constexpr int kSubClaim = 32;                     // listed vertices a block takes at a time
+constexpr long long kSubFew = 8192;               // fewer listed vertices take a block each
 constexpr int kSubHubThreads = 1024;
 constexpr long long kSubHubBits = 1ll << 20;      // bitmap span of a hub row (128 KiB)
 
@@ -207,10 +237,13 @@ __device__ __forceinline__ void add_out(int *o, unsigned long long x)
 // are the only ones read, as in the reference's vertex-list kernel,
 // src/clusteringCount.cu:266-312).  Edges with u == v or a list shorter
 // than two are skipped like the reference (:292-294).  Two kernels:
-//   * subset_kernel, a block per listed vertex of degree <= kSubHubMin: N(v)
-//     goes to a shared hash table; for each neighbour u, N(u) is probed into
-//     the table when it is not much longer, otherwise the shorter row is
-//     binary-searched in the longer.  It writes 0 for the longer rows;
+//   * subset_kernel, rows of at most kSubHubMin neighbours, a warp for those
+//     of at most kSubWarpRow, a block for the others.  N(v) goes to a shared
+//     hash table.  The sum counts adjacent pairs (u, w) of N(v) both ways
+//     round, so a pair need be found from one end only: the rows of the short
+//     neighbours (not much longer than v's) are looked up in the table, where
+//     finding a long w counts twice, and pairs of long neighbours are searched
+//     for, one of each two.  It writes 0 for the longer rows;
 //   * subset_hub_kernel, all blocks on every longer ("hub") row: each block
 //     sets N(v) in a shared bitmap over the row's id span and takes every
 //     gridDim.x-th neighbour, whose row its warps probe into the bitmap with
@@ -221,90 +254,410 @@ __device__ __forceinline__ void add_out(int *o, unsigned long long x)
 //     search.
 // Spreading a hub over the whole GPU matters: on a power-law graph a single
 // hub's probes outnumber those of thousands of ordinary rows.
+// A neighbour row is long from here on (elements), for a listed row of dv.
+__host__ __device__ __forceinline__ int subset_long(int dv)
+{
+    return dv > 16 ? 4 * dv : 64;
+}
+
+template <typename IndT>
+struct SubWarpSmem {
+    IndT key[4 * kSubWarpRow];
+    unsigned char far[4 * kSubWarpRow];           // the slot's member is a long neighbour
+    unsigned char longs[kSubWarpRow];             // index of each long neighbour in the row
+};
+
+template <typename IndT>
+struct SubBlockSmem {
+    IndT key[kSubSlots];
+    unsigned char far[kSubSlots];
+    unsigned short longs[kSubHubMin];             // index of each long neighbour in the row,
+    unsigned short mids[kSubHubMin];              // of each short one of over kSubList entries
+};
+
+template <typename IndT>
+struct SubSmem {
+    union {
+        SubWarpSmem<IndT> warp[kSubThreads / 32];
+        SubBlockSmem<IndT> block;
+    };
+    int row[kSubClaim], wide[kSubClaim];          // claimed vertices: warp rows, block rows
+    int n_row, n_wide, next, n_long, n_mid;
+    unsigned long long sum;
+};
+
+template <typename IndT>
+__device__ __forceinline__ bool cas_empty(IndT *slot, IndT key)
+{
+    if (sizeof(IndT) == 4)
+        return atomicCAS(reinterpret_cast<int *>(slot), -1, (int)key) == -1;
+    return atomicCAS(reinterpret_cast<unsigned long long *>(slot), ~0ull,
+                     (unsigned long long)key) == ~0ull;
+}
+
+// N(v)'s table: slot of w, or -1.
+template <typename IndT>
+__device__ __forceinline__ int sub_find(const IndT *key, int lg, IndT w)
+{
+    const unsigned int mask = (1u << lg) - 1u;
+    unsigned int s = hash_slot((int)w, lg);
+    IndT k = key[s];
+    while (k != w && k != (IndT)-1) {
+        s = (s + 1) & mask;
+        k = key[s];
+    }
+    return k == w ? (int)s : -1;
+}
+
+// Neighbour e of v, to the table; true for a long one.
+template <typename OffT, typename IndT>
+__device__ __forceinline__ bool sub_insert(const OffT *__restrict__ off, IndT u, long long v,
+                                           int dv, IndT *key, unsigned char *far, int lg, int &du)
+{
+    const unsigned int mask = (1u << lg) - 1u;
+    const long long d = (long long)off[u + 1] - (long long)off[u];
+    const bool lng = u != v && d > subset_long(dv);
+    du = u != v && !lng ? (int)d : 0;
+    unsigned int s = hash_slot((int)u, lg);
+    while (!cas_empty(&key[s], u)) s = (s + 1) & mask;
+    far[s] = lng;
+    return lng;
+}
+
+constexpr int kSubList = 64;                      // longer rows are looked up one by one
+
+// Hits of row u (ub, len) in the table, by the warp, 128 elements at a time; a
+// long w counts twice.
+template <typename IndT>
+__device__ __forceinline__ unsigned int sub_row(const IndT *__restrict__ row, int len,
+                                                const IndT *key, const unsigned char *far, int lg)
+{
+    constexpr int kPer = 4;
+    unsigned int acc = 0;
+    for (int i0 = threadIdx.x & 31; i0 < len; i0 += 32 * kPer) {
+        IndT x[kPer];
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) x[j] = i0 + 32 * j < len ? row[i0 + 32 * j] : (IndT)-2;
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            if (i0 + 32 * j >= len) break;
+            const int s = sub_find(key, lg, x[j]);
+            if (s >= 0) acc += 1u + far[s];
+        }
+    }
+    return acc;
+}
+
+// The rows of 32 neighbours of v (this lane's is u, if any) that have at most
+// kSubList entries, looked up by the warp as one stream; with `all` also the
+// other short ones.
+template <typename OffT, typename IndT>
+__device__ __forceinline__ unsigned long long
+sub_stream(const OffT *__restrict__ off, const IndT *__restrict__ ind, bool has, IndT u,
+           long long v, int dv, const IndT *key, const unsigned char *far, int lg, bool all)
+{
+    constexpr int kPer = 4;
+    const int lane = threadIdx.x & 31;
+    long long ub = 0;
+    int du = 0;
+    if (has && u != v) {
+        ub = (long long)off[u];
+        const long long d = (long long)off[u + 1] - ub;
+        du = d >= 2 && d <= subset_long(dv) ? (int)d : 0;
+    }
+    unsigned long long acc = 0;
+    unsigned int rows = all ? __ballot_sync(0xffffffffu, du > kSubList) : 0u;
+    while (rows) {
+        const int src = __ffs(rows) - 1;
+        rows &= rows - 1;
+        acc += sub_row(ind + __shfl_sync(0xffffffffu, ub, src),
+                       __shfl_sync(0xffffffffu, du, src), key, far, lg);
+    }
+    const int len = du <= kSubList ? du : 0;
+    const int incl = warp_incl_scan(len);
+    const int total = __shfl_sync(0xffffffffu, incl, 31);
+    const long long start = ub - (incl - len);
+    for (int f0 = 0; f0 < total; f0 += 32 * kPer) {
+        IndT x[kPer];
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            const int f = f0 + 32 * j + lane;
+            const long long at = __shfl_sync(0xffffffffu, start, warp_corank(incl, f));
+            x[j] = f < total ? ind[at + f] : (IndT)-2;
+        }
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            const int s = sub_find(key, lg, x[j]);
+            if (s >= 0) acc += 1u + far[s];
+        }
+    }
+    return acc;
+}
+
+// Pairs first, first + stride, ... of the n long neighbours longs[] of v:
+// whether the one is in the other's row, the shorter of the two.
+template <typename OffT, typename IndT, typename Idx>
+__device__ __forceinline__ unsigned long long
+sub_pairs(const OffT *__restrict__ off, const IndT *__restrict__ ind, long long vb,
+          const Idx *longs, int n, int first, int stride)
+{
+    constexpr int kPer = 4;                        // searches in flight per thread
+    const int pairs = n * (n - 1) / 2;
+    unsigned long long acc = 0;
+    for (int p0 = first; p0 < pairs; p0 += kPer * stride) {
+        IndT key[kPer];
+        long long lo[kPer];
+        long long len[kPer];
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            const int p = p0 + j * stride;
+            len[j] = 0;
+            if (p >= pairs) continue;
+            int i = (int)((sqrtf(8.0f * (float)p + 1.0f) + 1.0f) * 0.5f);
+            while (i * (i - 1) / 2 > p) --i;
+            while (i * (i + 1) / 2 <= p) ++i;
+            const IndT a = ind[vb + longs[i]], b = ind[vb + longs[p - i * (i - 1) / 2]];
+            const long long ab = off[a], da = (long long)off[a + 1] - ab;
+            const long long bb = off[b], db = (long long)off[b + 1] - bb;
+            lo[j] = da < db ? ab : bb;
+            len[j] = da < db ? da : db;
+            key[j] = da < db ? b : a;
+        }
+        bool more = true;
+        while (more) {
+            IndT x[kPer];
+#pragma unroll
+            for (int j = 0; j < kPer; ++j)
+                x[j] = len[j] > 0 ? ind[lo[j] + (len[j] >> 1)] : (IndT)-1;
+            more = false;
+#pragma unroll
+            for (int j = 0; j < kPer; ++j) {
+                if (len[j] <= 0) continue;
+                const long long half = len[j] >> 1;
+                if (x[j] < key[j]) {
+                    lo[j] += half + 1;
+                    len[j] -= half + 1;
+                } else {
+                    acc += x[j] == key[j];
+                    len[j] = x[j] == key[j] ? 0 : half;
+                }
+                more |= len[j] > 0;
+            }
+        }
+    }
+    return 2 * acc;
+}
+
 template <typename OffT, typename IndT, typename VtxT, typename OutT>
 __global__ void __launch_bounds__(kSubThreads)
 subset_kernel(const OffT *__restrict__ off, const IndT *__restrict__ ind,
-              const VtxT *__restrict__ vertex, long long count,
-              OutT *__restrict__ out)
+              const VtxT *__restrict__ vertex, long long count, OutT *__restrict__ out,
+              const int *__restrict__ skip, int claim, int warp_row, int hub_min)
 {
-    __shared__ long long s_keys[kSubSlots];
-    __shared__ unsigned long long s_sum;
-    auto block = cg::this_thread_block();
-    auto warp = cg::tiled_partition<32>(block);
-    const int wid = warp.meta_group_rank(), lane = warp.thread_rank();
-    constexpr int nwarps = kSubThreads / 32;
-    for (long long k = blockIdx.x; k < count; k += gridDim.x) {
-        const long long v = (long long)vertex[k];
-        const long long vb = off[v], ve = off[v + 1], dv = ve - vb;
-        if (dv > kSubHubMin) {
-            if (threadIdx.x == 0) out[k] = 0;
-            continue;                              // uniform across the block
-        }
-        if (threadIdx.x == 0) s_sum = 0;
-        int log2t = 5;
-        while ((1ll << log2t) < 2 * dv) ++log2t;
-        const unsigned int mask = (1u << log2t) - 1;
-        for (int i = threadIdx.x; i <= (int)mask; i += kSubThreads) s_keys[i] = -1;
+    extern __shared__ __align__(16) unsigned char smem[];
+    SubSmem<IndT> &sm = *reinterpret_cast<SubSmem<IndT> *>(smem);
+    if (skip && *skip) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // a row by the whole block
+    auto block_row = [&](long long k, long long v, long long vb, int dv) {
+        const int lg = ceil_log2(dv > 16 ? 2 * (long long)dv : 32);
         __syncthreads();
-        for (long long i = threadIdx.x; i < dv; i += kSubThreads) {
-            const long long key = (long long)ind[vb + i];
-            unsigned int slot = hash_slot((int)key, log2t);
-            while (true) {
-                unsigned long long prev = atomicCAS((unsigned long long *)&s_keys[slot],
-                                                    (unsigned long long)-1ll,
-                                                    (unsigned long long)key);
-                if (prev == (unsigned long long)-1ll) break;
-                slot = (slot + 1) & mask;
-            }
+        if (threadIdx.x == 0) { sm.sum = 0; sm.n_long = sm.n_mid = sm.next = 0; }
+        for (int i = threadIdx.x; i < (1 << lg); i += kSubThreads) sm.block.key[i] = (IndT)-1;
+        __syncthreads();
+        for (int i = threadIdx.x; i < dv; i += kSubThreads) {
+            int du;
+            if (sub_insert(off, ind[vb + i], v, dv, sm.block.key, sm.block.far, lg, du))
+                sm.block.longs[atomicAdd(&sm.n_long, 1)] = (unsigned short)i;
+            else if (du > kSubList)
+                sm.block.mids[atomicAdd(&sm.n_mid, 1)] = (unsigned short)i;
         }
         __syncthreads();
         unsigned long long acc = 0;
-        if (dv >= 2) {
-            // warps take neighbours u in turn
-            for (long long e = vb + wid; e < ve; e += nwarps) {
-                const long long u = (long long)ind[e];
-                const long long ub = off[u], ue = off[u + 1], du = ue - ub;
-                if (u == v || du < 2) continue;
-                if (du <= 4 * dv) {
-                    for (long long i0 = lane; i0 < du; i0 += 128) {
-                        long long wv[4];
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const long long i = i0 + 32 * j;
-                            wv[j] = i < du ? (long long)ind[ub + i] : -1;
-                        }
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            if (wv[j] < 0) continue;
-                            unsigned int slot = hash_slot((int)wv[j], log2t);
-                            while (true) {
-                                const long long kk = s_keys[slot];
-                                if (kk == wv[j]) { ++acc; break; }
-                                if (kk == -1) break;
-                                slot = (slot + 1) & mask;
-                            }
-                        }
-                    }
-                } else {
-                    acc += search_shorter(ind, vb, dv, ub, du, lane);
-                }
+        for (int i = warp; i < sm.n_mid; i += kSubThreads / 32) {
+            const IndT u = ind[vb + sm.block.mids[i]];
+            const long long ub = off[u];
+            acc += sub_row(ind + ub, (int)((long long)off[u + 1] - ub), sm.block.key,
+                           sm.block.far, lg);
+        }
+        // a share of the neighbours that keeps all warps busy on a short row
+        const int each = min(32, max(4, div_up(dv, kSubThreads / 32)));
+        for (int i = warp * each; i < dv; i += each * (kSubThreads / 32)) {
+            const bool has = lane < each && i + lane < dv;
+            acc += sub_stream(off, ind, has, has ? ind[vb + i + lane] : (IndT)0, v, dv,
+                              sm.block.key, sm.block.far, lg, false);
+        }
+        acc += sub_pairs(off, ind, vb, sm.block.longs, sm.n_long, (int)threadIdx.x,
+                         kSubThreads);
+        const unsigned long long ws =
+            cg::reduce(cg::tiled_partition<32>(cg::this_thread_block()), acc,
+                       cg::plus<unsigned long long>());
+        if (lane == 0 && ws) atomicAdd(&sm.sum, ws);
+        __syncthreads();
+        if (threadIdx.x == 0) { out[k] = (OutT)sm.sum; sm.next = 0; }
+    };
+    if (claim == 1) {
+        for (long long k = blockIdx.x; k < count; k += gridDim.x) {
+            const long long v = (long long)vertex[k];
+            const long long vb = off[v], dv = (long long)off[v + 1] - vb;
+            if (dv < 2 || dv > hub_min) {
+                if (threadIdx.x == 0) out[k] = 0;
+            } else {
+                block_row(k, v, vb, (int)dv);
             }
         }
-        const unsigned long long ws = cg::reduce(warp, acc, cg::plus<unsigned long long>());
-        if (lane == 0 && ws) atomicAdd(&s_sum, ws);
-        __syncthreads();
-        if (threadIdx.x == 0) out[k] = (OutT)s_sum;
-        __syncthreads();
+        return;
     }
+    const long long claims = div_up<long long>(count, claim);
+    for (long long c = blockIdx.x; c < claims; c += gridDim.x) {
+        // part the claimed vertices (spread over the list) by row length
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            const long long k = c + claims * threadIdx.x;
+            long long dv = -1;
+            if (lane < claim && k < count) {
+                const long long v = (long long)vertex[k];
+                dv = (long long)off[v + 1] - (long long)off[v];
+                if (dv > hub_min) out[k] = 0;
+            }
+            const unsigned int below = (1u << lane) - 1u;
+            const bool narrow = dv >= 0 && dv <= warp_row;
+            const bool wide = dv > warp_row && dv <= hub_min;
+            const unsigned int mn = __ballot_sync(0xffffffffu, narrow);
+            const unsigned int mw = __ballot_sync(0xffffffffu, wide);
+            if (narrow) sm.row[__popc(mn & below)] = lane;
+            if (wide) sm.wide[__popc(mw & below)] = lane;
+            if (lane == 0) {
+                sm.n_row = __popc(mn);
+                sm.n_wide = __popc(mw);
+                sm.next = 0;
+            }
+        }
+        __syncthreads();
+        for (int r = 0; r < sm.n_wide; ++r) {
+            const long long k = c + claims * sm.wide[r];
+            const long long v = (long long)vertex[k];
+            block_row(k, v, off[v], (int)((long long)off[v + 1] - (long long)off[v]));
+        }
+        __syncthreads();
+        SubWarpSmem<IndT> &ws = sm.warp[warp];
+        while (true) {
+            int r = 0;
+            if (lane == 0) r = atomicAdd(&sm.next, 1);
+            r = __shfl_sync(0xffffffffu, r, 0);
+            if (r >= sm.n_row) break;
+            const long long k = c + claims * sm.row[r];
+            const long long v = (long long)vertex[k];
+            const long long vb = off[v];
+            const int dv = (int)((long long)off[v + 1] - vb);
+            const int lg = ceil_log2(dv > 8 ? 4 * (long long)dv : 32);
+            __syncwarp();
+            for (int i = lane; i < (1 << lg); i += 32) ws.key[i] = (IndT)-1;
+            __syncwarp();
+            int n_long = 0;
+            for (int i0 = 0; i0 < dv; i0 += 32) {
+                const bool has = i0 + lane < dv;
+                int du;
+                const bool lng = has && sub_insert(off, ind[vb + i0 + lane], v, dv, ws.key,
+                                                   ws.far, lg, du);
+                const unsigned int m = __ballot_sync(0xffffffffu, lng);
+                if (lng) ws.longs[n_long + __popc(m & ((1u << lane) - 1u))] =
+                    (unsigned char)(i0 + lane);
+                n_long += __popc(m);
+            }
+            __syncwarp();
+            unsigned long long acc = 0;
+            if (dv >= 2) {
+                for (int i0 = 0; i0 < dv; i0 += 32) {
+                    const bool has = i0 + lane < dv;
+                    acc += sub_stream(off, ind, has, has ? ind[vb + i0 + lane] : (IndT)0, v, dv,
+                                      ws.key, ws.far, lg, true);
+                }
+                acc += sub_pairs(off, ind, vb, ws.longs, n_long, lane, 32);
+            }
+            acc = cg::reduce(cg::tiled_partition<32>(cg::this_thread_block()), acc,
+                             cg::plus<unsigned long long>());
+            if (lane == 0) out[k] = (OutT)acc;
+        }
+    }
+}
+
+// What the listed vertices' own rows cost, in looked-up elements (a search in
+// a long row as 16), against counting the whole graph: *whole is set when they
+// are more than kSubWhole per adjacency entry, or when one row that a block
+// takes alone is more than one per kSubRow entries.  R-MAT graphs count at some
+// 50 ps an entry (uniform ones at half of that); listed rows take some 5 ps an
+// element, 1 ns for a block alone.
+constexpr unsigned long long kSubWhole = 16, kSubRow = 16;
+
+template <typename OffT>
+__global__ void subset_cost_kernel(const OffT *__restrict__ off, const int *__restrict__ ind,
+                                   const int *__restrict__ vertex, long long count,
+                                   unsigned long long limit, unsigned long long *cost, int *whole)
+{
+    const int lane = threadIdx.x & 31;
+    const long long warps = ((long long)gridDim.x * blockDim.x) >> 5;
+    unsigned long long mine = 0;
+    for (long long k = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < count;
+         k += warps) {
+        const long long v = vertex[k], vb = off[v];
+        const int dv = (int)((long long)off[v + 1] - vb);
+        const bool hub = dv > kSubHubMin;
+        // 128 neighbours at a time; of a longer row than 256, a sample
+        const int each = dv > 256 ? dv / 256 : 1;
+        unsigned int longs = 0;
+        for (int i0 = 0; i0 < dv; i0 += 128 * each) {
+            long long du[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int i = i0 + 32 * j + lane;
+                const int u = i < dv ? ind[vb + i] : -1;
+                du[j] = u >= 0 ? (long long)off[u + 1] - (long long)off[u] : -1;
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (du[j] < 0) continue;
+                if (hub || du[j] <= subset_long(dv)) mine += (unsigned long long)du[j] * each;
+                else longs += each;
+            }
+        }
+        longs = __reduce_add_sync(0xffffffffu, longs);
+        const unsigned long long pairs = 8ull * longs * longs;
+        if (lane == 0) {
+            mine += pairs;
+            if (!hub && pairs * kSubRow > limit / kSubWhole) *whole = 1;
+        }
+    }
+    mine = cg::reduce(cg::tiled_partition<32>(cg::this_thread_block()), mine,
+                      cg::plus<unsigned long long>());
+    if (lane == 0 && mine) {
+        const unsigned long long before = atomicAdd(cost, mine);
+        if (before <= limit && before + mine > limit) *whole = 1;
+    }
+}
+
+// r of the listed vertices after a count of the whole graph (*whole set).
+__global__ void subset_gather_kernel(const Data w, const int *__restrict__ vertex,
+                                     long long count, long long *__restrict__ out)
+{
+    if (!*w.gate) return;
+    const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= count) return;
+    const int v = vertex[k];
+    unsigned long long t = w.tacc[v];
+    const int key = w.key[v];
+    if (key > kKeyTop - w.recs[0].core) t += w.tcore[kKeyTop - key];
+    out[k] = (long long)(2 * t);
 }
 
 template <typename OffT, typename IndT, typename VtxT, typename OutT>
 __global__ void __launch_bounds__(kSubHubThreads, 1)
 subset_hub_kernel(const OffT *__restrict__ off, const IndT *__restrict__ ind,
-                  const VtxT *__restrict__ vertex, long long count,
-                  OutT *__restrict__ out)
+                      const VtxT *__restrict__ vertex, long long count,
+                  OutT *__restrict__ out, const int *__restrict__ skip, long long hub_min)
 {
     extern __shared__ unsigned int s_bits[];          // kSubHubBits / 32 words
+    if (skip && *skip) return;
     __shared__ long long s_hub[kSubHubThreads];
     __shared__ int s_nhub;
     __shared__ long long s_lo, s_hi;
@@ -325,7 +678,7 @@ subset_hub_kernel(const OffT *__restrict__ off, const IndT *__restrict__ ind,
         const long long kk = c0 + threadIdx.x;
         if (kk < count) {
             const long long v = (long long)vertex[kk];
-            if ((long long)off[v + 1] - (long long)off[v] > kSubHubMin)
+            if ((long long)off[v + 1] - (long long)off[v] > hub_min)
                 s_hub[atomicAdd(&s_nhub, 1)] = kk;
         }
         __syncthreads();
@@ -430,17 +783,30 @@ subset_hub_kernel(const OffT *__restrict__ off, const IndT *__restrict__ ind,
     }
 }
 
+// skip: device flag (nullable); set, the kernels leave out as it is.
 template <typename OffT, typename IndT, typename VtxT, typename OutT>
 gtc_status launch_subset(const OffT *off, const IndT *ind, const VtxT *vertex,
-                         long long count, OutT *out, cudaStream_t stream)
+                         long long count, OutT *out, cudaStream_t stream,
+                         const int *skip = nullptr)
 {
     if (count <= 0) return GTC_OK;
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    long long blocks = count < (long long)sms * 8 ? count : (long long)sms * 8;
-    subset_kernel<OffT, IndT, VtxT, OutT><<<(unsigned)blocks, kSubThreads, 0, stream>>>(
-        off, ind, vertex, count, out);
+    auto rows = subset_kernel<OffT, IndT, VtxT, OutT>;
+    const int rsmem = (int)sizeof(SubSmem<IndT>);
+    if (cudaFuncSetAttribute(rows, cudaFuncAttributeMaxDynamicSharedMemorySize, rsmem) !=
+        cudaSuccess)
+        return GTC_ERR_CUDA;
+    // few vertices: a block each, for the time is that of the longest row, and
+    // more rows shared by the whole GPU; many: a warp each for short rows
+    const bool few = count < kSubFew;
+    const int claim = count < kSubFew / 8 ? 1 : (few ? 8 : kSubClaim);
+    const long long hub_min = count < 2 * kSubFew ? kSubHubMin / 4 : kSubHubMin;
+    const long long claims = div_up<long long>(count, claim);
+    const long long blocks = claims < (long long)sms * 8 ? claims : (long long)sms * 8;
+    rows<<<(unsigned)blocks, kSubThreads, rsmem, stream>>>(
+        off, ind, vertex, count, out, skip, claim, few ? kSubWarpRow / 2 : kSubWarpRow, (int)hub_min);
     // the hub kernel adds to what subset_kernel wrote (0 for hubs), in
     // stream order
     auto hub = subset_hub_kernel<OffT, IndT, VtxT, OutT>;
@@ -448,8 +814,41 @@ gtc_status launch_subset(const OffT *off, const IndT *ind, const VtxT *vertex,
     if (cudaFuncSetAttribute(hub, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
         cudaSuccess)
         return GTC_ERR_CUDA;
-    hub<<<(unsigned)sms, kSubHubThreads, smem, stream>>>(off, ind, vertex, count, out);
+    hub<<<(unsigned)sms, kSubHubThreads, smem, stream>>>(off, ind, vertex, count, out, skip, hub_min);
     return cudaGetLastError() == cudaSuccess ? GTC_OK : GTC_ERR_CUDA;
+}
+
+// Whether counting the whole graph may be the cheaper way to a subset of
+// `count` of its n vertices: on R-MAT graphs it is from some n / 200 on.  The
+// estimate and the launches that end at once cost 35 us, which fewer vertices
+// of a uniform graph take altogether.
+bool subset_may_count(long long n, long long nnz, long long count)
+{
+    return nnz > 0 && count >= 16384 && n <= 256 * count;
+}
+
+// A subset of a graph of known size, with a workspace: a cost estimate on the
+// device picks between the listed rows and a count of the whole graph, whose
+// kernels end at once when they are not picked.
+template <typename OffT>
+gtc_status launch_subset_ws(const OffT *off, const int *ind, long long n, long long nnz,
+                            const int *vertex, long long count, long long *out, void *ws,
+                            size_t ws_bytes, cudaStream_t stream)
+{
+    unsigned long long *cost = static_cast<unsigned long long *>(ws);
+    int *whole = reinterpret_cast<int *>(cost + 1);
+    if (cudaMemsetAsync(ws, 0, 16, stream) != cudaSuccess) return GTC_ERR_CUDA;
+    const long long want = div_up<long long>(count, 8);
+    subset_cost_kernel<OffT><<<(unsigned)(want < 1184 ? want : 1184), 256, 0, stream>>>(
+        off, ind, vertex, count, kSubWhole * (unsigned long long)nnz, cost, whole);
+    Data w;
+    gtc_status st = run_count<OffT>(off, ind, n, nnz, true, nullptr, nullptr, nullptr, nullptr,
+                                    static_cast<char *>(ws) + 256, ws_bytes - 256, stream,
+                                    RowConfig{}, nullptr, nullptr, whole, &w);
+    if (st != GTC_OK) return st;
+    subset_gather_kernel<<<(unsigned)div_up<long long>(count, 256), 256, 0, stream>>>(w, vertex,
+                                                                                     count, out);
+    return launch_subset(off, ind, vertex, count, out, stream, whole);
 }
 
 // ================================================================== compat
@@ -683,6 +1082,38 @@ gtc_status gtc_count_subset(const void *d_off, int off_bits, const int32_t *d_in
         return launch_subset(static_cast<const long long *>(d_off), d_ind, d_vertex, count,
                              reinterpret_cast<long long *>(d_out), as_stream(stream));
     return GTC_ERR_INVALID_ARGUMENT;
+}
+
+gtc_status gtc_subset_workspace_size(int64_t n, int64_t nnz, int off_bits, int64_t count,
+                                     size_t *bytes)
+{
+    if (!bytes || n < 0 || nnz < 0 || count < 0 || (off_bits != 32 && off_bits != 64))
+        return GTC_ERR_INVALID_ARGUMENT;
+    *bytes = 0;
+    if (n <= 0x7fffffffll && subset_may_count(n, nnz, count))
+        *bytes = 256 + make_plan(n, nnz, off_bits, true).bytes;
+    return GTC_OK;
+}
+
+gtc_status gtc_count_subset_ws(const void *d_off, int off_bits, const int32_t *d_ind, int64_t n,
+                               int64_t nnz, const int32_t *d_vertex, int64_t count,
+                               int64_t *d_out, void *d_workspace, size_t ws_bytes,
+                               gtc_stream_t stream)
+{
+    size_t need = 0;
+    const gtc_status st = gtc_subset_workspace_size(n, nnz, off_bits, count, &need);
+    if (st != GTC_OK) return st;
+    if (need == 0 || ws_bytes < 256 + make_plan(n, nnz, off_bits, true).need)
+        return gtc_count_subset(d_off, off_bits, d_ind, d_vertex, count, d_out, stream);
+    if (!d_off || !d_ind || !d_vertex || !d_out || !d_workspace ||
+        (reinterpret_cast<uintptr_t>(d_workspace) & 255))
+        return GTC_ERR_INVALID_ARGUMENT;
+    long long *out = reinterpret_cast<long long *>(d_out);
+    if (off_bits == 32)
+        return launch_subset_ws(static_cast<const int *>(d_off), d_ind, n, nnz, d_vertex, count,
+                                out, d_workspace, ws_bytes, as_stream(stream));
+    return launch_subset_ws(static_cast<const long long *>(d_off), d_ind, n, nnz, d_vertex, count,
+                            out, d_workspace, ws_bytes, as_stream(stream));
 }
 
 gtc_status gtc_compat_last_status(void)

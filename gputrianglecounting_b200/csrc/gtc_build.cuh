@@ -5,39 +5,11 @@
 #include <cooperative_groups.h>
 #include <cooperative_groups/scan.h>
 
-#include "gtc_internal.cuh"
+#include "gtc_data.cuh"
 
 namespace gtc {
 
 namespace cg = cooperative_groups;
-
-// What the kernels of one count read and write.
-struct Data {
-    const int *ind;                 // neighbour ids, graph-local in a batch
-    long long n, nnz;
-    const long long *vstart;        // batch: vertex starts, else null
-    long long graphs;
-    GraphRec *recs;
-    unsigned int *hist;             // kBuckets per graph; counts, then cursors
-    int *key;                       // degree, or kKeyTop - position for core vertices
-    int *gid;                       // batch: graph of a vertex
-    VInfo *vinfo;
-    int *find;                      // forward lists; core members as -1 - position
-    int *wide;                      // rows that blocks take
-    int2 *litem;                    // placement items of long rows: {row, chunk}
-    unsigned int *u;                // bit matrices
-    long long ucap;                 // words of it
-    unsigned long long *tacc;       // t(v) without the core's credits (null: global count only)
-    unsigned long long *tcore;      // credits of core vertices: [first vertex + position]
-    unsigned long long *gsum;       // batch: sum of t per graph
-    Counters *ctr;
-    unsigned int *status;
-    int word;                       // sizeof(unsigned int)
-};
-template <typename OffT>
-struct View : Data {
-    const OffT *off;
-};
 
 template <typename OffT>
 __device__ __forceinline__ int row_degree(const View<OffT> &w, long long v)
@@ -61,12 +33,13 @@ __device__ __forceinline__ int graph_of(const long long *__restrict__ vstart, lo
 // is not posted as a long row, the most core vertices.  The core is worth its
 // bit matrix where degrees are skewed: a vertex of at least kCoreDegreeRatio
 // times the mean degree (uniform graphs have none, so they pay nothing but
-// the empty launches).  A small graph so dense that its whole bit matrix is
-// no larger than its adjacency lists (mean degree >= n / 32) is all core.
+// the empty launches).  A small graph of mean degree 64 or more, so dense that
+// its whole bit matrix is no larger than its adjacency lists (mean degree >=
+// n / 32), is all core.
 __host__ __device__ __forceinline__ void core_limits(long long n, long long nnz, long long room,
                                                      int &dmin, int &long_min, int &kcap)
 {
-    const bool all = n <= room && n <= kCoreMax && n * n <= 32 * nnz;
+    const bool all = n <= room && n <= kCoreMax && n * n <= 32 * nnz && nnz >= 64 * n;
     const long long least = div_up<long long>(kCoreDegreeRatio * nnz, n > 0 ? n : 1);
     dmin = all ? 1 : (int)(least > kCoreMinDegree ? least : kCoreMinDegree);
     long_min = all ? 0 : kShortRow;
@@ -200,6 +173,7 @@ template <typename OffT, bool BATCH>
 __global__ void __launch_bounds__(kThreads)
 degree_kernel(const View<OffT> w, GraphRec lim, bool ids, bool choose)
 {
+    if (gated(w)) return;
     __shared__ int s_g;
     __shared__ bool s_last;
     const int lane = threadIdx.x & 31;
@@ -300,6 +274,7 @@ __global__ void zero_bits_kernel(const Data w)
 template <typename OffT>
 __global__ void key_rows_kernel(const View<OffT> w, bool zero)
 {
+    if (gated(w)) return;
     if (zero) zero_bits(w);
     const long long rows = (long long)w.ctr->wide_rows;
     const long long stride = (long long)gridDim.x * blockDim.x;
@@ -389,30 +364,6 @@ __device__ __forceinline__ void place_chunk(const View<OffT> &w, int2 it)
                 kx[j] > kmin ? (int)((unsigned int)kx[j] ^ 0x80000000u) : x[j];
         p += __popc(fwd[j]);
     }
-}
-
-__device__ __forceinline__ int warp_incl_scan(int v)
-{
-    const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const int o = __shfl_up_sync(0xffffffffu, v, d);
-        if (lane >= d) v += o;
-    }
-    return v;
-}
-
-// The lane i whose [incl_i - count_i, incl_i) holds f (incl: this lane's
-// inclusive prefix of a per-lane count).
-__device__ __forceinline__ int warp_corank(int incl, int f)
-{
-    int i = 0;
-#pragma unroll
-    for (int step = 16; step >= 1; step >>= 1) {
-        const int v = __shfl_sync(0xffffffffu, incl, i + step - 1);
-        if (v <= f) i += step;
-    }
-    return i;
 }
 
 // Lanes [lo, hi) as a mask; empty for hi <= lo.
@@ -566,6 +517,7 @@ template <typename OffT, bool BATCH>
 __global__ void __launch_bounds__(kThreads)
 place_kernel(const View<OffT> w, bool do_wide, bool do_short)
 {
+    if (gated(w)) return;
     const int lane = threadIdx.x & 31;
     const long long warps = (long long)gridDim.x * (kThreads / 32);
     const long long warp = (long long)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);

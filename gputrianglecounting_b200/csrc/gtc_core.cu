@@ -123,7 +123,7 @@ Plan make_plan(long long n, long long nnz, int off_bits, bool per_vertex, long l
     } else {
         const long long most = n < kCoreMax ? n : kCoreMax;
         const long long full = 4ll * u_row((int)most);
-        if (n <= kCoreMax && n * n <= 32 * nnz && u < full) u = full;
+        if (n <= kCoreMax && n * n <= 32 * nnz && nnz >= 64 * n && u < full) u = full;
         if (u > full) u = full;
     }
     p.bytes = align256(o + (size_t)u);
@@ -279,7 +279,7 @@ gtc_status run_count(const OffT *off, const int *ind, long long n, long long nnz
                      bool per_vertex, long long *r, long long *t, double *lcc,
                      long long *global, void *ws, size_t ws_bytes,
                      cudaStream_t stream, const RowConfig &cfg, CountTimings *timing,
-                     const Batch *batch)
+                     const Batch *batch, const int *gate, Data *data)
 {
     const long long graphs = batch ? batch->num_graphs : 0;
     const Plan p = make_plan(n, nnz, (int)sizeof(OffT) * 8, per_vertex, graphs);
@@ -296,6 +296,7 @@ gtc_status run_count(const OffT *off, const int *ind, long long n, long long nnz
     w.vstart = batch ? batch->vstart : nullptr;
     w.graphs = graphs;
     w.word = (int)sizeof(unsigned int);
+    w.gate = gate;
     w.status = reinterpret_cast<unsigned int *>(base + p.o_status);
     w.ctr = reinterpret_cast<Counters *>(base + p.o_counters);
     w.recs = reinterpret_cast<GraphRec *>(base + p.o_recs);
@@ -312,6 +313,7 @@ gtc_status run_count(const OffT *off, const int *ind, long long n, long long nnz
     w.tcore = reinterpret_cast<unsigned long long *>(base + p.o_tcore);
     w.gsum = batch && batch->graph_T ? reinterpret_cast<unsigned long long *>(base + p.o_gsum)
                                      : nullptr;
+    if (data) *data = w;
     if (n == 0) {
         if (timing)
             for (int i = 0; i < 5; ++i) cudaEventRecord(timing->ev[i], stream);
@@ -344,10 +346,10 @@ gtc_status run_count(const OffT *off, const int *ind, long long n, long long nnz
 template gtc_status run_count<int>(const int *, const int *, long long, long long, bool,
                                    long long *, long long *, double *, long long *, void *,
                                    size_t, cudaStream_t, const RowConfig &, CountTimings *,
-                                   const Batch *);
+                                   const Batch *, const int *, Data *);
 template gtc_status run_count<long long>(const long long *, const int *, long long, long long,
                                          bool, long long *, long long *, double *, long long *,
                                          void *, size_t, cudaStream_t, const RowConfig &,
-                                         CountTimings *, const Batch *);
+                                         CountTimings *, const Batch *, const int *, Data *);
 
 }  // namespace gtc

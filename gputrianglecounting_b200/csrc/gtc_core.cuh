@@ -5,6 +5,8 @@
 
 namespace gtc {
 
+struct Data;
+
 // Launch plan of one count.
 struct RowConfig {
     // Heavy graphs (mean degree > 24): wide and short rows in launches of
@@ -47,13 +49,17 @@ struct Plan {
 };
 
 Plan make_plan(long long n, long long nnz, int off_bits, bool per_vertex, long long graphs = 0);
+
 RowConfig pick_row_config(long long n, long long nnz);
 
+// gate: device flag (nullable); while it is 0 the kernels end at once.  data
+// (nullable) receives where the count's arrays are.
 template <typename OffT>
 gtc_status run_count(const OffT *off, const int *ind, long long n, long long nnz,
                      bool per_vertex, long long *r, long long *t, double *lcc,
                      long long *global, void *ws, size_t ws_bytes,
                      cudaStream_t stream, const RowConfig &cfg,
-                     CountTimings *timing, const Batch *batch = nullptr);
+                     CountTimings *timing, const Batch *batch = nullptr,
+                     const int *gate = nullptr, Data *data = nullptr);
 
 }  // namespace gtc

@@ -19,25 +19,44 @@ __device__ __forceinline__ unsigned int warp_sum(unsigned int x)
     return __reduce_add_sync(0xffffffffu, x);
 }
 
-// 32 x 32 bit transpose: bit c of lane r's result is bit r of lane c's x.  At
-// distance k the lanes swap the halves of every 2k-bit field; a rotation by k
-// (back for the upper lanes) aligns the partner's bits.
-__device__ __forceinline__ unsigned int transpose32(unsigned int x, int lane)
-{
-    unsigned int y = __shfl_xor_sync(0xffffffffu, x, 16);
-    x = __byte_perm(x, y, lane & 16 ? 0x3276 : 0x5410);
-    y = __shfl_xor_sync(0xffffffffu, x, 8);
-    x = __byte_perm(x, y, lane & 8 ? 0x3715 : 0x6240);
-#pragma unroll
-    for (int k = 4; k >= 1; k >>= 1) {
-        const unsigned int low = k == 4 ? 0x0f0f0f0fu : (k == 2 ? 0x33333333u : 0x55555555u);
-        const unsigned int keep = lane & k ? ~low : low;
-        y = __shfl_xor_sync(0xffffffffu, x, k);
-        y = __funnelshift_l(y, y, lane & k ? 32 - k : k);
-        x = (x & keep) | (y & ~keep);
+// A lane's constants of the 32 x 32 bit transpose.  They are kept (the
+// compiler is not to derive them anew for every transpose).
+struct Transposer {
+    unsigned int sel16, sel8, keep4, keep2, keep1;
+    int rot4, rot2, rot1;
+
+    static __device__ __forceinline__ unsigned int held(unsigned int x)
+    {
+        unsigned int y;
+        asm volatile("mov.b32 %0, %1;" : "=r"(y) : "r"(x));
+        return y;
     }
-    return x;
-}
+    __device__ __forceinline__ explicit Transposer(int lane)
+    {
+        sel16 = held(lane & 16 ? 0x3276 : 0x5410);
+        sel8 = held(lane & 8 ? 0x3715 : 0x6240);
+        keep4 = held(lane & 4 ? 0xf0f0f0f0u : 0x0f0f0f0fu);
+        keep2 = held(lane & 2 ? 0xccccccccu : 0x33333333u);
+        keep1 = held(lane & 1 ? 0xaaaaaaaau : 0x55555555u);
+        rot4 = (int)held(lane & 4 ? 28 : 4);
+        rot2 = (int)held(lane & 2 ? 30 : 2);
+        rot1 = (int)held(lane & 1 ? 31 : 1);
+    }
+    // Bit c of lane r's result is bit r of lane c's x.  At distance k the lanes
+    // swap the halves of every 2k-bit field; a rotation by k (back for the upper
+    // lanes) aligns the partner's bits.
+    __device__ __forceinline__ unsigned int operator()(unsigned int x) const
+    {
+        x = __byte_perm(x, __shfl_xor_sync(0xffffffffu, x, 16), sel16);
+        x = __byte_perm(x, __shfl_xor_sync(0xffffffffu, x, 8), sel8);
+        unsigned int y = __shfl_xor_sync(0xffffffffu, x, 4);
+        x = (x & keep4) | (__funnelshift_l(y, y, rot4) & ~keep4);
+        y = __shfl_xor_sync(0xffffffffu, x, 2);
+        x = (x & keep2) | (__funnelshift_l(y, y, rot2) & ~keep2);
+        y = __shfl_xor_sync(0xffffffffu, x, 1);
+        return (x & keep1) | (__funnelshift_l(y, y, rot1) & ~keep1);
+    }
+};
 
 // Credit of a list element: vertices in tacc, core positions in tcore.
 __device__ __forceinline__ void credit(const Data &w, long long v0, int shift, int m,
@@ -265,7 +284,8 @@ __device__ __forceinline__ CoreView core_view(const Data &w, int v)
 // A row of at most kWarpList members (32 E) by a warp, sorted in registers.
 template <int E, bool PV>
 __device__ __forceinline__ void core_warp_row(const Data &w, const VInfo &vi, const CoreView &cv,
-                                              CoreWarpSmem &sm, unsigned long long &tri)
+                                              const Transposer &tr, CoreWarpSmem &sm,
+                                              unsigned long long &tri)
 {
     const int lane = threadIdx.x & 31;
     int p[E];
@@ -299,7 +319,7 @@ __device__ __forceinline__ void core_warp_row(const Data &w, const VInfo &vi, co
             keep = 0xffffffffu;
             v += __popc(hb);
             // an index modulo 32 belongs to one lane
-            if (PV) sm.cnt[tq * 32 + lane] += __popc(transpose32(hb, lane));
+            if (PV) sm.cnt[tq * 32 + lane] += __popc(tr(hb));
         }
         tot += v;
         if (PV) sm.cnt[si] += v;
@@ -320,7 +340,7 @@ __device__ __forceinline__ void core_warp_row(const Data &w, const VInfo &vi, co
 // of more than kMemberChunk members go chunk by chunk.
 template <bool PV>
 __device__ void core_block_row(const Data &w, const VInfo &vi, int core, const CoreView &cv,
-                               CoreBlockSmem &sm, unsigned long long &tri)
+                               const Transposer &tr, CoreBlockSmem &sm, unsigned long long &tri)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int words = (core + 31) >> 5;
@@ -417,7 +437,7 @@ __device__ void core_block_row(const Data &w, const VInfo &vi, int core, const C
                     if (si >= ns) hb = 0;
                     v += __popc(hb);
                     if (PV) {
-                        const unsigned int c = __popc(transpose32(hb, lane));
+                        const unsigned int c = __popc(tr(hb));
                         if (c) atomicAdd(&sm.qcnt[tq * 32 + lane], c);
                     }
                 }
@@ -460,20 +480,21 @@ template <bool PV, bool BATCH>
 __device__ __forceinline__ void core_wide_rows(const Data &w, CoreSmem &sm,
                                                unsigned long long &tri)
 {
+    const Transposer tr(threadIdx.x & 31);
     wide_rows(
         w, sm.claim, &w.ctr->core_long_next, &w.ctr->core_wide_next, kWarpList,
         [](const VInfo &vi) { return (vi.dk & INT32_MAX) >= 2; },
         [&](int v, const VInfo &vi) {
             core_block_row<PV>(w, vi, w.recs[BATCH ? w.gid[v] : 0].core,
-                               core_view<PV, BATCH>(w, v), sm.block, tri);
+                               core_view<PV, BATCH>(w, v), tr, sm.block, tri);
         },
         [&](int v, const VInfo &vi) {
             const CoreView cv = core_view<PV, BATCH>(w, v);
             CoreWarpSmem &ws = sm.warp[threadIdx.x >> 5];
-            if (vi.fdeg <= 32) core_warp_row<1, PV>(w, vi, cv, ws, tri);
-            else if (vi.fdeg <= 64) core_warp_row<2, PV>(w, vi, cv, ws, tri);
-            else if (vi.fdeg <= 128) core_warp_row<4, PV>(w, vi, cv, ws, tri);
-            else core_warp_row<8, PV>(w, vi, cv, ws, tri);
+            if (vi.fdeg <= 32) core_warp_row<1, PV>(w, vi, cv, tr, ws, tri);
+            else if (vi.fdeg <= 64) core_warp_row<2, PV>(w, vi, cv, tr, ws, tri);
+            else if (vi.fdeg <= 128) core_warp_row<4, PV>(w, vi, cv, tr, ws, tri);
+            else core_warp_row<8, PV>(w, vi, cv, tr, ws, tri);
         });
 }
 
@@ -752,6 +773,7 @@ tile_rows(const Data &w, long long u0, const VInfo &vi, int g, bool act, TileSme
         }
         __syncwarp();
         // symmetric: with the transposed blocks
+        const Transposer tr(lane);
         unsigned int block[kTileWords][kTileWords];
 #pragma unroll
         for (int k = 0; k < kTileWords; ++k)
@@ -761,7 +783,7 @@ tile_rows(const Data &w, long long u0, const VInfo &vi, int g, bool act, TileSme
         for (int k = 0; k < kTileWords; ++k) {
 #pragma unroll
             for (int j = 0; j < kTileWords; ++j)
-                sm.adj[k][j * 32 + lane] = block[k][j] | transpose32(block[j][k], lane);
+                sm.adj[k][j * 32 + lane] = block[k][j] | tr(block[j][k]);
             sm.rowbits[k][lane] = 0;
             if (PV) sm.credit[k * 32 + lane] = 0;
         }
@@ -1086,11 +1108,11 @@ __device__ __forceinline__ bool has_core(const Data &w)
 }
 
 template <bool PV, bool BATCH>
-__global__ void __launch_bounds__(kThreads, 5)
+__global__ void __launch_bounds__(kThreads, 4)
 core_kernel(const Data w, bool do_wide, bool do_short, int batch)
 {
     __shared__ CoreSmem sm;
-    if (!has_core<BATCH>(w)) return;
+    if (gated(w) || !has_core<BATCH>(w)) return;
     unsigned long long tri = 0;
     if (do_wide) core_wide_rows<PV, BATCH>(w, sm, tri);
     if (do_short)
@@ -1105,6 +1127,7 @@ __global__ void __launch_bounds__(kThreads, 5)
 list_kernel(const Data w, bool do_wide, bool do_short, int batch)
 {
     extern __shared__ __align__(16) unsigned char smem[];
+    if (gated(w)) return;
     ListSmem<Pos> &sm = *reinterpret_cast<ListSmem<Pos> *>(smem);
     unsigned long long tri = 0;
     if (do_wide && w.ctr->wide_rows > 0) {
@@ -1126,6 +1149,7 @@ __global__ void __launch_bounds__(kThreads, 4)
 count_kernel(const Data w, int batch)
 {
     extern __shared__ __align__(16) unsigned char smem[];
+    if (gated(w)) return;
     union Smem {
         ListSmem<Pos> list;
         CoreSmem core;

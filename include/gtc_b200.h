@@ -215,6 +215,24 @@ gtc_status gtc_count_subset(const void *d_off, int off_bits,
                             gtc_stream_t stream);
 
 /*
+ * gtc_count_subset for a graph whose size is known, with a workspace.  A
+ * large subset of a skewed graph costs more than a count of the whole graph
+ * (65,536 of R-MAT scale 20's vertices ten times as much), so an estimate on
+ * the device picks the cheaper of the two; the result is the same.
+ * gtc_subset_workspace_size writes 0 when a count of the whole graph is never
+ * the cheaper way (few listed vertices); with no or too little workspace the
+ * call is gtc_count_subset.  d_workspace is 256-byte aligned.  Asynchronous on
+ * `stream`.
+ */
+gtc_status gtc_subset_workspace_size(int64_t n, int64_t nnz, int off_bits,
+                                     int64_t count, size_t *bytes);
+gtc_status gtc_count_subset_ws(const void *d_off, int off_bits,
+                               const int32_t *d_ind, int64_t n, int64_t nnz,
+                               const int32_t *d_vertex, int64_t count,
+                               int64_t *d_out, void *d_workspace,
+                               size_t ws_bytes, gtc_stream_t stream);
+
+/*
  * Batched counting: many independent graphs in one pipeline run (no
  * counterpart in the reference, whose host path counts one graph per
  * kernelCall, src/gpurun.cu:2-56).
