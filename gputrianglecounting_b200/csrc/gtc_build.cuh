@@ -435,8 +435,11 @@ __device__ __forceinline__ void split_rows(const View<OffT> &w, long long u0, in
             len = half;
         }
     }
-    // a row with an id out of range has no list
-    row_record(w, v, lo, bad || e <= lo ? 0 : (int)(e - lo), 0, kShortListIds, listed);
+    // ids above the range are the last ones of an ascending row
+    if (bad)
+        for (long long i = lo; i < e; ++i)
+            if ((unsigned int)w.ind[i] >= nv) e = i;
+    row_record(w, v, lo, e > lo ? (int)(e - lo) : 0, 0, kShortListIds, listed);
 }
 
 // Rows u0 .. u0 + 31 of other graphs that are not long rows.

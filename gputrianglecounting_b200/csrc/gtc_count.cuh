@@ -567,36 +567,33 @@ constexpr int kNoProbe = INT32_MIN + 1;           // never a list element nor kN
 // A tile: consecutive short rows with at most kTileEdges members in all, of
 // which at most kTileIds are distinct.
 constexpr int kTileEdges = 192, kTileIds = 96, kTileWords = kTileIds / 32;
-constexpr int kTileSlots = 1024;
+constexpr int kTileSlots = 2048;
 constexpr int kTileLong = 32;                     // longer lists are taken by the whole warp
-constexpr unsigned short kNoEdge = 0xffff;
+constexpr int kNoId = 0xff, kClaimed = 0x80;      // a slot that is empty, that a lane claims
 
 template <typename Pos>
 struct __align__(16) TileSmem {
-    unsigned short slot[kTileSlots];              // first edge whose member hashes here
+    unsigned char slot[kTileSlots];               // number of the member that hashes here
     unsigned int adj[kTileWords][kTileIds];       // adjacency among the tile's distinct members
-    union {
-        Pos start[kTileIds];                      // a streamed list's begin, less its elements before
-        unsigned int rowbits[kTileWords][32];     // a row's members
-    };
+    unsigned int rowbits[kTileWords][32];         // a row's members
+    Pos start[kTileIds];                          // a streamed list's begin, less its elements before
     union {
         unsigned int begins[kTileIds];            // bit f: a list begins at element f of the stream
         unsigned int credit[kTileIds];
     };
-    int member[kTileEdges];                       // an edge's member
-    unsigned char same[kTileEdges];               // ... the first edge with that member
-    unsigned char row[kTileEdges];                // ... its row
-    unsigned char num[kTileEdges];                // ... its member's number
-    unsigned char first[kTileIds];                // first edge of a number
+    int member[kTileIds];                         // a number's member
+    unsigned short edge[kTileEdges];              // the number of an edge's member, its row << 8
     unsigned char owner[kTileIds];                // number whose list is the k-th of the stream
+    unsigned char from[32];                       // lane of the k-th row that takes part
 };
 static_assert(kTileLong * kTileIds <= 32 * kTileIds, "begins holds a bit per streamed element");
+static_assert(kTileIds <= kClaimed, "numbers and claims share a byte");
 
 // Empties a warp's table; every tile leaves it empty again.
 template <typename Pos>
 __device__ __forceinline__ void tile_init(TileSmem<Pos> &sm)
 {
-    for (int k = threadIdx.x & 31; k < kTileSlots / 2; k += 32)
+    for (int k = threadIdx.x & 31; k < kTileSlots / 4; k += 32)
         reinterpret_cast<unsigned int *>(sm.slot)[k] = 0xffffffffu;
     __syncwarp();
 }
@@ -610,34 +607,46 @@ __device__ __forceinline__ void tile_init(TileSmem<Pos> &sm)
 // popc(members of p & neighbours of q) triangles: those in which q is the
 // middle and those in which it is the highest vertex, so that is q's credit,
 // and half a row's sum is p's.  The pairs of core members are not among them
-// (their lists are not looked up).  The table is a tenth full, so a look-up
-// that finds nothing mostly ends at its first slot.
+// (their lists are not looked up).  Shared-memory wavefronts bound it, so the
+// table is a twentieth full -- a look-up that finds nothing mostly ends at its
+// first slot -- and its bytes are the numbers themselves.
 template <bool PV, bool BATCH, typename Pos>
 __device__ __forceinline__ void
 tile_rows(const Data &w, long long u0, const VInfo &vi, int g, bool act, TileSmem<Pos> &sm,
           unsigned long long &tri)
 {
     constexpr int kPer = 4;
+    constexpr unsigned int kAll = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    const unsigned int below = (1u << lane) - 1u;
+    const unsigned int below = (1u << lane) - 1u, upto = below | (1u << lane);
     constexpr unsigned int kMask = kTileSlots - 1;
     constexpr int kLog = ilog2(kTileSlots);
-    const int fd = act ? vi.fdeg : 0;
-    const int incl = warp_incl_scan(fd);
-    const int total = __shfl_sync(0xffffffffu, incl, 31);
-    const Pos start = (Pos)vi.fbeg - (Pos)(incl - fd);
+    // the rows that take part, in the first lanes
+    const unsigned int acts = __ballot_sync(kAll, act);
+    const int rows = __popc(acts);
+    if (rows == 0) return;
+    __syncwarp();
+    if (act) sm.from[__popc(acts & below)] = (unsigned char)lane;
+    __syncwarp();
+    const int src = lane < rows ? sm.from[lane] : 0;
+    int fd = __shfl_sync(kAll, vi.fdeg, src);
+    if (lane >= rows) fd = 0;
+    const int incl = warp_incl_scan(fd), excl = incl - fd;
+    const int total = __shfl_sync(kAll, incl, 31);
+    const Pos start = __shfl_sync(kAll, (Pos)vi.fbeg, src) - (Pos)excl;
+    const int gr = BATCH ? __shfl_sync(kAll, g, src) : 0;
     for (int base = 0; base < total;) {
-        // rows that may join: one graph (core members are positions in it)
+        // rows r0 .. r1 - 1, r1 <= r2: one graph (core members are positions in it)
+        const int r0 = __popc(__ballot_sync(kAll, lane < rows && incl <= base));
         int stop = total;
         long long v0 = 0;
         const GraphRec *rec = w.recs;
         if (BATCH) {
-            const int f0 = __ffs(__ballot_sync(0xffffffffu, incl > base)) - 1;
-            const int gf = __shfl_sync(0xffffffffu, g, f0);
-            const unsigned int other = __ballot_sync(0xffffffffu, fd > 0 && lane > f0 && g != gf);
-            const int o = other ? __ffs(other) - 1 : 0;
-            const int excl = __shfl_sync(0xffffffffu, incl - fd, o);
-            if (other) stop = excl;
+            const int gf = __shfl_sync(kAll, gr, r0);
+            const unsigned int other =
+                __ballot_sync(kAll, lane < rows && lane > r0 && gr != gf);
+            const int at = __shfl_sync(kAll, excl, other ? __ffs(other) - 1 : 0);
+            if (other) stop = at;
             rec += gf;
             v0 = rec->v0;
         }
@@ -649,67 +658,93 @@ tile_rows(const Data &w, long long u0, const VInfo &vi, int g, bool act, TileSme
 #pragma unroll
             for (int j = 0; j < kTileIds / 32; ++j) sm.adj[k][j * 32 + lane] = 0;
             sm.begins[k * 32 + lane] = 0;
+            sm.rowbits[k][lane] = 0;
         }
+        __syncwarp();
         // number the members, 32 edges at a time while there is room
-        int n = 0, seen = 0;
+        int n = 0, seen = 0, row = r0 - 1;
         for (; seen < stop && n <= kTileIds - 32; seen += 32) {
-            const int e = seen + lane;
-            const int i = warp_corank(incl, base + e);
-            const Pos f = __shfl_sync(0xffffffffu, start, i);
-            const bool in = e < stop;
-            int m = 0;
-            if (in) {
-                m = ls.base[f + (Pos)(base + e)];
-                sm.member[e] = m;
-                sm.row[e] = (unsigned char)i;
-            }
-            __syncwarp();
-            bool won = false;
-            if (in) {
-                unsigned int h = hash_slot(m, kLog);
-                unsigned short old;
-                while (true) {
-                    old = atomicCAS(&sm.slot[h], kNoEdge, (unsigned short)e);
-                    won = old == kNoEdge;
-                    if (won || sm.member[old] == m) break;
-                    h = (h + 1) & kMask;
+            const int e = seen + lane, b = excl - base - seen;
+            const unsigned int heads =
+                __reduce_or_sync(kAll, lane < rows && b >= 0 && b < 32 ? 1u << b : 0u);
+            const int i = row + __popc(heads & upto);
+            row += __popc(heads);
+            const Pos f = __shfl_sync(kAll, start, i);
+            bool todo = e < stop;
+            const int m = todo ? ls.base[f + (Pos)(base + e)] : 0;
+            unsigned int h = hash_slot(m, kLog);
+            int id = 0;
+            while (__any_sync(kAll, todo)) {
+                const int x = todo ? sm.slot[h] : 0;
+                bool mine = false;
+                __syncwarp();                     // all have read before any claims
+                if (todo) {
+                    if (x == kNoId) {
+                        sm.slot[h] = (unsigned char)(kClaimed | lane);
+                        mine = true;
+                    } else if (sm.member[x] == m) {
+                        id = x;
+                        todo = false;
+                    } else {
+                        h = (h + 1) & kMask;
+                    }
                 }
-                sm.same[e] = (unsigned char)(won ? e : old);
+                __syncwarp();
+                // of the lanes that claim a slot one has it, those with the
+                // same member share its number, the others go on
+                const int by = mine ? sm.slot[h] & 31 : lane;
+                const bool won = mine && by == lane;
+                const unsigned int wm = __ballot_sync(kAll, won);
+                if (wm == 0) continue;
+                if (won) id = n + __popc(wm & below);
+                const int mb = __shfl_sync(kAll, m, by), ib = __shfl_sync(kAll, id, by);
+                if (mine) {
+                    if (mb == m) {
+                        id = ib;
+                        todo = false;
+                    } else {
+                        h = (h + 1) & kMask;
+                    }
+                }
+                if (won) {
+                    sm.slot[h] = (unsigned char)id;
+                    sm.member[id] = m;
+                }
+                n += __popc(wm);
+                __syncwarp();
             }
-            const unsigned int wm = __ballot_sync(0xffffffffu, won);
-            if (won) {
-                const int id = n + __popc(wm & below);
-                sm.num[e] = (unsigned char)id;
-                sm.first[id] = (unsigned char)e;
+            if (e < stop) {
+                sm.edge[e] = (unsigned short)(id | i << 8);
+                atomicOr(&sm.rowbits[id >> 5][i], 1u << (id & 31));
             }
-            n += __popc(wm);
         }
         seen = min(seen, stop);
         __syncwarp();
         // whole rows only: the edges of a cut row come again in the next tile
-        const int r1 = __popc(__ballot_sync(0xffffffffu, incl - base <= seen));
-        const int edges = __shfl_sync(0xffffffffu, incl, r1 - 1) - base;
-        // in[j] collects who points at number j
-        auto look = [&](unsigned int *in, unsigned int bit, int y) {
+        const int r1 = __popc(__ballot_sync(kAll, lane < rows && incl - base <= seen));
+        const int edges = __shfl_sync(kAll, incl, r1 - 1) - base;
+        // y is a list element of number id
+        auto look = [&](int y, auto &&owner) {
             unsigned int h = hash_slot(y, kLog);
-            unsigned short e = sm.slot[h];
-            while (e != kNoEdge) {
-                if (sm.member[e] == y) {
-                    atomicOr(&in[sm.num[e]], bit);
+            int x = sm.slot[h];
+            while (x != kNoId) {
+                if (sm.member[x] == y) {
+                    const int id = owner();
+                    atomicOr(&sm.adj[id >> 5][x], 1u << (id & 31));
                     break;
                 }
                 h = (h + 1) & kMask;
-                e = sm.slot[h];
+                x = sm.slot[h];
             }
         };
-        // the distinct members' lists: lay out the stream
-        int qlen[kTileIds / 32];
-        Pos qfb[kTileIds / 32];
+        // the lists of the members of the whole rows: lay out the stream
+        int qlen[kTileWords];
+        Pos qfb[kTileWords];
 #pragma unroll
-        for (int k = 0; k < kTileIds / 32; ++k) {
-            const int id = k * 32 + lane;
-            const int e = id < n ? sm.first[id] : edges;
-            const int x = e < edges ? sm.member[e] : -1;
+        for (int k = 0; k < kTileWords; ++k) {
+            const unsigned int used =
+                __reduce_or_sync(kAll, lane < r1 ? sm.rowbits[k][lane] : 0u);
+            const int x = (used >> lane) & 1u ? sm.member[k * 32 + lane] : -1;
             qlen[k] = 0;
             qfb[k] = 0;
             if (x >= 0) {
@@ -720,10 +755,10 @@ tile_rows(const Data &w, long long u0, const VInfo &vi, int g, bool act, TileSme
         }
         int lists = 0, elements = 0;
 #pragma unroll
-        for (int k = 0; k < kTileIds / 32; ++k) {
+        for (int k = 0; k < kTileWords; ++k) {
             const int len = qlen[k] <= kTileLong ? qlen[k] : 0;
             const int li = warp_incl_scan(len), le = elements + li - len;
-            const unsigned int have = __ballot_sync(0xffffffffu, len > 0);
+            const unsigned int have = __ballot_sync(kAll, len > 0);
             if (len > 0) {
                 const int o = lists + __popc(have & below);
                 sm.start[o] = qfb[k] - (Pos)le;
@@ -731,7 +766,7 @@ tile_rows(const Data &w, long long u0, const VInfo &vi, int g, bool act, TileSme
                 atomicOr(&sm.begins[le >> 5], 1u << (le & 31));
             }
             lists += __popc(have);
-            elements += __shfl_sync(0xffffffffu, li, 31);
+            elements += __shfl_sync(kAll, li, 31);
         }
         __syncwarp();
         // look its elements up, 128 at a time
@@ -742,31 +777,30 @@ tile_rows(const Data &w, long long u0, const VInfo &vi, int g, bool act, TileSme
             for (int j = 0; j < kPer; ++j) {
                 const int f = f0 + 32 * j + lane;
                 const unsigned int word = f0 + 32 * j < elements ? sm.begins[(f0 >> 5) + j] : 0u;
-                o[j] = o0 + __popc(word & (below | (1u << lane)));
+                o[j] = o0 + __popc(word & upto);
                 o0 += __popc(word);
                 y[j] = f < elements ? ls.base[sm.start[o[j]] + (Pos)f] : kNoProbe;
             }
 #pragma unroll
             for (int j = 0; j < kPer; ++j) {
                 if (f0 + 32 * j >= elements) break;
-                const int id = sm.owner[o[j]];
-                look(sm.adj[id >> 5], 1u << (id & 31), y[j]);
+                look(y[j], [&] { return (int)sm.owner[o[j]]; });
             }
         }
         // the long lists, one by one
 #pragma unroll
-        for (int k = 0; k < kTileIds / 32; ++k) {
-            unsigned int longs = __ballot_sync(0xffffffffu, qlen[k] > kTileLong);
+        for (int k = 0; k < kTileWords; ++k) {
+            unsigned int longs = __ballot_sync(kAll, qlen[k] > kTileLong);
             while (longs) {
                 const int q = __ffs(longs) - 1;
                 longs &= longs - 1;
-                const int *list = ls.base + (long long)__shfl_sync(0xffffffffu, qfb[k], q);
-                const int ql = __shfl_sync(0xffffffffu, qlen[k], q);
+                const int *list = ls.base + (long long)__shfl_sync(kAll, qfb[k], q);
+                const int ql = __shfl_sync(kAll, qlen[k], q);
                 for (int j = lane; j < ql; j += 64) {
                     const int y0 = list[j];
                     const int y1 = j + 32 < ql ? list[j + 32] : kNoProbe;
-                    look(sm.adj[k], 1u << q, y0);
-                    if (y1 != kNoProbe) look(sm.adj[k], 1u << q, y1);
+                    look(y0, [&] { return k * 32 + q; });
+                    if (y1 != kNoProbe) look(y1, [&] { return k * 32 + q; });
                 }
                 __syncwarp();
             }
@@ -784,14 +818,7 @@ tile_rows(const Data &w, long long u0, const VInfo &vi, int g, bool act, TileSme
 #pragma unroll
             for (int j = 0; j < kTileWords; ++j)
                 sm.adj[k][j * 32 + lane] = block[k][j] | tr(block[j][k]);
-            sm.rowbits[k][lane] = 0;
             if (PV) sm.credit[k * 32 + lane] = 0;
-        }
-        __syncwarp();
-        for (int e = lane; e < edges; e += 32) {
-            const int id = sm.num[sm.same[e]];
-            sm.num[e] = (unsigned char)id;
-            atomicOr(&sm.rowbits[id >> 5][sm.row[e]], 1u << (id & 31));
         }
         __syncwarp();
         // count
@@ -800,7 +827,7 @@ tile_rows(const Data &w, long long u0, const VInfo &vi, int g, bool act, TileSme
             const int e = e0 + lane;
             unsigned int c = 0;
             if (e < edges) {
-                const int id = sm.num[e], r = sm.row[e];
+                const int id = sm.edge[e] & 0xff, r = sm.edge[e] >> 8;
 #pragma unroll
                 for (int k = 0; k < kTileWords; ++k)
                     c += __popc(sm.rowbits[k][r] & sm.adj[k][id]);
@@ -810,9 +837,9 @@ tile_rows(const Data &w, long long u0, const VInfo &vi, int g, bool act, TileSme
                 // a row's edges are consecutive: its lane takes a difference
                 // of prefix sums
                 const int ps = warp_incl_scan((int)c);
-                const int lo = max(incl - fd - base - e0, 0), hi = min(incl - base - e0, 32);
-                const int top = __shfl_sync(0xffffffffu, ps, (hi - 1) & 31);
-                const int bot = __shfl_sync(0xffffffffu, ps, (lo - 1) & 31);
+                const int lo = max(excl - base - e0, 0), hi = min(incl - base - e0, 32);
+                const int top = __shfl_sync(kAll, ps, (hi - 1) & 31);
+                const int bot = __shfl_sync(kAll, ps, (lo - 1) & 31);
                 if (hi > lo) sum += (unsigned int)(top - (lo > 0 ? bot : 0));
             } else {
                 sum += c;
@@ -821,21 +848,21 @@ tile_rows(const Data &w, long long u0, const VInfo &vi, int g, bool act, TileSme
         __syncwarp();
         if (PV) {
             sum >>= 1;
-            if (sum) add64(&w.tacc[u0 + lane], sum);
+            if (sum) add64(&w.tacc[u0 + src], sum);
             tri += sum;
         } else {
             sum = warp_sum(sum) >> 1;
             tri += lane == 0 ? sum : 0u;
         }
         for (int id = lane; id < n; id += 32) {
-            const int e = sm.first[id], m = sm.member[e];
+            const int m = sm.member[id];
             if (PV) {
                 const unsigned int c = sm.credit[id];
                 if (c) credit(w, v0, ls.shift, m, c);
             }
             unsigned int h = hash_slot(m, kLog);
-            while (sm.slot[h] != (unsigned short)e) h = (h + 1) & kMask;
-            sm.slot[h] = kNoEdge;
+            while (sm.slot[h] != id) h = (h + 1) & kMask;
+            sm.slot[h] = (unsigned char)kNoId;
         }
         base += edges;
     }
