@@ -498,9 +498,67 @@ __device__ __forceinline__ void core_wide_rows(const Data &w, CoreSmem &sm,
         });
 }
 
-// Up to 32 consecutive rows by a warp, one after another: a lane per member of
-// the row (at most kShortList), every core member q in turn broadcast to the
-// members above it.
+// Short rows of at most W members, 32 / W at a time, W lanes each: a lane per
+// member, every core member q of a row in turn tested against the core members
+// above it, four q in flight.
+template <int W, bool PV, bool BATCH>
+__device__ __forceinline__ void core_rows(const Data &w, long long u0, const VInfo &vi, int g,
+                                          unsigned int rows, unsigned long long &tri)
+{
+    constexpr int kGroups = 32 / W;
+    const int lane = threadIdx.x & 31, grp = lane / W, gl = lane % W, g0 = grp * W;
+    const unsigned int gmask = (W == 32 ? 0xffffffffu : (1u << W) - 1u) << g0;
+    while (rows) {
+        int r = -1;
+#pragma unroll
+        for (int k = 0; k < kGroups; ++k) {
+            if (k == grp && rows) r = __ffs(rows) - 1;
+            rows &= rows - 1;
+        }
+        const long long fb = __shfl_sync(0xffffffffu, vi.fbeg, r & 31);
+        const int fd = __shfl_sync(0xffffffffu, vi.fdeg, r & 31);
+        const int m = r >= 0 && gl < fd ? w.find[fb + gl] : 0;
+        const bool core = m < 0;
+        const int pos = ~m;
+        const int rb = core ? u_row(pos) : INT32_MAX;   // ascending with the position
+        const unsigned int *up = w.u + (core ? pos >> 5 : 0);
+        long long v0 = 0;
+        if (BATCH) {
+            const GraphRec *rec = &w.recs[__shfl_sync(0xffffffffu, g, r & 31)];
+            up += rec->ubase;
+            v0 = rec->v0;
+        }
+        unsigned int qm = __ballot_sync(0xffffffffu, core) & gmask;
+        unsigned int cq = 0, cs = 0;
+        while (__any_sync(0xffffffffu, qm != 0)) {
+            int q[4];
+            unsigned int x[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                q[j] = __ffs(qm) - 1;
+                qm &= qm - 1;
+                const int rq = __shfl_sync(0xffffffffu, rb, q[j] & 31);
+                x[j] = q[j] >= 0 && rb < rq ? __ldg(up + rq) : 0u;
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const bool hit = (x[j] >> (pos & 31)) & 1u;
+                const unsigned int h = __ballot_sync(0xffffffffu, hit) & gmask;
+                cs += hit;
+                if (lane == q[j]) cq += __popc(h);
+            }
+        }
+        unsigned int tot = cq;
+#pragma unroll
+        for (int d = W / 2; d > 0; d >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, d);
+        if (PV) {
+            if (core && cq + cs) add64(&w.tcore[v0 + pos], cq + cs);
+            if (gl == 0 && tot) add64(&w.tacc[u0 + r], tot);
+        }
+        tri += gl == 0 ? tot : 0u;
+    }
+}
+
 template <bool PV, bool BATCH>
 __device__ __forceinline__ void core_short_rows(const Data &w, long long u0, int batch,
                                                 unsigned long long &tri)
@@ -512,52 +570,13 @@ __device__ __forceinline__ void core_short_rows(const Data &w, long long u0, int
         vi = w.vinfo[u0 + lane];
         if (BATCH) g = w.gid[u0 + lane];
     }
-    unsigned int rows = __ballot_sync(0xffffffffu, vi.dk >= 2);   // not a wide row
-    while (rows) {
-        const int r = __ffs(rows) - 1;
-        rows &= rows - 1;
-        const long long fb = __shfl_sync(0xffffffffu, vi.fbeg, r);
-        const int fd = __shfl_sync(0xffffffffu, vi.fdeg, r);
-        const int m = lane < fd ? w.find[fb + lane] : 0;
-        const bool core = m < 0;
-        const int pos = ~m;
-        const int rb = core ? u_row(pos) : INT32_MAX;   // ascending with the position
-        const unsigned int *up = w.u + (core ? pos >> 5 : 0);
-        long long v0 = 0;
-        if (BATCH) {
-            const GraphRec *rec = &w.recs[__shfl_sync(0xffffffffu, g, r)];
-            up += rec->ubase;
-            v0 = rec->v0;
-        }
-        unsigned int qm = __ballot_sync(0xffffffffu, core);
-        unsigned int cq = 0, cs = 0;
-        while (qm) {
-            int q[4];
-            unsigned int x[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                q[j] = qm ? __ffs(qm) - 1 : -1;
-                qm &= qm - 1;
-                const int rq = __shfl_sync(0xffffffffu, rb, q[j] & 31);
-                x[j] = (q[j] >= 0 && rb < rq) ? __ldg(up + rq) : 0u;
-            }
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const bool hit = (x[j] >> (pos & 31)) & 1u;
-                const unsigned int h = __ballot_sync(0xffffffffu, hit);
-                cs += hit;
-                if (lane == q[j]) cq += __popc(h);
-            }
-        }
-        const unsigned int tot = warp_sum(cq);
-        if (tot) {
-            if (PV) {
-                if (core && cq + cs) add64(&w.tcore[v0 + pos], cq + cs);
-                if (lane == 0) add64(&w.tacc[u0 + r], tot);
-            }
-            tri += lane == 0 ? tot : 0u;
-        }
-    }
+    const bool act = vi.dk >= 2;                  // not a wide row
+    const unsigned int narrow = __ballot_sync(0xffffffffu, act && vi.fdeg <= 8);
+    const unsigned int mid = __ballot_sync(0xffffffffu, act && vi.fdeg > 8 && vi.fdeg <= 16);
+    const unsigned int full = __ballot_sync(0xffffffffu, act && vi.fdeg > 16);
+    if (narrow) core_rows<8, PV, BATCH>(w, u0, vi, g, narrow, tri);
+    if (mid) core_rows<16, PV, BATCH>(w, u0, vi, g, mid, tri);
+    if (full) core_rows<32, PV, BATCH>(w, u0, vi, g, full, tri);
 }
 
 // ====================================================== other members (lists)
