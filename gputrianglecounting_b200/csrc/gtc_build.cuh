@@ -139,6 +139,63 @@ __device__ __forceinline__ void choose_core(unsigned int *hist, int dmin, int kc
     uniform = !s_any;
 }
 
+// Whether a uniform graph's rows get signatures (one block): where they fit in
+// the graph's part of find, which such a graph leaves unused, and less than a
+// quarter of sampled pairs of neighbours are neighbours themselves.  A pair
+// that the signature lets pass is searched for, so signatures pay where most
+// pairs are none (ER 900K, mean degree 30: SIGN_ER); on a mesh, where half of
+// the pairs are edges and tiles of rows share members, they do not (RGG 4M:
+// SIGN_RGG).
+template <typename OffT>
+__device__ __forceinline__ bool use_signatures(const View<OffT> &w, GraphRec &rec)
+{
+    constexpr int kPer = 4;                          // samples per warp, in flight together
+    __shared__ int s_seen, s_closed;
+    const long long first = (long long)w.off[rec.v0], last = (long long)w.off[rec.v0 + rec.nv];
+    const long long base = div_up<long long>(first, kSigWords) * kSigWords;
+    if (w.n < kSignedCall || rec.nv < kSignedGraph ||
+        base + (long long)kSigWords * rec.nv > last)
+        return false;
+    if (threadIdx.x == 0) s_seen = s_closed = 0;
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    long long b[kPer], d[kPer];
+    int y[kPer];
+    unsigned int h[kPer];
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+        h[j] = (unsigned int)((threadIdx.x >> 5) * kPer + j + 1) * 0x9E3779B1u;
+        const long long v = rec.v0 + (((unsigned long long)h[j] * (unsigned int)rec.nv) >> 32);
+        b[j] = (long long)w.off[v];
+        d[j] = (long long)w.off[v + 1] - b[j];
+    }
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+        const bool pair = d[j] >= 2;
+        const unsigned int i = pair ? h[j] % (unsigned int)(d[j] - 1) : 0u;
+        const unsigned int k = pair ? i + 1 + (h[j] >> 7) % (unsigned int)(d[j] - 1 - i) : 0u;
+        const int x = pair ? w.ind[b[j] + i] : -1;
+        y[j] = pair ? w.ind[b[j] + k] : -1;
+        const bool in = (unsigned int)x < (unsigned int)rec.nv;
+        b[j] = in ? (long long)w.off[rec.v0 + x] : 0;
+        d[j] = in ? (long long)w.off[rec.v0 + x + 1] - b[j] : -1;
+    }
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+        bool hit = false;
+        for (long long i = lane; i < d[j]; i += 32) hit |= w.ind[b[j] + i] == y[j];
+        hit = __any_sync(0xffffffffu, hit);
+        if (lane == 0 && d[j] >= 0) {
+            atomicAdd(&s_seen, 1);
+            if (hit) atomicAdd(&s_closed, 1);
+        }
+    }
+    __syncthreads();
+    const bool yes = 4 * s_closed < s_seen;
+    if (yes) rec.ubase = base;
+    return yes;
+}
+
 // Long row i of the wide list: its record, its placement items and, for a
 // core vertex, its key.
 template <typename OffT>
@@ -170,7 +227,7 @@ __device__ __forceinline__ void key_row(const View<OffT> &w, long long i)
 // finish chooses the core, which saves a launch; with `ids` (batch) the graph
 // ids and limits are found here too.
 template <typename OffT, bool BATCH>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 8)
 degree_kernel(const View<OffT> w, GraphRec lim, bool ids, bool choose)
 {
     if (gated(w)) return;
@@ -213,7 +270,7 @@ degree_kernel(const View<OffT> w, GraphRec lim, bool ids, bool choose)
             if (lng) w.wide[at + __popc(m & ((1u << lane) - 1u))] = (int)v;
         }
     }
-    if (!choose) return;
+    if (BATCH || !choose) return;
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) s_last = atomicAdd(&w.ctr->blocks_done, 1u) == gridDim.x - 1;
@@ -221,6 +278,7 @@ degree_kernel(const View<OffT> w, GraphRec lim, bool ids, bool choose)
     if (!s_last) return;
     __threadfence();
     choose_core(w.hist, lim.dmin, lim.kcap, lim.min_bucket, lim.core, lim.uniform);
+    if (lim.uniform && use_signatures(w, lim)) lim.uniform = kSigned;
     if (threadIdx.x == 0) w.recs[0] = lim;
 }
 
@@ -233,6 +291,7 @@ choose_core_kernel(const View<OffT> w, GraphRec lim, bool limits)
     if (BATCH) lim = limits ? batch_limits(w, g) : w.recs[g];
     int min_bucket = 0, core = 0, uniform = 0;
     choose_core(w.hist + g * kBuckets, lim.dmin, lim.kcap, min_bucket, core, uniform);
+    if (uniform && use_signatures(w, lim)) uniform = kSigned;
     if (threadIdx.x == 0) {
         lim.uniform = uniform;
         lim.min_bucket = min_bucket;
@@ -383,18 +442,26 @@ __device__ __forceinline__ void row_record(const Data &w, long long v, long long
     w.vinfo[v] = VInfo{fbeg, fdeg, dk};
 }
 
+// The signatures of 32 rows, a lane each: bits[word][lane].
+typedef unsigned int SignSmem[kSigWords][32];
+
 // Those of rows u0 .. u0 + 31 that are of uniform graphs (mine): where the ids
-// above the row's own begin.
+// above the row's own begin, and the signature of those ids.
 template <typename OffT, bool BATCH>
-__device__ __forceinline__ void split_rows(const View<OffT> &w, long long u0, int g, bool mine)
+__device__ __forceinline__ void split_rows(const View<OffT> &w, long long u0, int g, bool mine,
+                                           SignSmem &bits)
 {
     const int lane = threadIdx.x & 31;
     const long long v = u0 + lane;
     long long b = 0, e = 0;
     int vl = 0, long_min = 0;
     unsigned int nv = 0;
+    unsigned int *sign = nullptr;
     if (mine) {
         const GraphRec *rec = &w.recs[g];
+        if (rec->uniform == kSigned)
+            sign = reinterpret_cast<unsigned int *>(w.find) + rec->ubase +
+                   kSigWords * (v - (BATCH ? rec->v0 : 0));
         b = (long long)w.off[v];
         e = (long long)w.off[v + 1];
         nv = BATCH ? (unsigned int)rec->nv : (unsigned int)w.n;
@@ -425,7 +492,13 @@ __device__ __forceinline__ void split_rows(const View<OffT> &w, long long u0, in
     if (!mine) return;
     const bool listed = (int)(e - b) > long_min;
     long long lo = b;
-    int len = (int)(e - b);
+    if (bad) {
+        // ids out of range are first or last in the row
+        while (lo < e && !((unsigned int)w.ind[lo] < nv && w.ind[lo] > vl)) ++lo;
+        for (long long i = lo; i < e; ++i)
+            if ((unsigned int)w.ind[i] >= nv) e = i;
+    }
+    int len = bad ? 0 : (int)(e - b);
     while (len > 0) {
         const int half = len >> 1;
         if (w.ind[lo + half] <= vl) {
@@ -435,11 +508,25 @@ __device__ __forceinline__ void split_rows(const View<OffT> &w, long long u0, in
             len = half;
         }
     }
-    // ids above the range are the last ones of an ascending row
-    if (bad)
-        for (long long i = lo; i < e; ++i)
-            if ((unsigned int)w.ind[i] >= nv) e = i;
     row_record(w, v, lo, e > lo ? (int)(e - lo) : 0, 0, kShortListIds, listed);
+    if (!sign) return;
+#pragma unroll
+    for (int k = 0; k < kSigWords; ++k) bits[k][lane] = 0;
+    const int *list = w.ind + lo;
+    const int n = (int)(e - lo);
+    for (int i = 0; i < n; i += 4) {
+        int y[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) y[j] = list[min(i + j, n - 1)];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const Sign x = sign_of(y[j]);
+            bits[x.word][lane] |= x.bits;
+        }
+    }
+    uint4 *to = reinterpret_cast<uint4 *>(sign);
+    to[0] = make_uint4(bits[0][lane], bits[1][lane], bits[2][lane], bits[3][lane]);
+    to[1] = make_uint4(bits[4][lane], bits[5][lane], bits[6][lane], bits[7][lane]);
 }
 
 // Rows u0 .. u0 + 31 of other graphs that are not long rows.
@@ -517,9 +604,10 @@ __device__ __forceinline__ void stream_rows(const View<OffT> &w, long long u0, i
 }
 
 template <typename OffT, bool BATCH>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 5)
 place_kernel(const View<OffT> w, bool do_wide, bool do_short)
 {
+    __shared__ SignSmem s_sign[kThreads / 32];
     if (gated(w)) return;
     const int lane = threadIdx.x & 31;
     const long long warps = (long long)gridDim.x * (kThreads / 32);
@@ -534,7 +622,8 @@ place_kernel(const View<OffT> w, bool do_wide, bool do_short)
     while (u0 < w.n) {
         const int g = BATCH && u0 + lane < w.n ? w.gid[u0 + lane] : 0;
         const bool in = u0 + lane < w.n, uniform = in && w.recs[g].uniform;
-        if (__any_sync(0xffffffffu, uniform)) split_rows<OffT, BATCH>(w, u0, g, uniform);
+        if (__any_sync(0xffffffffu, uniform))
+            split_rows<OffT, BATCH>(w, u0, g, uniform, s_sign[threadIdx.x >> 5]);
         if (__any_sync(0xffffffffu, in && !uniform)) stream_rows<OffT, BATCH>(w, u0, g);
         if (warps * 32 >= w.n) break;
         if (lane == 0) u0 = 32 * (warps + (long long)atomicAdd(&w.ctr->place_next, 1ull));

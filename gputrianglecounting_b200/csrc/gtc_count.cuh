@@ -3,6 +3,7 @@
 // epilogue.
 #pragma once
 
+#include <cuda_pipeline.h>
 #include <type_traits>
 
 #include "gtc_build.cuh"
@@ -590,9 +591,18 @@ constexpr int kTileSlots = 2048;
 constexpr int kTileLong = 32;                     // longer lists are taken by the whole warp
 constexpr int kNoId = 0xff, kClaimed = 0x80;      // a slot that is empty, that a lane claims
 
+// Of SignedRows: rows' members, their signatures, pairs to search for.
+constexpr int kPairs = 64;
+
+struct SignedSmem {
+    unsigned int sign[2][kSigWords * 35];         // 32 signatures and a gap between four groups
+    int member[2][32];
+    int q[kPairs], s[kPairs];
+    unsigned char row[kPairs];
+};
+
 template <typename Pos>
-struct __align__(16) TileSmem {
-    unsigned char slot[kTileSlots];               // number of the member that hashes here
+struct TileData {
     unsigned int adj[kTileWords][kTileIds];       // adjacency among the tile's distinct members
     unsigned int rowbits[kTileWords][32];         // a row's members
     Pos start[kTileIds];                          // a streamed list's begin, less its elements before
@@ -604,6 +614,15 @@ struct __align__(16) TileSmem {
     unsigned short edge[kTileEdges];              // the number of an edge's member, its row << 8
     unsigned char owner[kTileIds];                // number whose list is the k-th of the stream
     unsigned char from[32];                       // lane of the k-th row that takes part
+};
+
+template <typename Pos>
+struct __align__(16) TileSmem {
+    unsigned char slot[kTileSlots];               // number of the member that hashes here
+    union {
+        TileData<Pos> tile;
+        SignedSmem sign;
+    };
 };
 static_assert(kTileLong * kTileIds <= 32 * kTileIds, "begins holds a bit per streamed element");
 static_assert(kTileIds <= kClaimed, "numbers and claims share a byte");
@@ -631,9 +650,11 @@ __device__ __forceinline__ void tile_init(TileSmem<Pos> &sm)
 // first slot -- and its bytes are the numbers themselves.
 template <bool PV, bool BATCH, typename Pos>
 __device__ __forceinline__ void
-tile_rows(const Data &w, long long u0, const VInfo &vi, int g, bool act, TileSmem<Pos> &sm,
+tile_rows(const Data &w, long long u0, const VInfo &vi, int g, bool act, TileSmem<Pos> &smem,
           unsigned long long &tri)
 {
+    TileData<Pos> &sm = smem.tile;
+    unsigned char *const slot = smem.slot;
     constexpr int kPer = 4;
     constexpr unsigned int kAll = 0xffffffffu;
     const int lane = threadIdx.x & 31;
@@ -694,12 +715,12 @@ tile_rows(const Data &w, long long u0, const VInfo &vi, int g, bool act, TileSme
             unsigned int h = hash_slot(m, kLog);
             int id = 0;
             while (__any_sync(kAll, todo)) {
-                const int x = todo ? sm.slot[h] : 0;
+                const int x = todo ? slot[h] : 0;
                 bool mine = false;
                 __syncwarp();                     // all have read before any claims
                 if (todo) {
                     if (x == kNoId) {
-                        sm.slot[h] = (unsigned char)(kClaimed | lane);
+                        slot[h] = (unsigned char)(kClaimed | lane);
                         mine = true;
                     } else if (sm.member[x] == m) {
                         id = x;
@@ -711,7 +732,7 @@ tile_rows(const Data &w, long long u0, const VInfo &vi, int g, bool act, TileSme
                 __syncwarp();
                 // of the lanes that claim a slot one has it, those with the
                 // same member share its number, the others go on
-                const int by = mine ? sm.slot[h] & 31 : lane;
+                const int by = mine ? slot[h] & 31 : lane;
                 const bool won = mine && by == lane;
                 const unsigned int wm = __ballot_sync(kAll, won);
                 if (wm == 0) continue;
@@ -726,7 +747,7 @@ tile_rows(const Data &w, long long u0, const VInfo &vi, int g, bool act, TileSme
                     }
                 }
                 if (won) {
-                    sm.slot[h] = (unsigned char)id;
+                    slot[h] = (unsigned char)id;
                     sm.member[id] = m;
                 }
                 n += __popc(wm);
@@ -745,7 +766,7 @@ tile_rows(const Data &w, long long u0, const VInfo &vi, int g, bool act, TileSme
         // y is a list element of number id
         auto look = [&](int y, auto &&owner) {
             unsigned int h = hash_slot(y, kLog);
-            int x = sm.slot[h];
+            int x = slot[h];
             while (x != kNoId) {
                 if (sm.member[x] == y) {
                     const int id = owner();
@@ -753,7 +774,7 @@ tile_rows(const Data &w, long long u0, const VInfo &vi, int g, bool act, TileSme
                     break;
                 }
                 h = (h + 1) & kMask;
-                x = sm.slot[h];
+                x = slot[h];
             }
         };
         // the lists of the members of the whole rows: lay out the stream
@@ -880,12 +901,199 @@ tile_rows(const Data &w, long long u0, const VInfo &vi, int g, bool act, TileSme
                 if (c) credit(w, v0, ls.shift, m, c);
             }
             unsigned int h = hash_slot(m, kLog);
-            while (sm.slot[h] != id) h = (h + 1) & kMask;
-            sm.slot[h] = (unsigned char)kNoId;
+            while (slot[h] != id) h = (h + 1) & kMask;
+            slot[h] = (unsigned char)kNoId;
         }
         base += edges;
     }
 }
+
+// Rows of a graph with signatures.  A pair (q, s) of a row's members, q < s,
+// is an edge only if q's signature has s's bits.  W lanes per row, a member s
+// each: the members' signatures are put side by side, and a lane reads its word
+// of each in turn -- a warp's reads lie in eight neighbouring banks, one
+// wavefront per step.  Pairs that pass are queued and searched for 32 at a time.
+template <bool PV, bool BATCH, typename Pos>
+struct SignedRows {
+    const Data &w;
+    SignedSmem &sm;
+    const long long u0;
+    const VInfo &vi;
+    const int g, lane;
+    int queued;
+    unsigned long long tri;
+
+    // the last n (at most 32) queued pairs: s looked for in q's list
+    __device__ __forceinline__ void search(int n)
+    {
+        __syncwarp();
+        const int at = queued - n + lane;
+        const int r = lane < n ? sm.row[at] : 0;
+        const int v0 = BATCH ? (int)w.recs[__shfl_sync(0xffffffffu, g, r)].v0 : 0;
+        if (lane < n) {
+            const int q = sm.q[at], s = sm.s[at];
+            const VInfo qi = w.vinfo[q + v0];
+            const int *list = w.ind + qi.fbeg;
+            int lo = 0, len = qi.fdeg;
+            while (len > 0) {                     // first element that is not below s
+                const int half = len >> 1;
+                if (list[lo + half] < s) {
+                    lo += half + 1;
+                    len -= half + 1;
+                } else {
+                    len = half;
+                }
+            }
+            if (lo < qi.fdeg && list[lo] == s) {
+                ++tri;
+                if (PV) {
+                    add64(&w.tacc[u0 + r], 1u);
+                    add64(&w.tacc[q + v0], 1u);
+                    add64(&w.tacc[s + v0], 1u);
+                }
+            }
+        }
+        queued -= n;
+        __syncwarp();
+    }
+    // bit k of hits: the pair of member k of the row, whose members are from
+    // member[0] on, and this lane's member s passed
+    __device__ __forceinline__ void queue(unsigned int hits, const int *member, int s, int r)
+    {
+        while (true) {
+            const unsigned int have = __ballot_sync(0xffffffffu, hits != 0);
+            if (have == 0) return;
+            if (hits) {
+                const int at = queued + __popc(have & ((1u << lane) - 1u));
+                sm.q[at] = member[__ffs(hits) - 1];
+                sm.s[at] = s;
+                sm.row[at] = (unsigned char)r;
+                hits &= hits - 1;
+            }
+            queued += __popc(have);
+            if (queued >= 32) search(32);
+        }
+    }
+    // bit k of the result: whether signature k, k = 0 .. steps - 1, of sign has
+    // y's bits (readable up to the next multiple of 8)
+    __device__ __forceinline__ unsigned int column(const unsigned int *sign, int y, int steps) const
+    {
+        const Sign m = sign_of(y);
+        const unsigned int *x = sign + m.word;
+        unsigned int hb = 0;
+        int i = 0;
+        for (; i < steps; i += 8, x += 8 * kSigWords) {
+            unsigned int v[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = x[kSigWords * j];
+#pragma unroll
+            for (int j = 0; j < 8; ++j)           // bits missing: none has the top bit
+                hb = __funnelshift_l((m.bits & ~v[j]) - 1u, hb, 1);
+        }
+        return i ? __brev(hb) >> (32 - i) : 0u;
+    }
+    // the lanes' members y of row r (in: there is one) and their signatures on
+    // their way to shared memory, two lanes per signature; groups of W lanes
+    // one signature apart, so that they read from banks of their own
+    template <int W>
+    __device__ __forceinline__ void fetch(int r, bool in, int y, int *member,
+                                          unsigned int *sign) const
+    {
+        const GraphRec *rec = &w.recs[BATCH ? __shfl_sync(0xffffffffu, g, r & 31) : 0];
+        const unsigned int at = (unsigned int)(rec->ubase / kSigWords) + (unsigned int)y;
+        const unsigned int ins = __ballot_sync(0xffffffffu, in);
+        member[lane] = y;
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int k = 16 * j + (lane >> 1), part = 4 * (lane & 1);
+            const unsigned int from = __shfl_sync(0xffffffffu, at, k);
+            if ((ins >> k) & 1u)
+                __pipeline_memcpy_async(sign + kSigWords * (k + k / W) + part,
+                                        w.find + (long long)kSigWords * from + part, 16);
+        }
+        __pipeline_commit();
+    }
+    // 32 / W rows at a time; the signatures of the next ones and the members of
+    // those after them are under way meanwhile
+    template <int W>
+    __device__ __forceinline__ void rows_of(unsigned int rows)
+    {
+        constexpr int kGroups = 32 / W;
+        const int grp = lane / W, gl = lane % W, g0 = grp * W;
+        struct Set {
+            int r, fd, y;
+        };
+        auto next = [&]() -> Set {
+            Set t{-1, 0, 0};
+#pragma unroll
+            for (int k = 0; k < kGroups; ++k) {
+                if (k == grp && rows) t.r = __ffs(rows) - 1;
+                rows &= rows - 1;
+            }
+            const long long fb = __shfl_sync(0xffffffffu, vi.fbeg, t.r & 31);
+            const int fd = __shfl_sync(0xffffffffu, vi.fdeg, t.r & 31);
+            if (t.r >= 0) t.fd = fd;
+            if (gl < t.fd) t.y = w.ind[fb + gl];
+            return t;
+        };
+        auto issue = [&](const Set &t, int b) {
+            fetch<W>(t.r, gl < t.fd, t.y, sm.member[b], sm.sign[b]);
+        };
+        if (rows == 0) return;
+        Set now = next(), then = next();
+        __syncwarp();
+        issue(now, 0);
+        for (int b = 0; __any_sync(0xffffffffu, now.r >= 0); b ^= 1) {
+            const Set after = next();
+            issue(then, b ^ 1);
+            __pipeline_wait_prior(1);
+            __syncwarp();
+            const int most = __reduce_max_sync(0xffffffffu, now.fd);
+            const unsigned int hits =
+                column(sm.sign[b] + kSigWords * (g0 + grp), now.y, most - 1);
+            queue(gl < now.fd ? hits & ((1u << gl) - 1u) : 0u, sm.member[b] + g0, now.y, now.r);
+            __syncwarp();
+            now = then;
+            then = after;
+        }
+        __pipeline_wait_prior(0);
+    }
+    // rows of 33 .. 64 members, two members s per lane
+    __device__ __forceinline__ void long_rows(unsigned int rows)
+    {
+        unsigned int *const sign = sm.sign[0];
+        while (rows) {
+            const int r = __ffs(rows) - 1;
+            rows &= rows - 1;
+            const long long fb = __shfl_sync(0xffffffffu, vi.fbeg, r);
+            const int fd = __shfl_sync(0xffffffffu, vi.fdeg, r);
+            const bool in = lane + 32 < fd;
+            const int y0 = w.ind[fb + lane], y1 = in ? w.ind[fb + 32 + lane] : 0;
+            __syncwarp();
+            fetch<32>(r, true, y0, sm.member[0], sign);
+            fetch<32>(r, in, y1, sm.member[1], sign + kSigWords * 32);
+            __pipeline_wait_prior(0);
+            __syncwarp();
+            const unsigned int below = (1u << lane) - 1u;
+            queue(column(sign, y0, 31) & below, sm.member[0], y0, r);
+            queue(in ? column(sign, y1, 32) : 0u, sm.member[0], y1, r);
+            const unsigned int hits = column(sign + kSigWords * 32, y1, fd - 33);
+            queue(in ? hits & below : 0u, sm.member[1], y1, r);
+        }
+    }
+    __device__ __forceinline__ void all(bool act)
+    {
+        const unsigned int r8 = __ballot_sync(0xffffffffu, act && vi.fdeg <= 8);
+        const unsigned int r16 = __ballot_sync(0xffffffffu, act && vi.fdeg > 8 && vi.fdeg <= 16);
+        const unsigned int r32 = __ballot_sync(0xffffffffu, act && vi.fdeg > 16 && vi.fdeg <= 32);
+        const unsigned int r64 = __ballot_sync(0xffffffffu, act && vi.fdeg > 32);
+        rows_of<8>(r8);
+        rows_of<16>(r16);
+        rows_of<32>(r32);
+        long_rows(r64);
+        if (queued) search(queued);
+    }
+};
 
 struct TableWarpSmem {
     int key[4 * kWarpTable];                      // kNoMember = empty
@@ -1105,9 +1313,11 @@ __device__ __forceinline__ void table_wide_rows(const Data &w, ListSmem<Pos> &sm
         });
 }
 
-template <bool PV, bool BATCH, typename Pos>
-__device__ __forceinline__ void list_short_rows(const Data &w, long long u0, int batch,
-                                                TileSmem<Pos> &sm, unsigned long long &tri)
+// Rows u0 .. u0 + batch - 1 that are short, those of graphs with signatures
+// (SIGN) and the others (TILE).
+template <bool PV, bool BATCH, bool TILE, bool SIGN, typename Pos>
+__device__ __forceinline__ void list_rows(const Data &w, long long u0, int batch,
+                                          TileSmem<Pos> &sm, unsigned long long &tri)
 {
     const int lane = threadIdx.x & 31;
     VInfo vi{0, 0, 0};
@@ -1118,7 +1328,13 @@ __device__ __forceinline__ void list_short_rows(const Data &w, long long u0, int
     }
     // not a wide row, at least one member outside the core and one more
     const bool act = vi.dk >= 0 && vi.fdeg >= 2 && vi.fdeg > vi.dk;
-    tile_rows<PV, BATCH, Pos>(w, u0, vi, g, act, sm, tri);
+    const bool sign = SIGN && act && (!TILE || w.recs[g].uniform == kSigned);
+    if (SIGN && __any_sync(0xffffffffu, sign)) {
+        SignedRows<PV, BATCH, Pos> rows{w, sm.sign, u0, vi, g, lane, 0, 0};
+        rows.all(sign);
+        tri += rows.tri;
+    }
+    if (TILE) tile_rows<PV, BATCH, Pos>(w, u0, vi, g, act && !sign, sm, tri);
 }
 
 // ================================================================== kernels
@@ -1145,6 +1361,26 @@ __device__ __forceinline__ void add_triangles(Counters *ctr, unsigned long long 
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) tri += __shfl_down_sync(0xffffffffu, tri, d);
     if ((threadIdx.x & 31) == 0 && tri) atomicAdd(&ctr->tri_total, tri);
+}
+
+// All short rows: rows(u0, ..) of list_rows, then also(u0).  A single graph is
+// all tiles or all signatures, each in a loop with registers of its own.
+template <bool PV, bool BATCH, typename Pos, class Also>
+__device__ __forceinline__ void list_short_rows(const Data &w, int batch, TileSmem<Pos> &sm,
+                                                unsigned long long &tri, const Also &also)
+{
+    unsigned long long *queue = &w.ctr->list_short_next;
+    if (!BATCH && w.recs[0].uniform == kSigned) {
+        warp_batches(queue, w.n, batch, [&](long long u0) {
+            list_rows<PV, BATCH, false, true, Pos>(w, u0, batch, sm, tri);
+        });
+        return;                                   // no core either
+    }
+    tile_init(sm);
+    warp_batches(queue, w.n, batch, [&](long long u0) {
+        list_rows<PV, BATCH, true, BATCH, Pos>(w, u0, batch, sm, tri);
+        also(u0);
+    });
 }
 
 template <bool BATCH>
@@ -1180,12 +1416,9 @@ list_kernel(const Data w, bool do_wide, bool do_short, int batch)
         table_wide_rows<PV, BATCH, Pos>(w, sm, tri);
         __syncthreads();
     }
-    if (do_short) {
-        tile_init(sm.tile[threadIdx.x >> 5]);
-        warp_batches(&w.ctr->list_short_next, w.n, batch, [&](long long u0) {
-            list_short_rows<PV, BATCH, Pos>(w, u0, batch, sm.tile[threadIdx.x >> 5], tri);
-        });
-    }
+    if (do_short)
+        list_short_rows<PV, BATCH, Pos>(w, batch, sm.tile[threadIdx.x >> 5], tri,
+                                        [](long long) {});
     add_triangles(w.ctr, tri);
 }
 
@@ -1209,11 +1442,10 @@ count_kernel(const Data w, int batch)
         table_wide_rows<PV, BATCH, Pos>(w, sm.list, tri);
         __syncthreads();
     }
-    tile_init(sm.list.tile[threadIdx.x >> 5]);
-    warp_batches(&w.ctr->list_short_next, w.n, batch, [&](long long u0) {
-        list_short_rows<PV, BATCH, Pos>(w, u0, batch, sm.list.tile[threadIdx.x >> 5], tri);
-        if (core) core_short_rows<PV, BATCH>(w, u0, batch, tri);
-    });
+    list_short_rows<PV, BATCH, Pos>(w, batch, sm.list.tile[threadIdx.x >> 5], tri,
+                                    [&](long long u0) {
+                                        if (core) core_short_rows<PV, BATCH>(w, u0, batch, tri);
+                                    });
     add_triangles(w.ctr, tri);
 }
 

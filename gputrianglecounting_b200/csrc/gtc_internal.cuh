@@ -60,17 +60,22 @@ struct __align__(16) VInfo {
     int dk;
 };
 
+// GraphRec::uniform of a graph whose rows have signatures (Sign).
+constexpr int kSigned = 2, kSigWords = 8;
+constexpr int kSignedGraph = 512;           // vertices of the smallest such graph,
+constexpr int kSignedCall = 32768;          // ... of the smallest call (all its graphs)
+
 // Per-graph record (one for a single graph, one per graph of a batch).
 struct GraphRec {
     long long v0 = 0;          // first vertex
-    long long ubase = 0;       // first word of the graph's bit matrix
+    long long ubase = 0;       // first word of the graph's bit matrix, or of its signatures in find
     int nv = 0;                // vertices
     int core = 0;              // core vertices K
     int min_bucket = kBuckets; // lowest degree bucket of the core
     int dmin = 0;              // lowest degree that may be core
     int long_min = 0;          // rows longer than this are placed by blocks
     int kcap = 0;              // most core vertices (bit-matrix space)
-    int uniform = 0;           // no vertex of core degree: rows ordered by id
+    int uniform = 0;           // no vertex of core degree: rows ordered by id; kSigned too
 };
 
 // Counters block in the workspace (device, zeroed at the start of a count).
@@ -113,6 +118,22 @@ __host__ __device__ __forceinline__ int u_row(int pos)
 __device__ __forceinline__ unsigned int hash_slot(int key, int log2_slots)
 {
     return ((unsigned int)key * 0x9E3779B1u) >> (32 - log2_slots);
+}
+
+// What a member sets in its row's signature: three bits of one word, one in
+// each third of its low 30.  A row of 15 members lets one in a hundred ids pass
+// that are none of them; with one bit anywhere in the 256 it was one in 17.
+struct Sign {
+    int word;
+    unsigned int bits;
+};
+
+__device__ __forceinline__ Sign sign_of(int y)
+{
+    const unsigned int h = (unsigned int)y * 0x9E3779B1u;
+    const unsigned int a = (h >> 21 & 0xff) * 10 >> 8, b = (h >> 13 & 0xff) * 10 >> 8,
+                       c = (h >> 5 & 0xff) * 10 >> 8;
+    return {(int)(h >> 29), (1u << a) | (0x400u << b) | (0x100000u << c)};
 }
 
 __host__ __device__ __forceinline__ int ceil_log2(long long v)
