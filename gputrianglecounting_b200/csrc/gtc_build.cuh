@@ -141,11 +141,14 @@ __device__ __forceinline__ void choose_core(unsigned int *hist, int dmin, int kc
 
 // Whether a uniform graph's rows get signatures (one block): where they fit in
 // the graph's part of find, which such a graph leaves unused, and less than a
-// quarter of sampled pairs of neighbours are neighbours themselves.  A pair
+// twelfth of sampled pairs of neighbours are neighbours themselves.  A pair
 // that the signature lets pass is searched for, so signatures pay where most
-// pairs are none (ER 900K, mean degree 30: SIGN_ER); on a mesh, where half of
-// the pairs are edges and tiles of rows share members, they do not (RGG 4M:
-// SIGN_RGG).
+// pairs are none; where many are edges, tiles of rows share members and do
+// better.  Place and list kernels, signatures and tiles: 524K vertices of mean
+// degree 30, no closed pairs 180 and 324 us, 4% 232 and 325, 15% 398 and 295,
+// 58% 1124 and 201; of mean degree 16, 4% 112 and 151, 15% 151 and 138.  The
+// sample costs 5 us, which calls of few vertices do not earn back (ER 16K: list
+// kernel 14.7 -> 11.8 us, degree kernel 4.4 -> 8.6).
 template <typename OffT>
 __device__ __forceinline__ bool use_signatures(const View<OffT> &w, GraphRec &rec)
 {
@@ -191,7 +194,7 @@ __device__ __forceinline__ bool use_signatures(const View<OffT> &w, GraphRec &re
         }
     }
     __syncthreads();
-    const bool yes = 4 * s_closed < s_seen;
+    const bool yes = 12 * s_closed < s_seen;
     if (yes) rec.ubase = base;
     return yes;
 }

@@ -1098,11 +1098,13 @@ struct SignedRows {
 struct TableWarpSmem {
     int key[4 * kWarpTable];                      // kNoMember = empty
     unsigned int cnt[4 * kWarpTable];
+    unsigned int bits[kWarpTable];
 };
 
 struct TableBlockSmem {
     int key[1 << kTableLog2];
     unsigned int cnt[1 << kTableLog2];
+    unsigned int bits[1 << (kTableLog2 - 2)];
     int next;
     unsigned int total;
 };
@@ -1117,22 +1119,38 @@ struct ListSmem {
     WideClaim claim;
 };
 
-// Shared-memory table of a row's members: linear probing, a counter per slot.
+// Shared-memory table of a row's members: linear probing, a counter per slot,
+// and eight bits per slot of which a member sets the one that it hashes to.
+// Most look-ups find nothing; of 32 some always met a slot that was taken, and
+// the warp walked on for them.  With the bits one in 30 does.
 struct MemberTable {
     int *key;
-    unsigned int *cnt;
+    unsigned int *cnt, *bits;
     int lg;
 
+    // all slots empty, by the lanes or threads `id` of `count`
+    template <bool PV>
+    __device__ __forceinline__ void clear(int id, int count) const
+    {
+        const int slots = 1 << lg;
+        for (int k = id; k < slots; k += count) {
+            key[k] = kNoMember;
+            if (PV) cnt[k] = 0;
+        }
+        for (int k = id; k < slots / 4; k += count) bits[k] = 0;
+    }
     __device__ __forceinline__ void insert(int m) const
     {
-        const unsigned int mask = (1u << lg) - 1u;
-        unsigned int s = hash_slot(m, lg);
+        const unsigned int mask = (1u << lg) - 1u, b = hash_slot(m, lg + 3);
+        atomicOr(&bits[b >> 5], 1u << (b & 31));
+        unsigned int s = b >> 3;
         while (atomicCAS(&key[s], kNoMember, m) != kNoMember) s = (s + 1) & mask;
     }
     __device__ __forceinline__ int find(int x) const
     {
-        const unsigned int mask = (1u << lg) - 1u;
-        unsigned int s = hash_slot(x, lg);
+        const unsigned int mask = (1u << lg) - 1u, b = hash_slot(x, lg + 3);
+        if (!((bits[b >> 5] >> (b & 31)) & 1u)) return -1;
+        unsigned int s = b >> 3;
         int k = key[s];
         while (k != x && k != kNoMember) {
             s = (s + 1) & mask;
@@ -1225,13 +1243,10 @@ __device__ __forceinline__ void table_warp_row(const Data &w, int v, const VInfo
     const Lists ls = lists_of<BATCH>(w, rec);
     const long long v0 = BATCH ? rec->v0 : 0;
     const int *list = ls.base + vi.fbeg;
-    const MemberTable tab{sm.key, sm.cnt, max(ceil_log2(4 * (long long)vi.fdeg), 5)};
+    const MemberTable tab{sm.key, sm.cnt, sm.bits, max(ceil_log2(4 * (long long)vi.fdeg), 5)};
     const int slots = 1 << tab.lg;
     __syncwarp();
-    for (int k = lane; k < slots; k += 32) {
-        sm.key[k] = kNoMember;
-        if (PV) sm.cnt[k] = 0;
-    }
+    tab.clear<PV>(lane, 32);
     __syncwarp();
     for (int k = lane; k < vi.fdeg; k += 32) tab.insert(list[k]);
     __syncwarp();
@@ -1261,15 +1276,15 @@ __device__ void table_block_row(const Data &w, int v, const VInfo &vi, const Gra
     const int *list = ls.base + vi.fbeg;
     __syncthreads();
     if (threadIdx.x == 0) sm.total = 0;
+    // members whose lists a warp takes at a time: four shares per warp at
+    // least (R-MAT 22, wide rows: 5140 us at 32 members always, 4726 so)
+    const int per = max(4, min(32, vi.fdeg / (4 * kThreads / 32)));
     for (int c0 = 0; c0 < vi.fdeg; c0 += kMemberChunk) {
         const int nm = min(vi.fdeg - c0, kMemberChunk);
-        const MemberTable tab{sm.key, sm.cnt,
+        const MemberTable tab{sm.key, sm.cnt, sm.bits,
                               min(max(ceil_log2(8 * (long long)nm), 6), kTableLog2)};
         const int slots = 1 << tab.lg;
-        for (int k = threadIdx.x; k < slots; k += kThreads) {
-            sm.key[k] = kNoMember;
-            if (PV) sm.cnt[k] = 0;
-        }
+        tab.clear<PV>(threadIdx.x, kThreads);
         if (threadIdx.x == 0) sm.next = 0;
         __syncthreads();
         for (int k = threadIdx.x; k < nm; k += kThreads) tab.insert(list[c0 + k]);
@@ -1277,10 +1292,10 @@ __device__ void table_block_row(const Data &w, int v, const VInfo &vi, const Gra
         unsigned int mine = 0;
         while (true) {
             int k = 0;
-            if (lane == 0) k = atomicAdd(&sm.next, 32);
+            if (lane == 0) k = atomicAdd(&sm.next, per);
             k = __shfl_sync(0xffffffffu, k, 0);
             if (k >= vi.fdeg) break;
-            mine += probe_members<PV, Pos>(w, ls, list, k, vi.fdeg, tab);
+            mine += probe_members<PV, Pos>(w, ls, list, k, min(k + per, vi.fdeg), tab);
         }
         __syncthreads();
         if (PV)
