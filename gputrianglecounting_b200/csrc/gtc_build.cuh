@@ -448,10 +448,10 @@ __device__ __forceinline__ void row_record(const Data &w, long long v, long long
 // The signatures of 32 rows, a lane each: bits[word][lane].
 typedef unsigned int SignSmem[kSigWords][32];
 
-// Those of rows u0 .. u0 + 31 that are of uniform graphs (mine): where the ids
+// Of the first `rows` rows from u0 on, those of uniform graphs (mine): where the ids
 // above the row's own begin, and the signature of those ids.
 template <typename OffT, bool BATCH>
-__device__ __forceinline__ void split_rows(const View<OffT> &w, long long u0, int g, bool mine,
+__device__ __forceinline__ void split_rows(const View<OffT> &w, long long u0, int rows, int g, bool mine,
                                            SignSmem &bits)
 {
     const int lane = threadIdx.x & 31;
@@ -474,11 +474,10 @@ __device__ __forceinline__ void split_rows(const View<OffT> &w, long long u0, in
     // ids out of range, looked for in the rows' entries as one stream
     bool bad = false;
     const int g0 = __shfl_sync(0xffffffffu, g, 0);
-    if (__all_sync(0xffffffffu, v >= w.n || (mine && g == g0))) {
+    if (__all_sync(0xffffffffu, lane >= rows || (mine && g == g0))) {
         const unsigned int n0 = __shfl_sync(0xffffffffu, nv, 0);
         const long long b0 = __shfl_sync(0xffffffffu, b, 0);
-        const int last = (int)min(31ll, w.n - 1 - u0);
-        const long long e1 = __shfl_sync(0xffffffffu, e, last);
+        const long long e1 = __shfl_sync(0xffffffffu, e, rows - 1);
         for (long long i = b0 + lane; i < e1; i += 128) {
 #pragma unroll
             for (int j = 0; j < 4; ++j)
@@ -532,9 +531,9 @@ __device__ __forceinline__ void split_rows(const View<OffT> &w, long long u0, in
     to[1] = make_uint4(bits[4][lane], bits[5][lane], bits[6][lane], bits[7][lane]);
 }
 
-// Rows u0 .. u0 + 31 of other graphs that are not long rows.
+// Of the first `rows` rows from u0 on, those of other graphs that are not long rows.
 template <typename OffT, bool BATCH>
-__device__ __forceinline__ void stream_rows(const View<OffT> &w, long long u0, int g)
+__device__ __forceinline__ void stream_rows(const View<OffT> &w, long long u0, int rows, int g)
 {
     constexpr int kPer = 4;
     const int lane = threadIdx.x & 31;
@@ -542,7 +541,7 @@ __device__ __forceinline__ void stream_rows(const View<OffT> &w, long long u0, i
     long long b = 0;
     int d = 0, kmin = kKeyTop, v0 = 0, nv = (int)w.n;
     bool mine = false;
-    if (v < w.n) {
+    if (lane < rows) {
         const GraphRec *rec = &w.recs[g];
         b = (long long)w.off[v];
         d = (int)((long long)w.off[v + 1] - b);
@@ -608,7 +607,7 @@ __device__ __forceinline__ void stream_rows(const View<OffT> &w, long long u0, i
 
 template <typename OffT, bool BATCH>
 __global__ void __launch_bounds__(kThreads, 5)
-place_kernel(const View<OffT> w, bool do_wide, bool do_short)
+place_kernel(const View<OffT> w, bool do_wide, bool do_short, int batch)
 {
     __shared__ SignSmem s_sign[kThreads / 32];
     if (gated(w)) return;
@@ -621,15 +620,17 @@ place_kernel(const View<OffT> w, bool do_wide, bool do_short)
         for (long long i = warp; i < items; i += warps) place_chunk<OffT, BATCH>(w, w.litem[i]);
     }
     if (!do_short) return;
-    long long u0 = warp * 32;
+    long long u0 = warp * batch;
     while (u0 < w.n) {
-        const int g = BATCH && u0 + lane < w.n ? w.gid[u0 + lane] : 0;
-        const bool in = u0 + lane < w.n, uniform = in && w.recs[g].uniform;
+        const int rows = (int)min((long long)batch, w.n - u0);
+        const bool in = lane < rows;
+        const int g = BATCH && in ? w.gid[u0 + lane] : 0;
+        const bool uniform = in && w.recs[g].uniform;
         if (__any_sync(0xffffffffu, uniform))
-            split_rows<OffT, BATCH>(w, u0, g, uniform, s_sign[threadIdx.x >> 5]);
-        if (__any_sync(0xffffffffu, in && !uniform)) stream_rows<OffT, BATCH>(w, u0, g);
-        if (warps * 32 >= w.n) break;
-        if (lane == 0) u0 = 32 * (warps + (long long)atomicAdd(&w.ctr->place_next, 1ull));
+            split_rows<OffT, BATCH>(w, u0, rows, g, uniform, s_sign[threadIdx.x >> 5]);
+        if (__any_sync(0xffffffffu, in && !uniform)) stream_rows<OffT, BATCH>(w, u0, rows, g);
+        if (warps * batch >= w.n) break;
+        if (lane == 0) u0 = batch * (warps + (long long)atomicAdd(&w.ctr->place_next, 1ull));
         u0 = __shfl_sync(0xffffffffu, u0, 0);
     }
 }

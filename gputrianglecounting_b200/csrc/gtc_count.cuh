@@ -151,6 +151,17 @@ __device__ __forceinline__ void warp_sort(int (&v)[E], int lane)
     }
 }
 
+// Whose first share this block takes of the second and third kind of work of
+// a kernel.  With less than two rows per warp most blocks have no other share,
+// and those that took wide rows should not have the first tiles too (R-MAT 10,
+// counting kernel: 13.9 us all from block 0 on, 12.4 shifted); with more the
+// blocks come free at different times (R-MAT 17: 127 us, 134 shifted).
+__device__ __forceinline__ long long first_block(long long n, unsigned int shift)
+{
+    const bool few = n < 2ll * gridDim.x * (kThreads / 32);
+    return few ? (blockIdx.x + shift) % gridDim.x : blockIdx.x;
+}
+
 // Longest list of a wide row that a warp takes: bit matrix, tables.
 constexpr int kWarpList = 256, kWarpTable = 128;
 constexpr int kClaim = 128;                       // most wide rows a block looks through at a time
@@ -169,8 +180,8 @@ struct WideClaim {
 // from queues.  A share's rows are spread over the list, whose neighbours tend
 // to be alike (generators give hubs the lowest ids).
 template <class Want, class ByBlock, class ByWarp>
-__device__ __forceinline__ void wide_rows(const Data &w, WideClaim &cl, unsigned long long *long_next,
-                                          unsigned long long *next, int most, const Want &want,
+__device__ __forceinline__ void wide_rows(const Data &w, WideClaim &cl, long long block,
+                                          unsigned long long *long_next, unsigned long long *next, int most, const Want &want,
                                           const ByBlock &by_block, const ByWarp &by_warp)
 {
     const long long rows = (long long)w.ctr->wide_rows;
@@ -180,7 +191,7 @@ __device__ __forceinline__ void wide_rows(const Data &w, WideClaim &cl, unsigned
     const int per_block = (int)min((long long)kClaim, max(8ll, rows / (4ll * gridDim.x)));
     const int per_warp = (int)min((long long)kWarpClaim, max(1ll, rows / (16 * warps)));
     long long claims = div_up<long long>(rows, per_block);
-    long long item = blockIdx.x;
+    long long item = block;
     while (item < claims) {
         __syncthreads();
         if (threadIdx.x == 0) cl.count = 0;
@@ -203,7 +214,7 @@ __device__ __forceinline__ void wide_rows(const Data &w, WideClaim &cl, unsigned
     }
     __syncthreads();
     claims = div_up<long long>(rows, per_warp);
-    item = (long long)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+    item = block * (kThreads / 32) + (threadIdx.x >> 5);
     while (item < claims) {
         const long long at = item + claims * lane;
         int v = 0;
@@ -483,7 +494,7 @@ __device__ __forceinline__ void core_wide_rows(const Data &w, CoreSmem &sm,
 {
     const Transposer tr(threadIdx.x & 31);
     wide_rows(
-        w, sm.claim, &w.ctr->core_long_next, &w.ctr->core_wide_next, kWarpList,
+        w, sm.claim, blockIdx.x, &w.ctr->core_long_next, &w.ctr->core_wide_next, kWarpList,
         [](const VInfo &vi) { return (vi.dk & INT32_MAX) >= 2; },
         [&](int v, const VInfo &vi) {
             core_block_row<PV>(w, vi, w.recs[BATCH ? w.gid[v] : 0].core,
@@ -1317,7 +1328,7 @@ __device__ __forceinline__ void table_wide_rows(const Data &w, ListSmem<Pos> &sm
 {
     // a member outside the core, and one more (core rows have none)
     wide_rows(
-        w, sm.claim, &w.ctr->table_long_next, &w.ctr->table_wide_next, kWarpTable,
+        w, sm.claim, first_block(w.n, gridDim.x / 4), &w.ctr->table_long_next, &w.ctr->table_wide_next, kWarpTable,
         [](const VInfo &vi) { return vi.fdeg >= 2 && vi.fdeg > (vi.dk & INT32_MAX); },
         [&](int v, const VInfo &vi) {
             table_block_row<PV, BATCH, Pos>(w, v, vi, &w.recs[BATCH ? w.gid[v] : 0], sm.block, tri);
@@ -1361,7 +1372,8 @@ __device__ __forceinline__ void warp_batches(unsigned long long *queue, long lon
                                              const Rows &rows)
 {
     const long long all = (long long)gridDim.x * (kThreads / 32) * batch;
-    long long u0 = ((long long)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5)) * batch;
+    const long long block = first_block(n, gridDim.x / 2);
+    long long u0 = (block * (kThreads / 32) + (threadIdx.x >> 5)) * batch;
     while (u0 < n) {
         rows(u0);
         if (all >= n) break;
