@@ -517,8 +517,8 @@ def run_b200(args, name: str, rank: int, world: int, with_baseline: bool = True)
 
 def launches_per_count(n: int, nnz: int, tuning: dict | None = None) -> int:
     """Kernels of one plain count with every output (the library's own plan:
-    5 with vertex-id labels, 6 from 2^18 rows on, 11 with degree-rank
-    labels)."""
+    5 in the joint form, 6 of them from 2^18 vertices on, 11 in the split
+    form)."""
     from gputrianglecounting_b200 import api
     return api.launch_plan(n, nnz, tuning=tuning)["launches"]
 
@@ -534,8 +534,10 @@ def int32_offsets(host_graph):
 
 def phase_breakdown(counter, g, flush, tuning: dict | None = None) -> dict:
     """Per-phase device time of one count with this tuning, from events the
-    library records between its phases (forward build / group kernel / block
-    kernel / epilogue), averaged over 3 runs."""
+    library records between its phases (forward build; forward lists, tiles and
+    tables; core pairs in the bit matrix; epilogue), averaged over 3 runs.  The
+    joint form below 2^18 vertices has lists and pairs in one kernel, timed as
+    lists."""
     import ctypes
 
     import torch
@@ -555,17 +557,17 @@ def phase_breakdown(counter, g, flush, tuning: dict | None = None) -> dict:
         res.append(list(times))
     torch.cuda.synchronize()
     avg = [sum(r[i] for r in res) / len(res) for i in range(4)]
-    return {"forward_build": avg[0], "group_kernel": avg[1], "block_kernel": avg[2],
+    return {"forward_build": avg[0], "lists": avg[1], "core_pairs": avg[2],
             "epilogue": avg[3]}
 
 
 # ------------------------------------------------------------------ batched
 
 def batch_launches(total_n: int, total_nnz: int, tuning: dict | None = None) -> int:
-    """Entry starts + globalize + the pipeline without its global-count
-    kernel + per-graph T; with degree-rank labels the batch's graph-major
-    ranks take a histogram, a 3-launch scan and a rank kernel in place of the
-    single graph's 3 rank launches (+2)."""
+    """Joint form: the single graph's kernels, the choice of the cores and
+    per-graph T.  Split form: the single graph's kernels but the global count,
+    the graphs' limits, the vertices' graphs, zeroed bit matrices, the core's
+    credits and per-graph T."""
     from gputrianglecounting_b200 import api
     extra = 2 if api.launch_plan(total_n, total_nnz, tuning=tuning)["labels"] == "degree-rank" \
         else 0
@@ -827,6 +829,15 @@ def main() -> None:
     cfg = CONFIGS[args.config]
     world = int(os.environ.get("WORLD_SIZE", "1"))
     rank = int(os.environ.get("RANK", "0"))
+    from oracle import oracle as O
+    if not O.ref_cpu_available():
+        args.no_cpu_baseline = True
+        if args.impl == "reference":
+            if rank == 0:
+                print(json.dumps({"impl": "reference", "unavailable":
+                                  "the reference's CPU code is not built (its sources are not "
+                                  "here)"}))
+            return
     if args.impl == "reference":
         run_reference(args, cfg, rank)
         return

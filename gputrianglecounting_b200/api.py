@@ -140,8 +140,8 @@ class TriangleCounter:
         mode "plain": per-vertex outputs (any of "r", "t", "lcc") + global.
         mode "oriented": global count only (the reference README's dest<src
         mode), no per-vertex bookkeeping.
-        tuning: optional launch-shape overrides (keys of gtc_tuning: group,
-        item_len, big_chunk, big_hash_max); they never change the result.
+        tuning: optional launch-shape overrides (keys of gtc_tuning; "labels"
+        picks joint or split launches); they never change the result.
         """
         off_bits = _check_csr_tensors(off, ind)
         if mode not in _MODES:
@@ -181,7 +181,7 @@ LABELS = {1: "vertex-id", 2: "degree-rank"}
 
 def launch_plan(n: int, nnz: int, mode: str = "plain", tuning: dict | None = None) -> dict:
     """What a count of an (n, nnz) graph would run, host-only: kernel launches
-    per count and the vertex labelling ("vertex-id" or "degree-rank")."""
+    per count and their form ("vertex-id": joint, "degree-rank": split)."""
     if mode not in _MODES:
         raise ValueError(f"mode must be one of {list(_MODES)}")
     tun = _lib.Tuning(**{k: int(v) for k, v in tuning.items()}) if tuning else None

@@ -4,22 +4,12 @@ Replaces the reference's brute-force sweep of 8 block sizes x 6
 threads-per-intersection values (allParamTestGPURun, src/gpurun.cu:115-176,
 grids in src/param.cu:2-6).  The knobs here never change a result (tested):
 
-  group        threshold between the warp-per-item kernel and the block
-               kernel: apexes with a forward list longer than 4*group go to
-               the block kernel ("warp vs block");
-  item_len     adjacency entries per warp work item (partition granularity);
-  big_chunk    adjacency entries per block work item;
-  big_hash_max longest forward list hashed in shared memory before the
-               block kernel switches to in-place binary search ("hash vs
-               search");
-  labels       the degree-ordering policy: vertex ids ordered by (degree,
-               id) (1) or degree ranks with rank-sorted forward lists and the
-               block kernel's rank bitmap (2);
-  region       warp-kernel hash slots per forward-list member (2 or 4):
-               rows per table batch against collisions;
-  rows         the group kernel's form with vertex-id labels: a warp per
-               work item with per-row hash regions (1) or per-row merges of
-               the id-ordered lists (2).
+  labels       joint launches (1: long and short rows in one kernel each) or
+               split ones (2: a kernel for each kind of row);
+  rows         2 asks for joint launches, like labels 1;
+  group, region, item_len, big_chunk, big_hash_max
+               checked by the library, which no longer needs them: its kernels
+               choose these shapes from the rows.
 
 A graph's *degree profile* -- size, mean degree and skew buckets -- keys a
 cache (in memory and, optionally, a JSON file), so each profile is tuned

@@ -3,29 +3,23 @@
 // A batch is the disjoint union of its graphs: graph g owns the vertex range
 // [vstart[g], vstart[g+1]) and the entry range [off[vstart[g]],
 // off[vstart[g+1]]) of one concatenated CSR whose adjacency holds *local* ids
-// (0 .. n_g-1).  The batch entry point turns local ids into union ids in one
-// pass and runs the single-graph pipeline (persistent kernels pulling work
-// items from device queues) once over the union; triangles never cross graphs,
-// so every per-vertex value is exactly the one the graph gets alone.  With
-// degree-rank labels the ranks are graph-major (each graph's vertices take the
-// consecutive ranks vstart[g] ..), so an apex's forward list spans only its own
-// graph's ranks and small graphs keep the block kernel's direct per-rank
-// counters.  A final kernel sums t over each graph's vertex range into that
-// graph's T.
+// (0 .. n_g-1).  The single-graph pipeline runs once over all vertices, each
+// with the record of its graph (limits, core, bit matrix, uniform or not); it
+// adds a graph's first vertex to an id where it reads one.  Triangles never
+// cross graphs, so every per-vertex value is exactly the one the graph gets
+// alone.  The epilogue sums t over each graph's vertices into its T.
 // The reference has no batched form; its per-graph operator is kernelCall
 // (src/clusteringCount.cu:415-467), which the one-launch-per-graph baseline
 // calls once per graph.
-#include <cooperative_groups.h>
-#include <cooperative_groups/reduce.h>
 
 #include "gtc_core.cuh"
 
-namespace cg = cooperative_groups;
 
 namespace gtc {
 namespace {
 
 constexpr int kChunk = 4096;     // entries (or vertices) per block
+constexpr int kPackThreads = 256;
 
 // Largest g in [0, G) with start[g] <= x (start non-decreasing, start[0] <= x).
 __device__ __forceinline__ long long owner(const long long *__restrict__ start, long long G,
@@ -65,6 +59,10 @@ __global__ void pack_vertices_kernel(const PackRef *__restrict__ refs,
     if (blockIdx.x == 0 && threadIdx.x == 0) off_out[total_n] = total_nnz;
 }
 
+// A block's chunk is mostly one graph's: then a plain copy with eight loads in
+// flight per thread (64 graphs, 53 M entries: 175 -> 90 us).
+static_assert(kChunk % (8 * kPackThreads) == 0, "whole rounds of a chunk");
+
 __global__ void pack_entries_kernel(const PackRef *__restrict__ refs,
                                     const long long *__restrict__ ebase, long long G,
                                     int *__restrict__ ind_out, long long total_nnz)
@@ -74,6 +72,19 @@ __global__ void pack_entries_kernel(const PackRef *__restrict__ refs,
     if (threadIdx.x == 0) s_g0 = owner(ebase, G, e_begin);
     __syncthreads();
     long long g = s_g0;
+    if (e_begin + kChunk <= ebase[g + 1]) {
+        constexpr int kFlight = 8;
+        const int *from = refs[g].ind + (e_begin - ebase[g]);
+        int *to = ind_out + e_begin;
+        for (int k = threadIdx.x; k < kChunk; k += kFlight * kPackThreads) {
+            int x[kFlight];
+#pragma unroll
+            for (int j = 0; j < kFlight; ++j) x[j] = from[k + j * kPackThreads];
+#pragma unroll
+            for (int j = 0; j < kFlight; ++j) to[k + j * kPackThreads] = x[j];
+        }
+        return;
+    }
     for (long long e = e_begin + threadIdx.x; e < e_begin + kChunk && e < total_nnz; e += blockDim.x) {
         while (g + 1 < G && ebase[g + 1] <= e) ++g;
         ind_out[e] = refs[g].ind[e - ebase[g]];
@@ -174,10 +185,10 @@ gtc_status gtc_batch_pack(int64_t num_graphs, const void *const *h_off, const vo
     if (cudaMemcpyAsync(d_vstart, d_vb, sizeof(long long) * (size_t)(num_graphs + 1),
                         cudaMemcpyDeviceToDevice, s) != cudaSuccess)
         return GTC_ERR_CUDA;
-    pack_vertices_kernel<<<(unsigned)div_up<long long>(total_n + 1, kChunk), 256, 0, s>>>(
+    pack_vertices_kernel<<<(unsigned)div_up<long long>(total_n + 1, kChunk), kPackThreads, 0, s>>>(
         d_refs, d_vb, d_eb, num_graphs, reinterpret_cast<long long *>(d_off), total_n, total_nnz);
     if (total_nnz > 0)
-        pack_entries_kernel<<<(unsigned)div_up<long long>(total_nnz, kChunk), 256, 0, s>>>(
+        pack_entries_kernel<<<(unsigned)div_up<long long>(total_nnz, kChunk), kPackThreads, 0, s>>>(
             d_refs, d_eb, num_graphs, d_ind, total_nnz);
     return cudaGetLastError() == cudaSuccess ? GTC_OK : GTC_ERR_CUDA;
 }

@@ -162,7 +162,8 @@ __device__ __forceinline__ long long first_block(long long n, unsigned int shift
     return few ? (blockIdx.x + shift) % gridDim.x : blockIdx.x;
 }
 
-// Longest list of a wide row that a warp takes: bit matrix, tables.
+// Longest list of a wide row that a warp takes: bit matrix, tables (tables of
+// 256 members for a warp, half full: R-MAT 22's wide rows 5300 us against 4726).
 constexpr int kWarpList = 256, kWarpTable = 128;
 constexpr int kClaim = 128;                       // most wide rows a block looks through at a time
 constexpr int kWarpClaim = 8;                     // ... a warp
@@ -291,7 +292,11 @@ __device__ __forceinline__ CoreView core_view(const Data &w, int v)
 // in ascending position (descending order) s has the lower index, so the pairs
 // are a lower triangle of index pairs, in tiles of 32 q by 32 s.  A lane holds
 // a member s and loads its word of 32 rows q.  A tile's hits are a 32 x 32 bit
-// matrix: rows count s, columns (transposed) count q.
+// matrix: rows count s, columns (transposed) count q.  Waits for the gathered
+// words bound it, then the shared loads of row offsets: eight instructions per
+// step of 32 pairs, 32 warps per SM at 64 registers (R-MAT 20, wide rows: 781
+// us; five blocks of 48 registers 1053 when this took 946; looking ids up in
+// shared tables of the longer lists, which this replaced, 2375).
 
 // A row of at most kWarpList members (32 E) by a warp, sorted in registers.
 template <int E, bool PV>
@@ -658,7 +663,9 @@ __device__ __forceinline__ void tile_init(TileSmem<Pos> &sm)
 // and half a row's sum is p's.  The pairs of core members are not among them
 // (their lists are not looked up).  Shared-memory wavefronts bound it, so the
 // table is a twentieth full -- a look-up that finds nothing mostly ends at its
-// first slot -- and its bytes are the numbers themselves.
+// first slot -- and its bytes are the numbers themselves (RGG 4M: 402 us, 87%
+// of the wavefront slots; per-row merges of sorted lists, 8 of 32 lanes busy,
+// took 863.  R-MAT 22's short rows: 2160 us, at 1024 slots 2433).
 template <bool PV, bool BATCH, typename Pos>
 __device__ __forceinline__ void
 tile_rows(const Data &w, long long u0, const VInfo &vi, int g, bool act, TileSmem<Pos> &smem,
@@ -924,6 +931,8 @@ tile_rows(const Data &w, long long u0, const VInfo &vi, int g, bool act, TileSme
 // each: the members' signatures are put side by side, and a lane reads its word
 // of each in turn -- a warp's reads lie in eight neighbouring banks, one
 // wavefront per step.  Pairs that pass are queued and searched for 32 at a time.
+// Instruction issue bounds it (70%): ER 900K of mean degree 30 takes 247 us,
+// tiles of the same rows 558.
 template <bool PV, bool BATCH, typename Pos>
 struct SignedRows {
     const Data &w;

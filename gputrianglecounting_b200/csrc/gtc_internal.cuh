@@ -149,17 +149,4 @@ __host__ __device__ __forceinline__ T div_up(T a, T b)
     return (a + b - 1) / b;
 }
 
-// Largest row r in [0, n) with off[r] <= e (e < off[n]): the row holding e.
-template <typename OffT>
-__device__ __forceinline__ long long row_of_entry(const OffT *__restrict__ off,
-                                                  long long n, long long e)
-{
-    long long lo = 0, hi = n;           // invariant: off[lo] <= e < off[hi]
-    while (hi - lo > 1) {
-        long long mid = (lo + hi) >> 1;
-        if ((long long)off[mid] <= e) lo = mid; else hi = mid;
-    }
-    return lo;
-}
-
 }  // namespace gtc

@@ -116,25 +116,17 @@ gtc_status gtc_count_status(const void *d_workspace, size_t ws_bytes,
  * choice).  Used by the autotuner, which replaces the reference's
  * block-size x threads-per-intersection sweep (src/gpurun.cu:115-176,
  * src/param.cu:2-6).  None of them changes the result.
- *   group        lanes that share one apex row in the group kernel: 4, 8,
- *                16 or 32; rows whose forward list is longer than
- *                4*group go to the block kernel
- *   item_len     adjacency entries per warp work item (a power of two, 32 .. 32768)
- *   big_chunk    adjacency entries per block-kernel work item (32 .. 32768)
- *   big_hash_max longest forward list the block kernel hashes in shared
- *                memory (<= 2048); longer lists are binary-searched in place
- *   labels       how forward lists name vertices: 1 = vertex ids (order by
- *                (degree, id)), 2 = degree ranks (vertices counting-sorted
- *                by degree, lists sorted by rank, block kernel on a rank
- *                bitmap); the library picks ranks for mean degree > 24
- *   region       warp-kernel hash slots per forward-list member: 2 or 4 (the
- *                library picks 2 for mean degree <= 24, else 4)
- *   rows         the group kernel's form: 1 = warp per work item with per-row
- *                hash regions, 2 = per-row merges of id-ordered forward lists
- *                (vertex-id labels only; with labels = 2 it is rejected, with
- *                labels = 0 it implies vertex ids).  The library picks 2 for
- *                single graphs with vertex-id labels and at least 2^18
- *                vertices, else 1
+ *   labels       1 = joint launches: long and short rows in one kernel each
+ *                (5 kernels per count, 6 from 2^18 vertices on); 2 = split
+ *                launches: a kernel for long and one for short rows (11).
+ *                The library splits above mean degree 24
+ *   rows         2 asks for joint launches too (rejected with labels = 2);
+ *                1 leaves the choice to labels
+ *   group, item_len, big_chunk, big_hash_max, region
+ *                checked (group 4, 8, 16 or 32; item_len a power of two from
+ *                32 to 32768; big_chunk 32 .. 32768; big_hash_max <= 2048;
+ *                region 2 or 4) and otherwise without effect: the kernels
+ *                choose these shapes from the rows themselves
  */
 typedef struct gtc_tuning {
     int group;
@@ -146,7 +138,7 @@ typedef struct gtc_tuning {
     int rows;
 } gtc_tuning;
 
-/* Values of gtc_tuning.labels. */
+/* Values of gtc_tuning.labels (vertex ids: joint, degree rank: split). */
 enum { GTC_LABELS_AUTO = 0, GTC_LABELS_VERTEX_ID = 1, GTC_LABELS_DEGREE_RANK = 2 };
 /* Values of gtc_tuning.rows. */
 enum { GTC_ROWS_AUTO = 0, GTC_ROWS_HASH = 1, GTC_ROWS_MERGE = 2 };
@@ -170,7 +162,9 @@ gtc_status gtc_count_tuned(const void *d_off, int off_bits,
 /*
  * Diagnostic: one synchronous per-vertex count on the legacy default stream
  * with CUDA events between the pipeline phases; writes the device time in ms
- * of {forward-list build, group kernel, block kernel, epilogue} to h_ms[4].
+ * of {forward-list build; forward lists: tiles and tables; pairs of core
+ * members in the bit matrix; epilogue} to h_ms[4].  One kernel does the second
+ * and third in joint launches below 2^18 vertices; its time is the second.
  * tuning: as for gtc_count_tuned (NULL = the library's choice).  Stands in for
  * the reference's chrono timing around launch + sync (src/gpurun.cu:17-47,
  * timedKernelCall :469-508).
