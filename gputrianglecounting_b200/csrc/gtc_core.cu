@@ -134,8 +134,10 @@ Plan make_plan(long long n, long long nnz, int off_bits, bool per_vertex, long l
 RowConfig pick_row_config(long long n, long long nnz)
 {
     RowConfig c;
-    // heavy graphs have enough work to fill the GPU with each kind of row
-    c.split = n > 0 && (double)nnz / (double)n > 24.0;
+    // heavy graphs have enough work to fill the GPU with each kind of row; even
+    // so R-MAT 20 takes 1547 us split and 1518 joint.  Smaller ones do not:
+    // R-MAT 17 223 us split, 174 joint
+    c.split = n >= kSmallGraph && (double)nnz / (double)n > 24.0;
     return c;
 }
 

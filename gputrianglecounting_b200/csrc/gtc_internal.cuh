@@ -29,15 +29,20 @@ namespace gtc {
 
 // ------------------------------------------------------------------ tuning
 constexpr int kThreads = 256;               // every pipeline kernel
-constexpr long long kSmallGraph = 1ll << 18;  // vertices from which the core keys get a launch
+// Vertices from which lists and core pairs get a kernel each: R-MAT 17 takes
+// 181 us in one kernel and 201 in two, R-MAT 20 of mean degree 16 697 and 661.
+constexpr long long kSmallGraph = 1ll << 18;
 constexpr int kShortRow = 64;               // longest row placed with its neighbours
-constexpr int kShortList = 32;              // longest forward list of a short row,
-constexpr int kShortListIds = 64;           // ... of a uniform graph
+// Longest forward list of a short row; of a uniform graph.  16 instead of 32:
+// R-MAT 20 1507 us instead of 1519, but the 512-graph batch 11.4 ms instead of
+// 10.6.  32 instead of 64: ER 900K of mean degree 30 400 us instead of 346.
+constexpr int kShortList = 32;
+constexpr int kShortListIds = 64;
 constexpr int kRowChunk = 256;              // entries of a longer row per placement item
 constexpr int kBuckets = 1024;              // degree buckets (counting sort of the core)
 constexpr int kCoreMax = 32768;             // most core vertices of a graph
 constexpr int kCoreMinDegree = kShortRow + 1;   // core rows are never short rows
-constexpr int kCoreDegreeRatio = 4;         // ... and have 4 times the mean degree at least
+constexpr int kCoreDegreeRatio = 2, kCoreDegreeOver = 16;   // ... of this multiple of the mean, plus
 constexpr int kMemberChunk = 1024;          // members of a wide row held at a time
 constexpr int kTableLog2 = 12;              // wide rows: shared hash slots
 constexpr int kKeyTop = 0x7fffffff;         // key of core position 0

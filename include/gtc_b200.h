@@ -119,7 +119,7 @@ gtc_status gtc_count_status(const void *d_workspace, size_t ws_bytes,
  *   labels       1 = joint launches: long and short rows in one kernel each
  *                (5 kernels per count, 6 from 2^18 vertices on); 2 = split
  *                launches: a kernel for long and one for short rows (11).
- *                The library splits above mean degree 24
+ *                The library splits above mean degree 24 from 2^18 vertices on
  *   rows         2 asks for joint launches too (rejected with labels = 2);
  *                1 leaves the choice to labels
  *   group, item_len, big_chunk, big_hash_max, region
