@@ -239,8 +239,16 @@ degree_kernel(const View<OffT> w, GraphRec lim, bool ids, bool choose)
     if (gated(w)) return;
     __shared__ int s_g;
     __shared__ bool s_last;
+    __shared__ unsigned int s_hist[BATCH ? 1 : kBuckets];
     const int lane = threadIdx.x & 31;
     const long long stride = (long long)gridDim.x * kThreads;
+    // a large graph's blocks count for themselves first: the buckets of the
+    // lowest core degrees are many vertices' (R-MAT 22: 105 us, 42 so)
+    const bool own = !BATCH && w.n > stride;
+    if (own) {
+        for (int k = threadIdx.x; k < kBuckets; k += kThreads) s_hist[k] = 0;
+        __syncthreads();
+    }
     for (long long v0 = (long long)blockIdx.x * kThreads; v0 < w.n; v0 += stride) {
         const long long v = v0 + threadIdx.x;
         if (BATCH && ids) {
@@ -266,7 +274,7 @@ degree_kernel(const View<OffT> w, GraphRec lim, bool ids, bool choose)
             lng = d > lim.long_min;
             const int bk = degree_bucket(d);
             if (lng && bk >= degree_bucket(lim.dmin))
-                atomicAdd(&w.hist[(long long)g * kBuckets + bk], 1u);
+                atomicAdd(own ? &s_hist[BATCH ? 0 : bk] : &w.hist[(long long)g * kBuckets + bk], 1u);
         }
         const unsigned int m = __ballot_sync(0xffffffffu, lng);
         if (m) {
@@ -275,6 +283,11 @@ degree_kernel(const View<OffT> w, GraphRec lim, bool ids, bool choose)
             at = __shfl_sync(0xffffffffu, at, 0);
             if (lng) w.wide[at + __popc(m & ((1u << lane) - 1u))] = (int)v;
         }
+    }
+    if (own) {
+        __syncthreads();
+        for (int k = threadIdx.x; k < kBuckets; k += kThreads)
+            if (s_hist[k]) atomicAdd(&w.hist[k], s_hist[k]);
     }
     if (BATCH || !choose) return;
     __threadfence();
@@ -454,24 +467,21 @@ __device__ __forceinline__ void row_record(const Data &w, long long v, long long
 typedef unsigned int SignSmem[kSigWords][32];
 
 // Of the first `rows` rows from u0 on, those of uniform graphs (mine): where the ids
-// above the row's own begin, and the signature of those ids.
-template <typename OffT, bool BATCH>
+// above the row's own begin (b, e: the lane's row), and the signature of those ids.
+template <typename OffT, bool BATCH, bool SIGN>
 __device__ __forceinline__ void split_rows(const View<OffT> &w, long long u0, int rows, int g, bool mine,
-                                           SignSmem &bits)
+                                           long long b, long long e, SignSmem &bits)
 {
     const int lane = threadIdx.x & 31;
     const long long v = u0 + lane;
-    long long b = 0, e = 0;
     int vl = 0, long_min = 0;
     unsigned int nv = 0;
     unsigned int *sign = nullptr;
     if (mine) {
         const GraphRec *rec = &w.recs[g];
-        if (rec->uniform == kSigned)
+        if (SIGN && rec->uniform == kSigned)
             sign = reinterpret_cast<unsigned int *>(w.find) + rec->ubase +
                    kSigWords * (v - (BATCH ? rec->v0 : 0));
-        b = (long long)w.off[v];
-        e = (long long)w.off[v + 1];
         nv = BATCH ? (unsigned int)rec->nv : (unsigned int)w.n;
         vl = (int)(v - (BATCH ? rec->v0 : 0));
         long_min = rec->long_min;
@@ -516,24 +526,26 @@ __device__ __forceinline__ void split_rows(const View<OffT> &w, long long u0, in
         }
     }
     row_record(w, v, lo, e > lo ? (int)(e - lo) : 0, 0, kShortListIds, listed);
-    if (!sign) return;
+    if constexpr (SIGN) {
+        if (!sign) return;
 #pragma unroll
-    for (int k = 0; k < kSigWords; ++k) bits[k][lane] = 0;
-    const int *list = w.ind + lo;
-    const int n = (int)(e - lo);
-    for (int i = 0; i < n; i += 4) {
-        int y[4];
+        for (int k = 0; k < kSigWords; ++k) bits[k][lane] = 0;
+        const int *list = w.ind + lo;
+        const int n = (int)(e - lo);
+        for (int i = 0; i < n; i += 4) {
+            int y[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) y[j] = list[min(i + j, n - 1)];
+            for (int j = 0; j < 4; ++j) y[j] = list[min(i + j, n - 1)];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const Sign x = sign_of(y[j]);
-            bits[x.word][lane] |= x.bits;
+            for (int j = 0; j < 4; ++j) {
+                const Sign x = sign_of(y[j]);
+                bits[x.word][lane] |= x.bits;
+            }
         }
+        uint4 *to = reinterpret_cast<uint4 *>(sign);
+        to[0] = make_uint4(bits[0][lane], bits[1][lane], bits[2][lane], bits[3][lane]);
+        to[1] = make_uint4(bits[4][lane], bits[5][lane], bits[6][lane], bits[7][lane]);
     }
-    uint4 *to = reinterpret_cast<uint4 *>(sign);
-    to[0] = make_uint4(bits[0][lane], bits[1][lane], bits[2][lane], bits[3][lane]);
-    to[1] = make_uint4(bits[4][lane], bits[5][lane], bits[6][lane], bits[7][lane]);
 }
 
 // Of the first `rows` rows from u0 on, those of other graphs that are not long rows.
@@ -626,13 +638,44 @@ place_kernel(const View<OffT> w, bool do_wide, bool do_short, int batch)
     }
     if (!do_short) return;
     long long u0 = warp * batch;
+    // the lane's row's entries, if it is `mine`; else none
+    auto ends = [&](long long u, bool mine, long long &b, long long &e) {
+        b = e = 0;
+        if (mine && u + lane < w.n) {
+            b = (long long)w.off[u + lane];
+            e = (long long)w.off[u + lane + 1];
+        }
+    };
+    if (!BATCH && w.recs[0].uniform && w.recs[0].uniform != kSigned) {
+        // rows alike, so fixed shares are even ones, and the next share's
+        // offsets can be on their way (RGG 4M 117 -> 95 us, of mean degree 4
+        // 97 -> 56).  With signatures to build they are not: the lowest ids
+        // have the longest lists (ER 900K 62 us from the queue, 79 so).
+        long long b, e;
+        ends(u0, lane < batch, b, e);
+        while (u0 < w.n) {
+            const long long u1 = u0 + warps * batch;
+            const int rows = (int)min((long long)batch, w.n - u0);
+            long long b1, e1;
+            ends(u1, lane < batch, b1, e1);
+            split_rows<OffT, BATCH, false>(w, u0, rows, 0, lane < rows, b, e,
+                                    s_sign[threadIdx.x >> 5]);
+            u0 = u1;
+            b = b1;
+            e = e1;
+        }
+        return;
+    }
     while (u0 < w.n) {
         const int rows = (int)min((long long)batch, w.n - u0);
         const bool in = lane < rows;
         const int g = BATCH && in ? w.gid[u0 + lane] : 0;
         const bool uniform = in && w.recs[g].uniform;
-        if (__any_sync(0xffffffffu, uniform))
-            split_rows<OffT, BATCH>(w, u0, rows, g, uniform, s_sign[threadIdx.x >> 5]);
+        if (__any_sync(0xffffffffu, uniform)) {
+            long long b, e;
+            ends(u0, uniform, b, e);
+            split_rows<OffT, BATCH, true>(w, u0, rows, g, uniform, b, e, s_sign[threadIdx.x >> 5]);
+        }
         if (__any_sync(0xffffffffu, in && !uniform)) stream_rows<OffT, BATCH>(w, u0, rows, g);
         if (warps * batch >= w.n) break;
         if (lane == 0) u0 = batch * (warps + (long long)atomicAdd(&w.ctr->place_next, 1ull));
