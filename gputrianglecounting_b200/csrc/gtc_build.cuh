@@ -386,7 +386,7 @@ __device__ __forceinline__ Lists lists_of(const Data &w, const GraphRec *rec)
 //     the ids above the row's begin.
 // The order within a list is arbitrary.  The gathers of keys, from L2, bound it,
 // four to eight in flight per lane: R-MAT 20 166 us (merge-path tiles with a sort
-// of the lists 480), RGG 4M 114 (185), the 512-graph batch 1665 (3308).
+// of the lists 480), RGG 4M 93 (185), the 512-graph batch 1675 (3308).
 template <typename OffT, bool BATCH>
 __device__ __forceinline__ void place_chunk(const View<OffT> &w, int2 it)
 {

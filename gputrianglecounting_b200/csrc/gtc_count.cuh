@@ -293,10 +293,10 @@ __device__ __forceinline__ CoreView core_view(const Data &w, int v)
 // are a lower triangle of index pairs, in tiles of 32 q by 32 s.  A lane holds
 // a member s and loads its word of 32 rows q.  A tile's hits are a 32 x 32 bit
 // matrix: rows count s, columns (transposed) count q.  Waits for the gathered
-// words bound it, then the shared loads of row offsets: eight instructions per
-// step of 32 pairs, 32 warps per SM at 64 registers (R-MAT 20, wide rows: 781
-// us; five blocks of 48 registers 1053 when this took 946; looking ids up in
-// shared tables of the longer lists, which this replaced, 2375).
+// words bound it, then L1 wavefronts (71%), at 32 warps per SM and 64 registers
+// (R-MAT 20, 1.19e9 pairs, wide rows: 781 us; five blocks of 48 registers 1053
+// when this took 946; looking ids up in shared tables of the longer lists,
+// which this replaced, 2375).
 
 // A row of at most kWarpList members (32 E) by a warp, sorted in registers.
 template <int E, bool PV>
