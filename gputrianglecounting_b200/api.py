@@ -15,6 +15,7 @@ kernels of libgtc_b200.so.  There is no CPU path.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 from dataclasses import dataclass
 
@@ -39,6 +40,28 @@ def _stream_handle(stream) -> int | None:
     if stream is None:
         stream = torch.cuda.current_stream()
     return stream.cuda_stream or None
+
+
+def _allocating_on(stream, device):
+    """Context in which torch allocates on the stream that a call launches on.
+    The caching allocator hands a block out again in the order of the stream it
+    was allocated on: with any other one, memory freed at the call's return
+    would be somebody else's while the kernels still use it, and a block could
+    be handed to them while earlier work of its own stream is still to come."""
+    if stream is None:
+        return contextlib.nullcontext()
+    if not isinstance(stream, torch.cuda.Stream):
+        handle = stream.cuda_stream
+        stream = (torch.cuda.ExternalStream(handle, device=device) if handle
+                  else torch.cuda.default_stream(device))
+    return torch.cuda.stream(stream)
+
+
+def _hand_out(t: torch.Tensor | None, stream) -> None:
+    """t, allocated on the launch stream, goes to a caller who reads it (having
+    waited) on the current one: its block stays taken until that has passed."""
+    if stream is not None and t is not None:
+        t.record_stream(torch.cuda.current_stream(t.device))
 
 
 def _check_csr_tensors(off: torch.Tensor, ind: torch.Tensor) -> int:
@@ -199,8 +222,6 @@ def count_subset(off: torch.Tensor, ind: torch.Tensor, vertices: torch.Tensor,
     off_bits = _check_csr_tensors(off, ind)
     if vertices.dtype != torch.int32 or not vertices.is_cuda:
         raise TypeError("vertices must be an int32 CUDA tensor")
-    vertices = vertices.contiguous()
-    out = torch.empty(vertices.numel(), dtype=torch.int64, device=off.device)
     lib = _lib.load()
     n, nnz = off.numel() - 1, ind.numel()
     need = ctypes.c_size_t(0)
@@ -208,11 +229,15 @@ def count_subset(off: torch.Tensor, ind: torch.Tensor, vertices: torch.Tensor,
     if vertices.numel() >= 1024:          # fewer never take a workspace
         check(lib.gtc_subset_workspace_size(n, nnz, off_bits, vertices.numel(),
                                             ctypes.byref(need)), "gtc_subset_workspace_size")
-    if need.value:
-        try:
-            ws = _alloc_workspace(need.value, off.device)
-        except GTCError:
-            pass                          # without a workspace: row by row
+    with _allocating_on(stream, off.device):
+        vertices = vertices.contiguous()
+        out = torch.empty(vertices.numel(), dtype=torch.int64, device=off.device)
+        if need.value:
+            try:
+                ws = _alloc_workspace(need.value, off.device)
+            except GTCError:
+                pass                      # without a workspace: row by row
+    _hand_out(out, stream)
     if ws is None:
         check(lib.gtc_count_subset(off.data_ptr(), off_bits, ind.data_ptr(),
                                    vertices.data_ptr(), vertices.numel(), out.data_ptr(),

@@ -1,0 +1,88 @@
+"""Calls on a stream that is not torch's current one: the memory they use is theirs
+until that stream is done with it.
+
+The lifetime tests launch nothing: the library's entry point is replaced by one that
+notes its pointers, and the caching allocator is asked for the same sizes again while
+the launch stream is held back.
+"""
+import numpy as np
+import pytest
+import torch
+
+from gputrianglecounting_b200 import _lib, api, graphs
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+
+HOLD = 100_000_000                      # clock cycles a stream is held back, some 50 ms
+
+
+class Noting:
+    """The library, but for one entry point, which notes its arguments and launches nothing."""
+
+    def __init__(self, name):
+        self._lib, self._name, self.args = _lib.load(), name, None
+
+    def __getattr__(self, name):
+        if name != self._name:
+            return getattr(self._lib, name)
+
+        def note(*args):
+            self.args = args
+            return 0
+        return note
+
+
+def held_stream(cuda):
+    s = torch.cuda.Stream(cuda)
+    with torch.cuda.stream(s):
+        torch.cuda._sleep(HOLD)
+    return s
+
+
+def handed_out_again(sizes, cuda):
+    """Pointers that the current stream's next allocations of these sizes get."""
+    tensors = [torch.empty(size, dtype=torch.uint8, device=cuda) for size in sizes for _ in range(4)]
+    return {t.data_ptr() for t in tensors}
+
+
+def test_subset_memory_outlives_the_call(cuda, monkeypatch):
+    g = graphs.erdos_renyi(60000, 8.0, 5, cuda)
+    v = torch.arange(80000, device=cuda, dtype=torch.int32)[::2] % g.n       # 40,000 vertices
+    v = torch.stack([v, v], 1)[:, 0]                                         # not contiguous
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    lib = Noting("gtc_count_subset_ws")
+    monkeypatch.setattr(api._lib, "load", lambda: lib)
+    s = held_stream(cuda)
+    out = api.count_subset(g.off, g.ind, v, stream=s)
+    ws, ws_bytes = lib.args[8], lib.args[9]
+    vertices, count = lib.args[5], lib.args[6]
+    assert lib.args[7] == out.data_ptr() and count == 40000
+    del out
+    again = handed_out_again([ws_bytes, 4 * count, 8 * count], cuda)
+    assert not s.query(), "the stream was not held back"
+    assert ws not in again and vertices not in again and lib.args[7] not in again
+
+
+def test_subset_on_a_side_stream(cuda):
+    """The current stream allocates and overwrites memory of the same sizes meanwhile, and is
+    itself behind when the call is made."""
+    g = graphs.rmat(16, 8, 3, device=cuda)
+    v = torch.randperm(g.n, device=cuda, generator=torch.Generator(cuda).manual_seed(1))
+    v = torch.stack([v[:40000].to(torch.int32)] * 2, 1)[:, 0]
+    r, _, _, _ = oracle.per_vertex(g.off.cpu().numpy(), g.ind.cpu().numpy())
+    want = r[v.cpu().numpy()]
+    size = api.TriangleCounter(cuda).workspace_bytes(g.n, g.nnz, 64) + 256
+    torch.cuda.synchronize()
+    s = torch.cuda.Stream(cuda)
+    torch.cuda._sleep(HOLD)
+    outs = []
+    for _ in range(4):
+        outs.append(api.count_subset(g.off, g.ind, v, stream=s))
+        junk = [torch.full((k,), 0x5a, dtype=torch.uint8, device=cuda)
+                for k in (size, 4 * v.numel(), 8 * v.numel())]
+        del junk
+    s.synchronize()
+    for out in outs:
+        assert np.array_equal(out.cpu().numpy(), want)
