@@ -29,6 +29,7 @@ __all__ = [
     "validate_csr", "kernelCall", "GTCError",
 ]
 
+_AS_IS = contextlib.nullcontext()
 _MODES = {"plain": MODE_PLAIN, "oriented": MODE_ORIENTED}
 
 
@@ -42,6 +43,15 @@ def _stream_handle(stream) -> int | None:
     return stream.cuda_stream or None
 
 
+def _torch_stream(stream, device) -> torch.cuda.Stream:
+    """The torch stream of anything that has a cuda_stream handle."""
+    if isinstance(stream, torch.cuda.Stream):
+        return stream
+    handle = stream.cuda_stream
+    return (torch.cuda.ExternalStream(handle, device=device) if handle
+            else torch.cuda.default_stream(device))
+
+
 def _allocating_on(stream, device):
     """Context in which torch allocates on the stream that a call launches on.
     The caching allocator hands a block out again in the order of the stream it
@@ -49,19 +59,41 @@ def _allocating_on(stream, device):
     would be somebody else's while the kernels still use it, and a block could
     be handed to them while earlier work of its own stream is still to come."""
     if stream is None:
-        return contextlib.nullcontext()
-    if not isinstance(stream, torch.cuda.Stream):
-        handle = stream.cuda_stream
-        stream = (torch.cuda.ExternalStream(handle, device=device) if handle
-                  else torch.cuda.default_stream(device))
-    return torch.cuda.stream(stream)
+        return _AS_IS
+    return torch.cuda.stream(_torch_stream(stream, device))
 
 
-def _hand_out(t: torch.Tensor | None, stream) -> None:
-    """t, allocated on the launch stream, goes to a caller who reads it (having
-    waited) on the current one: its block stays taken until that has passed."""
-    if stream is not None and t is not None:
-        t.record_stream(torch.cuda.current_stream(t.device))
+def _hand_out(stream, *tensors) -> None:
+    """The tensors, allocated on the launch stream, go to a caller who reads them
+    (having waited) on the current one: their blocks stay taken until that is
+    done with them too."""
+    if stream is not None:
+        for t in tensors:
+            if t is not None:
+                t.record_stream(torch.cuda.current_stream(t.device))
+
+
+class _Workspace:
+    """A workspace that is kept from call to call and grows."""
+
+    def __init__(self, device):
+        self.device = device
+        self.buffer: torch.Tensor | None = None
+        self._owner: int | None = None           # handle of the stream it was allocated on
+
+    def get(self, nbytes: int, stream, handle: int | None) -> torch.Tensor:
+        """At least nbytes for a call on `stream`, whose handle is given."""
+        if self.buffer is None or self.buffer.numel() < nbytes:
+            self.buffer = None
+            with _allocating_on(stream, self.device):
+                self.buffer = _alloc_workspace(nbytes, self.device)
+            self._owner = handle
+        elif handle != self._owner:
+            # the block, once dropped, stays taken until this stream is done with it too
+            if stream is None:
+                stream = torch.cuda.current_stream()
+            self.buffer.record_stream(_torch_stream(stream, self.device))
+        return self.buffer
 
 
 def _check_csr_tensors(off: torch.Tensor, ind: torch.Tensor) -> int:
@@ -128,7 +160,7 @@ class TriangleCounter:
         _lib.load()
         self.device = torch.device(device) if device is not None else torch.device(
             "cuda", torch.cuda.current_device())
-        self._ws: torch.Tensor | None = None
+        self._work = _Workspace(self.device)
 
     def workspace_bytes(self, n: int, nnz: int, off_bits: int, mode: str = "plain") -> int:
         out = ctypes.c_size_t(0)
@@ -136,24 +168,20 @@ class TriangleCounter:
               "gtc_workspace_size")
         return int(out.value)
 
-    def _workspace(self, nbytes: int) -> torch.Tensor:
-        if self._ws is None or self._ws.numel() < nbytes:
-            self._ws = None
-            # 256-byte alignment: torch's caching allocator returns 512-aligned blocks
-            self._ws = _alloc_workspace(nbytes, self.device)
-        return self._ws
+    def _workspace(self, nbytes: int, stream=None) -> torch.Tensor:
+        return self._work.get(nbytes, stream, _stream_handle(stream))
 
     def release(self) -> None:
         """Drop the cached workspace (it is re-allocated by the next count)."""
-        self._ws = None
+        self._work.buffer = None
 
     def check_status(self, stream=None) -> None:
         """Device-side error report of the last count on this counter (waits
         for `stream`): raises GTCError(GTC_ERR_INVALID_CSR) if that count met
         a neighbour id outside [0, n), which the kernels skip instead of
         dereferencing."""
-        if self._ws is not None:
-            _check_workspace_status(self._ws, stream)
+        if self._work.buffer is not None:
+            _check_workspace_status(self._work.buffer, stream)
 
     def count(self, off: torch.Tensor, ind: torch.Tensor, mode: str = "plain",
               outputs=("r", "t", "lcc"), out: TriangleCounts | None = None,
@@ -173,21 +201,24 @@ class TriangleCounter:
         if out is None:
             dev = off.device
             want = set(outputs) if mode == "plain" else set()
-            out = TriangleCounts(
-                r=torch.empty(n, dtype=torch.int64, device=dev) if "r" in want else None,
-                t=torch.empty(n, dtype=torch.int64, device=dev) if "t" in want else None,
-                lcc=torch.empty(n, dtype=torch.float64, device=dev) if "lcc" in want else None,
-                global_counts=torch.empty(3, dtype=torch.int64, device=dev),
-            )
+            with _allocating_on(stream, dev):
+                out = TriangleCounts(
+                    r=torch.empty(n, dtype=torch.int64, device=dev) if "r" in want else None,
+                    t=torch.empty(n, dtype=torch.int64, device=dev) if "t" in want else None,
+                    lcc=torch.empty(n, dtype=torch.float64, device=dev) if "lcc" in want else None,
+                    global_counts=torch.empty(3, dtype=torch.int64, device=dev),
+                )
+            _hand_out(stream, out.r, out.t, out.lcc, out.global_counts)
         ws_bytes = self.workspace_bytes(n, nnz, off_bits, mode)
-        ws = self._workspace(ws_bytes)
+        handle = _stream_handle(stream)
+        ws = self._work.get(ws_bytes, stream, handle)
         tun = None
         if tuning:
             tun = _lib.Tuning(**{k: int(v) for k, v in tuning.items()})
         st = _lib.load().gtc_count_tuned(
             off.data_ptr(), off_bits, ind.data_ptr() if nnz else None, n, nnz, _MODES[mode],
             _ptr(out.r), _ptr(out.t), _ptr(out.lcc), _ptr(out.global_counts),
-            ws.data_ptr(), ws.numel(), _stream_handle(stream),
+            ws.data_ptr(), ws.numel(), handle,
             ctypes.byref(tun) if tun is not None else None)
         check(st, "gtc_count")
         return out
@@ -237,7 +268,7 @@ def count_subset(off: torch.Tensor, ind: torch.Tensor, vertices: torch.Tensor,
                 ws = _alloc_workspace(need.value, off.device)
             except GTCError:
                 pass                      # without a workspace: row by row
-    _hand_out(out, stream)
+    _hand_out(stream, out)
     if ws is None:
         check(lib.gtc_count_subset(off.data_ptr(), off_bits, ind.data_ptr(),
                                    vertices.data_ptr(), vertices.numel(), out.data_ptr(),
@@ -255,8 +286,9 @@ def validate_csr(off: torch.Tensor, ind: torch.Tensor, stream=None) -> tuple[int
     off_bits = _check_csr_tensors(off, ind)
     n, nnz = off.numel() - 1, ind.numel()
     lib = _lib.load()
-    ws = torch.empty(lib.gtc_validate_workspace_size(n, nnz), dtype=torch.uint8,
-                     device=off.device)
+    with _allocating_on(stream, off.device):
+        ws = torch.empty(lib.gtc_validate_workspace_size(n, nnz), dtype=torch.uint8,
+                         device=off.device)
     reason = ctypes.c_int32(-1)
     check(lib.gtc_validate_csr(off.data_ptr(), off_bits, ind.data_ptr() if nnz else None, n, nnz,
                                ws.data_ptr(), ws.numel(), ctypes.byref(reason),

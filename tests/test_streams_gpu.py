@@ -86,3 +86,56 @@ def test_subset_on_a_side_stream(cuda):
     s.synchronize()
     for out in outs:
         assert np.array_equal(out.cpu().numpy(), want)
+
+
+def test_one_shot_count_memory_outlives_the_call(cuda, monkeypatch):
+    g = graphs.erdos_renyi(60000, 8.0, 5, cuda)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    lib = Noting("gtc_count_tuned")
+    monkeypatch.setattr(api._lib, "load", lambda: lib)
+    s = held_stream(cuda)
+    out = api.count_triangles(g.off, g.ind, stream=s)
+    r, t, lcc, total, ws, ws_bytes = lib.args[6:12]
+    assert r == out.r.data_ptr() and total == out.global_counts.data_ptr()
+    del out
+    again = handed_out_again([ws_bytes, 8 * g.n, 24], cuda)
+    assert not s.query(), "the stream was not held back"
+    assert not {r, t, lcc, total, ws} & again
+
+
+def test_counter_workspace_dropped_while_another_stream_uses_it(cuda, monkeypatch):
+    """A workspace allocated on the current stream, used on s, then outgrown."""
+    a, b = graphs.erdos_renyi(60000, 8.0, 5, cuda), graphs.erdos_renyi(90000, 8.0, 5, cuda)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    lib = Noting("gtc_count_tuned")
+    monkeypatch.setattr(api._lib, "load", lambda: lib)
+    counter = api.TriangleCounter(cuda)
+    counter.count(a.off, a.ind, mode="oriented")
+    s = held_stream(cuda)
+    counter.count(a.off, a.ind, mode="oriented", stream=s)
+    ws, ws_bytes = lib.args[10], lib.args[11]
+    counter.count(b.off, b.ind, mode="oriented")
+    assert lib.args[10] != ws
+    again = handed_out_again([ws_bytes], cuda)
+    assert not s.query(), "the stream was not held back"
+    assert ws not in again
+
+
+def test_one_shot_count_on_a_side_stream(cuda):
+    g = graphs.rmat(14, 8, 3, device=cuda)
+    r, t, _, _ = oracle.per_vertex(g.off.cpu().numpy(), g.ind.cpu().numpy())
+    size = api.TriangleCounter(cuda).workspace_bytes(g.n, g.nnz, 64)
+    torch.cuda.synchronize()
+    s = torch.cuda.Stream(cuda)
+    torch.cuda._sleep(HOLD)
+    outs = []
+    for _ in range(4):
+        outs.append(api.count_triangles(g.off, g.ind, stream=s))
+        assert api.validate_csr(g.off, g.ind, stream=s)[0] == 0
+        junk = [torch.full((k,), 0x5a, dtype=torch.uint8, device=cuda) for k in (size, 8 * g.n, 256)]
+        del junk
+    s.synchronize()
+    for out in outs:
+        assert np.array_equal(out.r.cpu().numpy(), r) and np.array_equal(out.t.cpu().numpy(), t)
