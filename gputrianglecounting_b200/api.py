@@ -387,31 +387,40 @@ class BatchCounter:
         _lib.load()
         self.device = torch.device(device) if device is not None else torch.device(
             "cuda", torch.cuda.current_device())
-        self._ws: torch.Tensor | None = None
+        self._work = _Workspace(self.device)
         self._pack_scratch: torch.Tensor | None = None
         self._pack_staging: torch.Tensor | None = None
+        self._pack_done: torch.cuda.Event | None = None   # the last pack's kernels
 
     def workspace_bytes(self, num_graphs: int, total_n: int, total_nnz: int) -> int:
         return batch_workspace_bytes(num_graphs, total_n, total_nnz)
 
     def reserve(self, num_graphs: int, total_n: int, total_nnz: int) -> None:
         """Allocate the workspace up front (e.g. before a CUDA-graph capture)."""
-        need = self.workspace_bytes(num_graphs, total_n, total_nnz)
-        if self._ws is None or self._ws.numel() < need:
-            self._ws = None
-            self._ws = _alloc_workspace(need, self.device)
+        self._work.get(self.workspace_bytes(num_graphs, total_n, total_nnz), None,
+                       _stream_handle(None))
 
     def release(self) -> None:
         """Drop the cached workspace and pack buffers."""
-        self._ws = None
+        self._work.buffer = None
+        self._drop_pack_buffers()
+
+    def __del__(self):
+        with contextlib.suppress(Exception):     # not half made, nor at the interpreter's end
+            self._drop_pack_buffers()
+
+    def _drop_pack_buffers(self) -> None:
+        if self._pack_done is not None:
+            # the staging buffer may still feed a copy, the scratch a kernel, on any stream
+            self._pack_done.synchronize()
         self._pack_scratch = None
         self._pack_staging = None
 
     def check_status(self, stream=None) -> None:
         """As TriangleCounter.check_status, for the last batch counted here
         (a local id outside its graph's [0, n_g) raises GTC_ERR_INVALID_CSR)."""
-        if self._ws is not None:
-            _check_workspace_status(self._ws, stream)
+        if self._work.buffer is not None:
+            _check_workspace_status(self._work.buffer, stream)
 
     def alloc_outputs(self, batch: BatchCSR, outputs=("r", "lcc", "graph_T")) -> BatchCounts:
         dev, n, G = self.device, batch.total_n, batch.num_graphs
@@ -424,15 +433,18 @@ class BatchCounter:
     def count(self, batch: BatchCSR, outputs=("r", "lcc", "graph_T"), out: BatchCounts | None = None,
               tuning: dict | None = None, stream=None) -> BatchCounts:
         G, n, nnz = batch.num_graphs, batch.total_n, batch.total_nnz
-        self.reserve(G, n, nnz)
+        handle = _stream_handle(stream)
+        ws = self._work.get(self.workspace_bytes(G, n, nnz), stream, handle)
         if out is None:
-            out = self.alloc_outputs(batch, outputs)
+            with _allocating_on(stream, self.device):
+                out = self.alloc_outputs(batch, outputs)
+            _hand_out(stream, out.r, out.t, out.lcc, out.graph_T)
         tun = _lib.Tuning(**{k: int(v) for k, v in tuning.items()}) if tuning else None
         check(_lib.load().gtc_count_batch(
             G, batch.vstart.data_ptr(), batch.off.data_ptr(),
             batch.ind.data_ptr() if nnz else None, n, nnz, _ptr(out.r), _ptr(out.t),
-            _ptr(out.lcc), _ptr(out.graph_T), self._ws.data_ptr(), self._ws.numel(),
-            ctypes.byref(tun) if tun is not None else None, _stream_handle(stream)),
+            _ptr(out.lcc), _ptr(out.graph_T), ws.data_ptr(), ws.numel(),
+            ctypes.byref(tun) if tun is not None else None, handle),
             "gtc_count_batch")
         return out
 
@@ -441,23 +453,32 @@ class BatchCounter:
         G = len(graphs)
         lib = _lib.load()
         need = int(lib.gtc_batch_pack_scratch_bytes(G))
+        handle = _stream_handle(stream)
         if self._pack_scratch is None or self._pack_scratch.numel() < need:
-            self._pack_scratch = torch.empty(need, dtype=torch.uint8, device=self.device)
+            self._drop_pack_buffers()
+            with _allocating_on(stream, self.device):
+                self._pack_scratch = torch.empty(need, dtype=torch.uint8, device=self.device)
             self._pack_staging = torch.empty(need, dtype=torch.uint8).pin_memory()
-        else:
-            # the staging buffer may still feed an earlier copy
-            torch.cuda.current_stream(self.device).synchronize()
+        elif self._pack_done is not None:
+            # the staging buffer may still feed an earlier copy, on any stream
+            self._pack_done.synchronize()
         offs = (ctypes.c_void_p * max(G, 1))(*[g.off.data_ptr() for g in graphs])
         inds = (ctypes.c_void_p * max(G, 1))(*[g.ind.data_ptr() for g in graphs])
         ns = (ctypes.c_int64 * max(G, 1))(*[g.n for g in graphs])
         nnzs = (ctypes.c_int64 * max(G, 1))(*[g.nnz for g in graphs])
         total_n, total_nnz = sum(g.n for g in graphs), sum(g.nnz for g in graphs)
-        vstart = torch.empty(G + 1, dtype=torch.int64, device=self.device)
-        off = torch.empty(total_n + 1, dtype=torch.int64, device=self.device)
-        ind = torch.empty(max(total_nnz, 1), dtype=torch.int32, device=self.device)[:total_nnz]
+        with _allocating_on(stream, self.device):
+            vstart = torch.empty(G + 1, dtype=torch.int64, device=self.device)
+            off = torch.empty(total_n + 1, dtype=torch.int64, device=self.device)
+            ind = torch.empty(max(total_nnz, 1), dtype=torch.int32, device=self.device)[:total_nnz]
+        _hand_out(stream, vstart, off, ind)
         check(lib.gtc_batch_pack(G, offs, inds, ns, nnzs, vstart.data_ptr(), off.data_ptr(),
                                  ind.data_ptr() if total_nnz else None,
                                  self._pack_scratch.data_ptr(), self._pack_scratch.numel(),
-                                 self._pack_staging.data_ptr(), _stream_handle(stream)),
+                                 self._pack_staging.data_ptr(), handle),
               "gtc_batch_pack")
+        if self._pack_done is None:
+            self._pack_done = torch.cuda.Event()
+        self._pack_done.record(torch.cuda.current_stream(self.device) if stream is None
+                               else _torch_stream(stream, self.device))
         return BatchCSR(vstart, off, ind)

@@ -139,3 +139,37 @@ def test_one_shot_count_on_a_side_stream(cuda):
     s.synchronize()
     for out in outs:
         assert np.array_equal(out.r.cpu().numpy(), r) and np.array_equal(out.t.cpu().numpy(), t)
+
+
+def test_batch_memory_outlives_the_call(cuda, monkeypatch):
+    gs = [graphs.erdos_renyi(20000, 8.0, k, cuda) for k in range(3)]
+    batch = graphs.concat_graphs(gs, cuda)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    lib = Noting("gtc_count_batch")
+    monkeypatch.setattr(api._lib, "load", lambda: lib)
+    s = held_stream(cuda)
+    out = api.BatchCounter(cuda).count(batch, stream=s)
+    r, _, lcc, total, ws, ws_bytes = lib.args[6:12]
+    assert r == out.r.data_ptr() and total == out.graph_T.data_ptr()
+    del out
+    again = handed_out_again([ws_bytes, 8 * batch.total_n, 24], cuda)
+    assert not s.query(), "the stream was not held back"
+    assert not {r, lcc, total, ws} & again
+
+
+def test_packs_in_flight_keep_their_staging(cuda):
+    """Packs on a stream that is held back, by one counter and by counters that are dropped at
+    once: each copies the graphs that it was given."""
+    gs = [graphs.erdos_renyi(3000 + 100 * k, 6.0, k, cuda) for k in range(6)]
+    torch.cuda.synchronize()
+    counter = api.BatchCounter(cuda)
+    s = held_stream(cuda)
+    one = [counter.pack(gs[k:k + 2], stream=s) for k in (0, 2, 4)]
+    other = [api.BatchCounter(cuda).pack(gs[k:k + 2], stream=s) for k in (0, 2, 4)]
+    s.synchronize()
+    for k, a, b in zip((0, 2, 4), one, other):
+        want = graphs.concat_graphs(gs[k:k + 2], cuda)
+        for got in (a, b):
+            assert torch.equal(got.vstart, want.vstart) and torch.equal(got.off, want.off)
+            assert torch.equal(got.ind, want.ind)
