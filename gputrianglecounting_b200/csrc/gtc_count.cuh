@@ -484,6 +484,7 @@ __device__ void core_block_row(const Data &w, const VInfo &vi, int core, const C
             __syncthreads();
         }
     }
+    // at most kCoreMax members: their pairs, 2^29, fit 32 bits
     const unsigned int ws = warp_sum(mine);
     if (lane == 0 && ws) atomicAdd(&sm.total, ws);
     __syncthreads();
@@ -1126,7 +1127,7 @@ struct TableBlockSmem {
     unsigned int cnt[1 << kTableLog2];
     unsigned int bits[1 << (kTableLog2 - 2)];
     int next;
-    unsigned int total;
+    unsigned long long total;                     // a row's triangles, of all its chunks
 };
 
 template <typename Pos>
@@ -1285,7 +1286,12 @@ __device__ __forceinline__ void table_warp_row(const Data &w, int v, const VInfo
 }
 
 // A longer one by the block, at most kMemberChunk members in the table at a
-// time (a quarter full at most).
+// time (a quarter full at most).  A row of f members has up to f (f - 1) / 2
+// triangles, more than 32 bits hold from f = 92,683 on, so its total is 64 bits
+// wide.  What a warp finds in one chunk is at most kMemberChunk per list, and f
+// stays below 2^22 (a degree that no one of f others is below, or that is at most
+// twice the mean and 16, takes f * f / 2 entries, 2^43): 32 bits hold it, and a
+// member's count, at most f, as well.
 template <bool PV, bool BATCH, typename Pos>
 __device__ void table_block_row(const Data &w, int v, const VInfo &vi, const GraphRec *rec,
                                 TableBlockSmem &sm, unsigned long long &tri)
@@ -1322,11 +1328,11 @@ __device__ void table_block_row(const Data &w, int v, const VInfo &vi, const Gra
             for (int k = threadIdx.x; k < slots; k += kThreads)
                 if (sm.cnt[k]) credit(w, v0, ls.shift, sm.key[k], sm.cnt[k]);
         const unsigned int ws = warp_sum(mine);
-        if (lane == 0 && ws) atomicAdd(&sm.total, ws);
+        if (lane == 0 && ws) atomicAdd(&sm.total, (unsigned long long)ws);
         __syncthreads();
     }
     if (threadIdx.x == 0 && sm.total) {
-        if (PV) add64(&w.tacc[v], sm.total);
+        if (PV) atomicAdd(&w.tacc[v], sm.total);
         tri += sm.total;
     }
 }
