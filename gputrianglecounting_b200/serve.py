@@ -176,6 +176,10 @@ class CountServer:
         return True
 
     def _finish(self, slot: _Slot, now: float) -> list[Request]:
+        if self.keep:
+            # the copies below run on the current stream, and the slot's next batch
+            # may get the memory that they read
+            slot.out.r.record_stream(torch.cuda.current_stream(self.device))
         T = slot.out.graph_T.cpu().numpy()
         vstart = slot.batch.vstart.cpu().numpy() if self.keep else None
         for i, req in enumerate(slot.requests):

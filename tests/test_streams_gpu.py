@@ -9,7 +9,7 @@ import numpy as np
 import pytest
 import torch
 
-from gputrianglecounting_b200 import _lib, api, graphs
+from gputrianglecounting_b200 import _lib, api, graphs, serve
 from oracle import oracle
 
 pytestmark = pytest.mark.gpu
@@ -173,3 +173,30 @@ def test_packs_in_flight_keep_their_staging(cuda):
         for got in (a, b):
             assert torch.equal(got.vstart, want.vstart) and torch.equal(got.off, want.off)
             assert torch.equal(got.ind, want.ind)
+
+
+def test_served_results_are_copied_before_the_slot_is_reused(cuda):
+    """The copies of a finished batch's r wait on a held-back stream while the slot's stream
+    allocates and overwrites memory of the same size."""
+    gs = [graphs.erdos_renyi(20000, 8.0, k, cuda) for k in range(3)]
+    server = serve.CountServer(gs, cuda, slots=1, keep_vertex_results=True)
+    slot = server.slots[0]
+    reqs = [serve.Request(k, k, 0.0, g.n, g.nnz) for k, g in enumerate(gs)]
+    torch.cuda.synchronize()
+    assert server._launch(slot, reqs)
+    slot.stream.synchronize()
+    want, size = slot.out.r.clone(), 8 * slot.out.r.numel()
+    torch.full((size,), 0, dtype=torch.uint8, device=cuda)     # its kernel is loaded now
+    torch.cuda.synchronize()
+
+    def held(*args, _of=torch.Tensor.clone):      # the host has T, the copies are yet to run
+        torch.cuda._sleep(HOLD)
+        return _of(*args)
+    with pytest.MonkeyPatch.context() as patch:
+        patch.setattr(torch.Tensor, "clone", held)
+        server._finish(slot, 0.0)
+    with torch.cuda.stream(slot.stream):
+        junk = [torch.full((size,), 0x5a, dtype=torch.uint8, device=cuda) for _ in range(8)]
+    torch.cuda.synchronize()
+    del junk
+    assert torch.equal(torch.cat([q.r for q in reqs]), want)
