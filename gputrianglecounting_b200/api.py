@@ -249,7 +249,13 @@ def launch_plan(n: int, nnz: int, mode: str = "plain", tuning: dict | None = Non
 
 def count_subset(off: torch.Tensor, ind: torch.Tensor, vertices: torch.Tensor,
                  stream=None) -> torch.Tensor:
-    """r(v) for each listed vertex (the reference's vertex-list overload)."""
+    """r(v) for each listed vertex (the reference's vertex-list overload).
+
+    The whole graph must be a simple symmetric CSR with sorted rows, as for a
+    count: from 16,384 vertices on the whole graph is counted where an estimate
+    finds that cheaper.  The C entry point gtc_count_subset (and kernelCall's
+    `vertex`) reads the listed rows and their neighbours' rows alone.
+    """
     off_bits = _check_csr_tensors(off, ind)
     if vertices.dtype != torch.int32 or not vertices.is_cuda:
         raise TypeError("vertices must be an int32 CUDA tensor")

@@ -212,7 +212,9 @@ gtc_status gtc_count_subset(const void *d_off, int off_bits,
  * gtc_count_subset for a graph whose size is known, with a workspace.  A
  * large subset of a skewed graph costs more than a count of the whole graph
  * (65,536 of R-MAT scale 20's vertices ten times as much), so an estimate on
- * the device picks the cheaper of the two; the result is the same.
+ * the device picks the cheaper of the two; the result is the same.  The whole
+ * graph must satisfy the input contract, also outside the rows that
+ * gtc_count_subset reads.
  * gtc_subset_workspace_size writes 0 when a count of the whole graph is never
  * the cheaper way (few listed vertices); with no or too little workspace the
  * call is gtc_count_subset.  d_workspace is 256-byte aligned.  Asynchronous on
