@@ -412,8 +412,10 @@ class BatchCounter:
         self._drop_pack_buffers()
 
     def __del__(self):
-        with contextlib.suppress(Exception):     # not half made, nor at the interpreter's end
+        try:
             self._drop_pack_buffers()
+        except Exception:                        # half made, or at the interpreter's end
+            pass
 
     def _drop_pack_buffers(self) -> None:
         if self._pack_done is not None:
