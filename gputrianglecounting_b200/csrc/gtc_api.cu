@@ -8,6 +8,7 @@
 #include <cstdio>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 
 #include "gtc_core.cuh"
 #include "gtc_data.cuh"
@@ -244,16 +245,22 @@ __device__ __forceinline__ void add_out(int *o, unsigned long long x)
 //     neighbours (not much longer than v's) are looked up in the table, where
 //     finding a long w counts twice, and pairs of long neighbours are searched
 //     for, one of each two.  It writes 0 for the longer rows;
-//   * subset_hub_kernel, all blocks on every longer ("hub") row: each block
-//     sets N(v) in a shared bitmap over the row's id span and takes every
-//     gridDim.x-th neighbour, whose row its warps probe into the bitmap with
+//   * subset_hub_kernel, longer ("hub") rows: each block that takes part in a
+//     row sets N(v) in a shared bitmap over the row's id span and takes every
+//     so-manieth neighbour, whose row its warps probe into the bitmap with
 //     coalesced loads; neighbour rows longer than 2,048 entries are queued
 //     and swept afterwards by all of the block's warps in 1,024-entry pieces,
 //     so that no warp is left alone with a hub's row; block sums are added to
 //     out[k].  A row whose span exceeds the bitmap falls back to the binary
-//     search.
-// Spreading a hub over the whole GPU matters: on a power-law graph a single
-// hub's probes outnumber those of thousands of ordinary rows.
+//     search.  All blocks take part in a row of more than kSubHubMin: on a
+//     power-law graph a single hub's probes outnumber those of thousands of
+//     ordinary rows.  Lists of less than 2 kSubFew vertices give it rows from a
+//     quarter of that on, too long to be left to one block at the end; those of
+//     1,024 vertices are shared out among teams of blocks, down to a block
+//     each.  All blocks on one after another take 7 us a row however small it
+//     is (2,000 vertices of an ER 100K of mean degree 600: 14.9 ms so, 1.8 by
+//     teams, 2.3 with a table and a block each; of 20 cliques of 600, 14.0, 1.15
+//     and 0.99 ms).
 // A neighbour row is long from here on (elements), for a listed row of dv.
 __host__ __device__ __forceinline__ int subset_long(int dv)
 {
@@ -658,8 +665,9 @@ subset_hub_kernel(const OffT *__restrict__ off, const IndT *__restrict__ ind,
 {
     extern __shared__ unsigned int s_bits[];          // kSubHubBits / 32 words
     if (skip && *skip) return;
+    // all blocks' rows from the front, teams' from the end
     __shared__ long long s_hub[kSubHubThreads];
-    __shared__ int s_nhub;
+    __shared__ int s_all[kSubHubThreads / 32], s_team[kSubHubThreads / 32];
     __shared__ long long s_lo, s_hi;
     __shared__ unsigned long long s_sum;
     constexpr int kBigRows = 64, kSplit = 2048, kPiece = 1024;
@@ -669,22 +677,48 @@ subset_hub_kernel(const OffT *__restrict__ off, const IndT *__restrict__ ind,
     auto warp = cg::tiled_partition<32>(block);
     const int wid = warp.meta_group_rank(), lane = warp.thread_rank();
     constexpr int nwarps = kSubHubThreads / 32;
-    const long long stride = (long long)gridDim.x * nwarps;   // neighbours per worker step
-    // the listed vertices are scanned a chunk at a time, every thread
-    // testing one; the hubs found are then taken one after another
+    // the listed vertices are scanned a chunk at a time, every thread testing
+    // one; all blocks find the same rows in the same order
     for (long long c0 = 0; c0 < count; c0 += kSubHubThreads) {
-        if (threadIdx.x == 0) s_nhub = 0;
-        __syncthreads();
         const long long kk = c0 + threadIdx.x;
+        long long dk = 0;
         if (kk < count) {
             const long long v = (long long)vertex[kk];
-            if ((long long)off[v + 1] - (long long)off[v] > hub_min)
-                s_hub[atomicAdd(&s_nhub, 1)] = kk;
+            dk = (long long)off[v + 1] - (long long)off[v];
+        }
+        if (!__syncthreads_or(dk > hub_min)) continue;
+        const bool all = dk > kSubHubMin, team = !all && dk > hub_min;
+        const unsigned int ma = __ballot_sync(0xffffffffu, all);
+        const unsigned int mt = __ballot_sync(0xffffffffu, team);
+        if (lane == 0) {
+            s_all[wid] = __popc(ma);
+            s_team[wid] = __popc(mt);
         }
         __syncthreads();
-        const int nh = s_nhub;
-        for (int h = 0; h < nh; ++h) {
-            const long long k = s_hub[h];
+        int na = 0, nt = 0, a0 = 0, t0 = 0;
+        for (int i = 0; i < nwarps; ++i) {
+            if (i == wid) {
+                a0 = na;
+                t0 = nt;
+            }
+            na += s_all[i];
+            nt += s_team[i];
+        }
+        const unsigned int below = (1u << lane) - 1u;
+        if (all) s_hub[a0 + __popc(ma & below)] = kk;
+        if (team) s_hub[kSubHubThreads - 1 - (t0 + __popc(mt & below))] = kk;
+        __syncthreads();
+        // rows for teams: as many teams of blocks as there are rows, if there are enough blocks
+        const int blocks = nt > 0 ? max(1, (int)gridDim.x / nt) : 1;
+        const int teams = (int)gridDim.x / blocks;
+        const int mine = (int)blockIdx.x / blocks;
+        const int rows = mine < teams && mine < nt ? div_up(nt - mine, teams) : 0;
+        for (int h = 0; h < na + rows; ++h) {
+            const bool whole = h < na;
+            const long long k = s_hub[whole ? h : kSubHubThreads - 1 - (mine + (h - na) * teams)];
+            const int size = whole ? (int)gridDim.x : blocks;
+            const int rank = whole ? (int)blockIdx.x : (int)blockIdx.x % blocks;
+            const long long stride = (long long)size * nwarps;    // neighbours per step
             const long long v = (long long)vertex[k];
             const long long vb = off[v], ve = off[v + 1], dv = ve - vb;
             // the row's id span (rows are sorted, but the bitmap must not
@@ -716,51 +750,48 @@ subset_hub_kernel(const OffT *__restrict__ off, const IndT *__restrict__ ind,
                 __syncthreads();
             }
             unsigned long long acc = 0;
+            typedef typename std::make_unsigned<IndT>::type Id;
+            const Id first = (Id)lo, last = use_bits ? (Id)span : 0;
             auto sweep = [&](long long b0, long long b1) {
-                // four loads in flight per lane
-                for (long long i0 = b0; i0 < b1; i0 += 128) {
-                    long long x[4];
+                constexpr int kPer = 32 / sizeof(IndT);    // loads in flight per lane
+                for (long long i0 = b0 + lane; i0 < b1; i0 += 32 * kPer) {
+                    Id x[kPer];
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const long long i = i0 + j * 32 + lane;
-                        x[j] = i < b1 ? (long long)ind[i] - lo : -1;
-                    }
+                    for (int j = 0; j < kPer; ++j)
+                        x[j] = i0 + 32 * j < b1 ? (Id)ind[i0 + 32 * j] - first : last;
+                    unsigned int hits = 0;
 #pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        if ((unsigned long long)x[j] < span)
-                            acc += (s_bits[x[j] >> 5] >> (x[j] & 31)) & 1u;
+                    for (int j = 0; j < kPer; ++j)
+                        if (x[j] < last) hits += (s_bits[x[j] >> 5] >> (x[j] & 31)) & 1u;
+                    acc += hits;
                 }
             };
-            for (long long e = vb + blockIdx.x + (long long)gridDim.x * wid; e < ve; e += stride) {
-                const long long u = (long long)ind[e];
-                const long long ub = off[u], ue = off[u + 1], du = ue - ub;
-                if (u == v || du < 2) continue;
-                if (use_bits && du > kSplit) {
-                    // a long row is shared by the block's warps after this loop
-                    int at = 0;
-                    if (lane == 0) at = atomicAdd(&s_nbig, 1);
-                    at = warp.shfl(at, 0);
-                    if (at < kBigRows) {
-                        if (lane == 0) { s_big_b[at] = ub; s_big_e[at] = ue; }
-                        continue;
-                    }
+            // the lanes find where 32 neighbours' rows are, which the warp then takes in turn
+            for (long long e0 = vb + rank + (long long)size * wid; e0 < ve; e0 += 32 * stride) {
+                long long ub = 0, ue = 0;
+                if (e0 + lane * stride < ve) {
+                    const long long u = (long long)ind[e0 + lane * stride];
+                    ub = off[u];
+                    ue = u == v ? ub : (long long)off[u + 1];
                 }
-                if (use_bits) {
-                    // four loads in flight per lane
-                    for (long long i0 = ub; i0 < ue; i0 += 128) {
-                        long long x[4];
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const long long i = i0 + j * 32 + lane;
-                            x[j] = i < ue ? (long long)ind[i] - lo : -1;
+                unsigned int todo = __ballot_sync(0xffffffffu, ue - ub >= 2);
+                while (todo) {
+                    const int src = __ffs(todo) - 1;
+                    todo &= todo - 1;
+                    const long long b0 = __shfl_sync(0xffffffffu, ub, src);
+                    const long long b1 = __shfl_sync(0xffffffffu, ue, src);
+                    if (use_bits && b1 - b0 > kSplit) {
+                        // a long row is shared by the block's warps after this loop
+                        int at = 0;
+                        if (lane == 0) at = atomicAdd(&s_nbig, 1);
+                        at = warp.shfl(at, 0);
+                        if (at < kBigRows) {
+                            if (lane == 0) { s_big_b[at] = b0; s_big_e[at] = b1; }
+                            continue;
                         }
-#pragma unroll
-                        for (int j = 0; j < 4; ++j)
-                            if ((unsigned long long)x[j] < span)
-                                acc += (s_bits[x[j] >> 5] >> (x[j] & 31)) & 1u;
                     }
-                } else {
-                    acc += search_shorter(ind, vb, dv, ub, du, lane);
+                    if (use_bits) sweep(b0, b1);
+                    else acc += search_shorter(ind, vb, dv, b0, b1 - b0, lane);
                 }
             }
             if (use_bits) {
@@ -779,7 +810,6 @@ subset_hub_kernel(const OffT *__restrict__ off, const IndT *__restrict__ ind,
             if (threadIdx.x == 0 && s_sum) add_out(&out[k], s_sum);
             __syncthreads();                       // s_bits, s_lo and s_sum are reused
         }
-        __syncthreads();                           // every thread has read s_nhub
     }
 }
 
