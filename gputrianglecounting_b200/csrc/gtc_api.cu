@@ -187,9 +187,9 @@ gtc_status run_validate(const OffT *off, const int *ind, long long n, long long 
 constexpr int kSubThreads = 256;
 constexpr int kSubWarpRow = 128;                  // longest listed row that a warp takes
 constexpr int kSubSlots = 4096;
-constexpr long long kSubHubMin = kSubSlots / 2;   // longer listed rows go to the hub kernel
-constexpr int kSubClaim = 32;                     // listed vertices a block takes at a time
-constexpr long long kSubFew = 8192;               // fewer listed vertices take a block each
+constexpr long long kSubHubMin = kSubSlots / 2;   // longer listed rows are hubs
+constexpr int kSubClaim = 32;                     // most listed vertices that a block takes
+constexpr long long kSubFew = 8192;               // of fewer a warp takes half as long rows
 constexpr int kSubHubThreads = 1024;
 constexpr long long kSubHubBits = 1ll << 20;      // bitmap span of a hub row (128 KiB)
 
@@ -238,13 +238,15 @@ __device__ __forceinline__ void add_out(int *o, unsigned long long x)
 // are the only ones read, as in the reference's vertex-list kernel,
 // src/clusteringCount.cu:266-312).  Edges with u == v or a list shorter
 // than two are skipped like the reference (:292-294).  Two kernels:
-//   * subset_kernel, rows of at most kSubHubMin neighbours, a warp for those
-//     of at most kSubWarpRow, a block for the others.  N(v) goes to a shared
-//     hash table.  The sum counts adjacent pairs (u, w) of N(v) both ways
-//     round, so a pair need be found from one end only: the rows of the short
-//     neighbours (not much longer than v's) are looked up in the table, where
-//     finding a long w counts twice, and pairs of long neighbours are searched
-//     for, one of each two.  It writes 0 for the longer rows;
+//   * subset_kernel, rows that are no hubs, a warp for those of at most
+//     kSubWarpRow (half of that in lists of less than kSubFew), a block for the
+//     others and for every row where the list has no more vertices than there
+//     are blocks at a time.  N(v) goes to a shared hash table.  The sum counts
+//     adjacent pairs (u, w) of N(v) both ways round, so a pair need be found
+//     from one end only: the rows of the short neighbours (not much longer than
+//     v's) are looked up in the table, where finding a long w counts twice, and
+//     pairs of long neighbours are searched for, one of each two.  It writes 0
+//     for the hubs;
 //   * subset_hub_kernel, longer ("hub") rows: each block that takes part in a
 //     row sets N(v) in a shared bitmap over the row's id span and takes every
 //     so-manieth neighbour, whose row its warps probe into the bitmap with
@@ -270,14 +272,12 @@ __host__ __device__ __forceinline__ int subset_long(int dv)
 template <typename IndT>
 struct SubWarpSmem {
     IndT key[4 * kSubWarpRow];
-    unsigned char far[4 * kSubWarpRow];           // the slot's member is a long neighbour
     unsigned char longs[kSubWarpRow];             // index of each long neighbour in the row
 };
 
 template <typename IndT>
 struct SubBlockSmem {
     IndT key[kSubSlots];
-    unsigned char far[kSubSlots];
     unsigned short longs[kSubHubMin];             // index of each long neighbour in the row,
     unsigned short mids[kSubHubMin];              // of each short one of over kSubList entries
 };
@@ -302,32 +302,37 @@ __device__ __forceinline__ bool cas_empty(IndT *slot, IndT key)
                      (unsigned long long)key) == ~0ull;
 }
 
-// N(v)'s table: slot of w, or -1.
+// In N(v)'s table a long neighbour has the top bit set: a byte beside the key
+// cost a second shared load per hit.
 template <typename IndT>
-__device__ __forceinline__ int sub_find(const IndT *key, int lg, IndT w)
+constexpr IndT kSubFar = (IndT)1 << (8 * sizeof(IndT) - 1);
+
+// What finding w in N(v)'s table counts: 0, 1, or 2 for a long neighbour.
+template <typename IndT>
+__device__ __forceinline__ unsigned int sub_find(const IndT *key, int lg, IndT w)
 {
     const unsigned int mask = (1u << lg) - 1u;
     unsigned int s = hash_slot((int)w, lg);
     IndT k = key[s];
-    while (k != w && k != (IndT)-1) {
+    while ((k & ~kSubFar<IndT>) != w && k != (IndT)-1) {
         s = (s + 1) & mask;
         k = key[s];
     }
-    return k == w ? (int)s : -1;
+    return k == (IndT)-1 ? 0u : (k < 0 ? 2u : 1u);
 }
 
-// Neighbour e of v, to the table; true for a long one.
+// Neighbour u of v, to the table; true for a long one.  The largest id is never
+// taken for one (with the bit it is an empty slot): its row is looked up whole.
 template <typename OffT, typename IndT>
 __device__ __forceinline__ bool sub_insert(const OffT *__restrict__ off, IndT u, long long v,
-                                           int dv, IndT *key, unsigned char *far, int lg, int &du)
+                                           int dv, IndT *key, int lg, int &du)
 {
     const unsigned int mask = (1u << lg) - 1u;
     const long long d = (long long)off[u + 1] - (long long)off[u];
-    const bool lng = u != v && d > subset_long(dv);
+    const bool lng = u != v && d > subset_long(dv) && u != ~kSubFar<IndT>;
     du = u != v && !lng ? (int)d : 0;
     unsigned int s = hash_slot((int)u, lg);
-    while (!cas_empty(&key[s], u)) s = (s + 1) & mask;
-    far[s] = lng;
+    while (!cas_empty(&key[s], lng ? (IndT)(u | kSubFar<IndT>) : u)) s = (s + 1) & mask;
     return lng;
 }
 
@@ -337,7 +342,7 @@ constexpr int kSubList = 64;                      // longer rows are looked up o
 // long w counts twice.
 template <typename IndT>
 __device__ __forceinline__ unsigned int sub_row(const IndT *__restrict__ row, int len,
-                                                const IndT *key, const unsigned char *far, int lg)
+                                                const IndT *key, int lg)
 {
     constexpr int kPer = 4;
     unsigned int acc = 0;
@@ -348,8 +353,7 @@ __device__ __forceinline__ unsigned int sub_row(const IndT *__restrict__ row, in
 #pragma unroll
         for (int j = 0; j < kPer; ++j) {
             if (i0 + 32 * j >= len) break;
-            const int s = sub_find(key, lg, x[j]);
-            if (s >= 0) acc += 1u + far[s];
+            acc += sub_find(key, lg, x[j]);
         }
     }
     return acc;
@@ -361,7 +365,7 @@ __device__ __forceinline__ unsigned int sub_row(const IndT *__restrict__ row, in
 template <typename OffT, typename IndT>
 __device__ __forceinline__ unsigned long long
 sub_stream(const OffT *__restrict__ off, const IndT *__restrict__ ind, bool has, IndT u,
-           long long v, int dv, const IndT *key, const unsigned char *far, int lg, bool all)
+           long long v, int dv, const IndT *key, int lg, bool all)
 {
     constexpr int kPer = 4;
     const int lane = threadIdx.x & 31;
@@ -370,7 +374,7 @@ sub_stream(const OffT *__restrict__ off, const IndT *__restrict__ ind, bool has,
     if (has && u != v) {
         ub = (long long)off[u];
         const long long d = (long long)off[u + 1] - ub;
-        du = d >= 2 && d <= subset_long(dv) ? (int)d : 0;
+        du = d >= 2 && (d <= subset_long(dv) || u == ~kSubFar<IndT>) ? (int)d : 0;
     }
     unsigned long long acc = 0;
     unsigned int rows = all ? __ballot_sync(0xffffffffu, du > kSubList) : 0u;
@@ -378,7 +382,7 @@ sub_stream(const OffT *__restrict__ off, const IndT *__restrict__ ind, bool has,
         const int src = __ffs(rows) - 1;
         rows &= rows - 1;
         acc += sub_row(ind + __shfl_sync(0xffffffffu, ub, src),
-                       __shfl_sync(0xffffffffu, du, src), key, far, lg);
+                       __shfl_sync(0xffffffffu, du, src), key, lg);
     }
     const int len = du <= kSubList ? du : 0;
     const int incl = warp_incl_scan(len);
@@ -394,8 +398,7 @@ sub_stream(const OffT *__restrict__ off, const IndT *__restrict__ ind, bool has,
         }
 #pragma unroll
         for (int j = 0; j < kPer; ++j) {
-            const int s = sub_find(key, lg, x[j]);
-            if (s >= 0) acc += 1u + far[s];
+            acc += sub_find(key, lg, x[j]);
         }
     }
     return acc;
@@ -456,7 +459,7 @@ sub_pairs(const OffT *__restrict__ off, const IndT *__restrict__ ind, long long 
 }
 
 template <typename OffT, typename IndT, typename VtxT, typename OutT>
-__global__ void __launch_bounds__(kSubThreads)
+__global__ void __launch_bounds__(kSubThreads, 4)
 subset_kernel(const OffT *__restrict__ off, const IndT *__restrict__ ind,
               const VtxT *__restrict__ vertex, long long count, OutT *__restrict__ out,
               const int *__restrict__ skip, int claim, int warp_row, int hub_min)
@@ -474,25 +477,35 @@ subset_kernel(const OffT *__restrict__ off, const IndT *__restrict__ ind,
         __syncthreads();
         for (int i = threadIdx.x; i < dv; i += kSubThreads) {
             int du;
-            if (sub_insert(off, ind[vb + i], v, dv, sm.block.key, sm.block.far, lg, du))
+            if (sub_insert(off, ind[vb + i], v, dv, sm.block.key, lg, du))
                 sm.block.longs[atomicAdd(&sm.n_long, 1)] = (unsigned short)i;
             else if (du > kSubList)
                 sm.block.mids[atomicAdd(&sm.n_mid, 1)] = (unsigned short)i;
         }
         __syncthreads();
         unsigned long long acc = 0;
-        for (int i = warp; i < sm.n_mid; i += kSubThreads / 32) {
-            const IndT u = ind[vb + sm.block.mids[i]];
-            const long long ub = off[u];
-            acc += sub_row(ind + ub, (int)((long long)off[u + 1] - ub), sm.block.key,
-                           sm.block.far, lg);
+        // the lanes find where 32 neighbours' rows are, which the warp then takes in turn
+        constexpr int kWarps = kSubThreads / 32;
+        for (int i0 = warp; i0 < sm.n_mid; i0 += 32 * kWarps) {
+            long long ub = 0;
+            int du = 0;
+            if (i0 + kWarps * lane < sm.n_mid) {
+                const IndT u = ind[vb + sm.block.mids[i0 + kWarps * lane]];
+                ub = off[u];
+                du = (int)((long long)off[u + 1] - ub);
+            }
+            const int n = min(32, div_up(sm.n_mid - i0, kWarps));
+            for (int k = 0; k < n; ++k)
+                acc += sub_row(ind + __shfl_sync(0xffffffffu, ub, k),
+                               __shfl_sync(0xffffffffu, du, k), sm.block.key, lg);
         }
         // a share of the neighbours that keeps all warps busy on a short row
-        const int each = min(32, max(4, div_up(dv, kSubThreads / 32)));
-        for (int i = warp * each; i < dv; i += each * (kSubThreads / 32)) {
+        const int each = min(32, max(4, div_up(dv, kWarps)));
+        const int from = sm.n_mid + sm.n_long < dv ? warp * each : dv;    // none left
+        for (int i = from; i < dv; i += each * kWarps) {
             const bool has = lane < each && i + lane < dv;
             acc += sub_stream(off, ind, has, has ? ind[vb + i + lane] : (IndT)0, v, dv,
-                              sm.block.key, sm.block.far, lg, false);
+                              sm.block.key, lg, false);
         }
         acc += sub_pairs(off, ind, vb, sm.block.longs, sm.n_long, (int)threadIdx.x,
                          kSubThreads);
@@ -565,8 +578,8 @@ subset_kernel(const OffT *__restrict__ off, const IndT *__restrict__ ind,
             for (int i0 = 0; i0 < dv; i0 += 32) {
                 const bool has = i0 + lane < dv;
                 int du;
-                const bool lng = has && sub_insert(off, ind[vb + i0 + lane], v, dv, ws.key,
-                                                   ws.far, lg, du);
+                const bool lng =
+                    has && sub_insert(off, ind[vb + i0 + lane], v, dv, ws.key, lg, du);
                 const unsigned int m = __ballot_sync(0xffffffffu, lng);
                 if (lng) ws.longs[n_long + __popc(m & ((1u << lane) - 1u))] =
                     (unsigned char)(i0 + lane);
@@ -578,7 +591,7 @@ subset_kernel(const OffT *__restrict__ off, const IndT *__restrict__ ind,
                 for (int i0 = 0; i0 < dv; i0 += 32) {
                     const bool has = i0 + lane < dv;
                     acc += sub_stream(off, ind, has, has ? ind[vb + i0 + lane] : (IndT)0, v, dv,
-                                      ws.key, ws.far, lg, true);
+                                      ws.key, lg, true);
                 }
                 acc += sub_pairs(off, ind, vb, ws.longs, n_long, lane, 32);
             }
@@ -824,17 +837,18 @@ gtc_status launch_subset(const OffT *off, const IndT *ind, const VtxT *vertex,
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     auto rows = subset_kernel<OffT, IndT, VtxT, OutT>;
-    const int rsmem = (int)sizeof(SubSmem<IndT>);
-    if (cudaFuncSetAttribute(rows, cudaFuncAttributeMaxDynamicSharedMemorySize, rsmem) !=
-        cudaSuccess)
-        return GTC_ERR_CUDA;
-    // few vertices: a block each, for the time is that of the longest row, and
-    // more rows shared by the whole GPU; many: a warp each for short rows
+    constexpr int rsmem = (int)sizeof(SubSmem<IndT>);
+    static_assert(rsmem <= 48 * 1024, "what a launch may have without asking");
+    // the vertices in as many shares as there are blocks at a time, or whole
+    // multiples of that, up to kSubClaim a share: 60,000 vertices of an ER 100K of
+    // mean degree 600 take 74 ms so, 98 at 32 a share and 1,184 blocks that took
+    // one share after another; rows of R-MAT 18 6.3 and 6.4 ms
     const bool few = count < kSubFew;
-    const int claim = count < kSubFew / 8 ? 1 : (few ? 8 : kSubClaim);
+    const long long fit = 4ll * sms;
+    const int claim = (int)div_up(count, fit * div_up(count, fit * kSubClaim));
     const long long hub_min = count < 2 * kSubFew ? kSubHubMin / 4 : kSubHubMin;
     const long long claims = div_up<long long>(count, claim);
-    const long long blocks = claims < (long long)sms * 8 ? claims : (long long)sms * 8;
+    const long long blocks = min(claims, (long long)INT_MAX);
     rows<<<(unsigned)blocks, kSubThreads, rsmem, stream>>>(
         off, ind, vertex, count, out, skip, claim, few ? kSubWarpRow / 2 : kSubWarpRow, (int)hub_min);
     // the hub kernel adds to what subset_kernel wrote (0 for hubs), in
