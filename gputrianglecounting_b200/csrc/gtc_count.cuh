@@ -1269,8 +1269,13 @@ __device__ __forceinline__ void table_warp_row(const Data &w, int v, const VInfo
     __syncwarp();
     tab.clear<PV>(lane, 32);
     __syncwarp();
-    for (int k = lane; k < vi.fdeg; k += 32) tab.insert(list[k]);
-    __syncwarp();
+    // all lanes make the same steps: after a loop that each leaves by itself the
+    // compiler ran all that follows for them apart where only the global count
+    // was asked for (ER 200K of mean degree 100: 2858 us, 1008 so; with counts 1097)
+    for (int k0 = 0; k0 < vi.fdeg; k0 += 32) {
+        if (k0 + lane < vi.fdeg) tab.insert(list[k0 + lane]);
+        __syncwarp();
+    }
     unsigned int mine = 0;
     for (int k = 0; k < vi.fdeg; k += 32) mine += probe_members<PV, Pos>(w, ls, list, k, vi.fdeg, tab);
     mine = warp_sum(mine);
