@@ -886,9 +886,11 @@ gtc_status launch_subset_ws(const OffT *off, const int *ind, long long n, long l
     subset_cost_kernel<OffT><<<(unsigned)(want < 1184 ? want : 1184), 256, 0, stream>>>(
         off, ind, vertex, count, kSubWhole * (unsigned long long)nnz, cost, whole);
     Data w;
+    RowConfig cfg = pick_row_config(n, nnz);
+    cfg.split = false;
     gtc_status st = run_count<OffT>(off, ind, n, nnz, true, nullptr, nullptr, nullptr, nullptr,
                                     static_cast<char *>(ws) + 256, ws_bytes - 256, stream,
-                                    RowConfig{}, nullptr, nullptr, whole, &w);
+                                    cfg, nullptr, nullptr, whole, &w);
     if (st != GTC_OK) return st;
     subset_gather_kernel<<<(unsigned)div_up<long long>(count, 256), 256, 0, stream>>>(w, vertex,
                                                                                      count, out);

@@ -12,6 +12,9 @@ struct RowConfig {
     // Heavy graphs (mean degree > 24): wide and short rows in launches of
     // their own; otherwise one launch takes both.  gtc_tuning.labels.
     bool split = false;
+    // Rows so long (mean degree >= 128, the graph not all core) that some are
+    // looked up in bitmaps, by a kernel of their own.
+    bool dense = false;
 };
 
 // Kernel launches of one run_count with this configuration (the epilogue

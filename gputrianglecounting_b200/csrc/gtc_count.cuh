@@ -175,23 +175,19 @@ struct WideClaim {
     long long item;
 };
 
-// The rows of the wide list that `want` (of the row's record): the blocks take
-// those of more than `most` members, each as a whole (by_block), then the
-// warps take the others (by_warp).  First shares are fixed, the next ones come
-// from queues.  A share's rows are spread over the list, whose neighbours tend
-// to be alike (generators give hubs the lowest ids).
-template <class Want, class ByBlock, class ByWarp>
-__device__ __forceinline__ void wide_rows(const Data &w, WideClaim &cl, long long block,
-                                          unsigned long long *long_next, unsigned long long *next, int most, const Want &want,
-                                          const ByBlock &by_block, const ByWarp &by_warp)
+// The rows of the wide list of more than `most` members that `want` (of the
+// row's record), each by a whole block (by_block).  First shares are fixed, the
+// next ones come from a queue.  A share's rows are spread over the list, whose
+// neighbours tend to be alike (generators give hubs the lowest ids).
+template <class Want, class ByBlock>
+__device__ __forceinline__ void wide_block_rows(const Data &w, WideClaim &cl, long long block,
+                                                unsigned long long *long_next, int most,
+                                                const Want &want, const ByBlock &by_block)
 {
     const long long rows = (long long)w.ctr->wide_rows;
-    const int lane = threadIdx.x & 31;
     // shares small enough that the last ones leave no long tail
-    const long long warps = (long long)gridDim.x * (kThreads / 32);
     const int per_block = (int)min((long long)kClaim, max(8ll, rows / (4ll * gridDim.x)));
-    const int per_warp = (int)min((long long)kWarpClaim, max(1ll, rows / (16 * warps)));
-    long long claims = div_up<long long>(rows, per_block);
+    const long long claims = div_up<long long>(rows, per_block);
     long long item = block;
     while (item < claims) {
         __syncthreads();
@@ -213,9 +209,23 @@ __device__ __forceinline__ void wide_rows(const Data &w, WideClaim &cl, long lon
         __syncthreads();
         item = cl.item;
     }
+}
+
+// The same, and those of at most `most` members by a warp each (by_warp).
+template <class Want, class ByBlock, class ByWarp>
+__device__ __forceinline__ void wide_rows(const Data &w, WideClaim &cl, long long block,
+                                          unsigned long long *long_next,
+                                          unsigned long long *next, int most, const Want &want,
+                                          const ByBlock &by_block, const ByWarp &by_warp)
+{
+    wide_block_rows(w, cl, block, long_next, most, want, by_block);
     __syncthreads();
-    claims = div_up<long long>(rows, per_warp);
-    item = block * (kThreads / 32) + (threadIdx.x >> 5);
+    const long long rows = (long long)w.ctr->wide_rows;
+    const int lane = threadIdx.x & 31;
+    const long long warps = (long long)gridDim.x * (kThreads / 32);
+    const int per_warp = (int)min((long long)kWarpClaim, max(1ll, rows / (16 * warps)));
+    const long long claims = div_up<long long>(rows, per_warp);
+    long long item = block * (kThreads / 32) + (threadIdx.x >> 5);
     while (item < claims) {
         const long long at = item + claims * lane;
         int v = 0;
@@ -1130,6 +1140,31 @@ struct TableBlockSmem {
     unsigned long long total;                     // a row's triangles, of all its chunks
 };
 
+// Of a row that is looked up in a bitmap: most vertices and core positions of its
+// graph, most members at a time; the longest list for which the table is taken, if
+// there are credits, in a graph of more than kBitFew vertices and in a smaller one.
+constexpr int kBitSpan = 1 << 17, kBitMembers = 4096;
+constexpr int kBitFew = 1 << 15, kBitList = 256, kBitListFew = 384;
+
+struct BitsSmem {
+    unsigned int bits[kBitSpan / 32];
+    unsigned short below[kBitSpan / 32];          // members in earlier words
+    unsigned int cnt[kBitMembers];
+    unsigned int wsum[kThreads / 32];
+    int next;
+    unsigned long long total;
+    WideClaim claim;
+};
+
+// Whether a row of a call with the bitmap kernel is that kernel's.
+template <bool PV, bool BATCH>
+__device__ __forceinline__ bool in_bitmap(const Data &w, const VInfo &vi, const GraphRec *rec)
+{
+    const long long span = (BATCH ? (long long)rec->nv : w.n) + rec->core;
+    return w.bitmaps && span <= kBitSpan &&
+           vi.fdeg > (!PV ? kWarpTable : span > kBitFew ? kBitList : kBitListFew);
+}
+
 template <typename Pos>
 struct ListSmem {
     union {
@@ -1181,15 +1216,41 @@ struct MemberTable {
     }
 };
 
+// Shared-memory bitmap of a row's members over all that its graph's lists can
+// name, vertices and core positions; a member's counter is the number of
+// members before it.  base: what a list calls the graph's first vertex.
+template <bool PV>
+struct MemberBits {
+    const unsigned int *bits;
+    const unsigned short *below;
+    unsigned int *cnt;
+    int base, nv;
+    unsigned int span;
+
+    __device__ __forceinline__ unsigned int index(int m) const
+    {
+        return m >= 0 ? (unsigned int)(m - base) : (unsigned int)nv + (unsigned int)~m;
+    }
+    __device__ __forceinline__ int find(int x) const
+    {
+        const unsigned int i = index(x), b = i & 31;
+        if (i >= span) return -1;
+        const unsigned int word = bits[i >> 5];
+        if (!((word >> b) & 1u)) return -1;
+        return PV ? below[i >> 5] + __popc(word & ((1u << b) - 1u)) : 0;
+    }
+};
+
 // The lists of the members of list[k .. k + 32) that are not core, looked up
-// by the warp: list by list, 128 elements at a time, where they are long, else
+// by the warp: list by list where they are long, 128 elements at a time, up to
+// the first above `last` (the row's highest member if lists are ascending), else
 // as one stream (finding each element's list costs as much as looking it up,
 // but short lists one by one would wait for memory one by one).  Returns this
 // lane's member's hits.
-template <bool PV, typename Pos>
+template <bool PV, typename Pos, class Table>
 __device__ __forceinline__ unsigned int probe_members(const Data &w, const Lists &ls,
-                                                      const int *list, int k, int n,
-                                                      const MemberTable &tab)
+                                                      const int *list, int k, int n, int last,
+                                                      const Table &tab)
 {
     constexpr int kPer = 4;
     const int lane = threadIdx.x & 31;
@@ -1217,6 +1278,7 @@ __device__ __forceinline__ unsigned int probe_members(const Data &w, const Lists
 #pragma unroll
                 for (int j = 0; j < kPer; ++j)
                     x[j] = j0 + 32 * j + lane < n ? ql[j0 + 32 * j + lane] : kNoProbe;
+                if (__shfl_sync(0xffffffffu, x[0], 0) > last) break;
 #pragma unroll
                 for (int j = 0; j < kPer; ++j) {
                     if (j0 + 32 * j >= n) break;
@@ -1277,7 +1339,7 @@ __device__ __forceinline__ void table_warp_row(const Data &w, int v, const VInfo
         __syncwarp();
     }
     unsigned int mine = 0;
-    for (int k = 0; k < vi.fdeg; k += 32) mine += probe_members<PV, Pos>(w, ls, list, k, vi.fdeg, tab);
+    for (int k = 0; k < vi.fdeg; k += 32) mine += probe_members<PV, Pos>(w, ls, list, k, vi.fdeg, INT32_MAX, tab);
     mine = warp_sum(mine);
     __syncwarp();
     if (mine) {
@@ -1326,12 +1388,93 @@ __device__ void table_block_row(const Data &w, int v, const VInfo &vi, const Gra
             if (lane == 0) k = atomicAdd(&sm.next, per);
             k = __shfl_sync(0xffffffffu, k, 0);
             if (k >= vi.fdeg) break;
-            mine += probe_members<PV, Pos>(w, ls, list, k, min(k + per, vi.fdeg), tab);
+            mine += probe_members<PV, Pos>(w, ls, list, k, min(k + per, vi.fdeg), INT32_MAX, tab);
         }
         __syncthreads();
         if (PV)
             for (int k = threadIdx.x; k < slots; k += kThreads)
                 if (sm.cnt[k]) credit(w, v0, ls.shift, sm.key[k], sm.cnt[k]);
+        const unsigned int ws = warp_sum(mine);
+        if (lane == 0 && ws) atomicAdd(&sm.total, (unsigned long long)ws);
+        __syncthreads();
+    }
+    if (threadIdx.x == 0 && sm.total) {
+        if (PV) atomicAdd(&w.tacc[v], sm.total);
+        tri += sm.total;
+    }
+}
+
+// A longer row of a graph of at most kBitSpan vertices and core positions, in a
+// bitmap of all of them: kBitMembers members at a time, so mostly in one pass over
+// the lists where the table makes one per kMemberChunk, and a hit needs no key.
+// Sums as in table_block_row.  ER 40K of mean degree 2,000 42 ms (table 91; binary
+// search of degree-sorted lists, which the tables replaced, 39), ring of 40K with
+// 1,000 neighbours each, in no order of ids, 11.5 (16.9; 11.3).  Where the lines
+// are, with credits: from 257 members on ER 40K of 500 takes 3.14 ms, RGG 100K of
+// 500 10.3, from 385 on 3.27 and 11.1; but 200 graphs ER 5K of 300 40.7 and 37.5,
+// R-MAT 14 of 256 0.285 from 129 on and 0.255.  Without credits from the first row
+// on that a block takes: ER 40K of 500 2.63 (table 3.11), RGG 100K 7.5 (10.1).
+template <bool PV, bool BATCH, typename Pos>
+__device__ void bits_block_row(const Data &w, int v, const VInfo &vi, const GraphRec *rec,
+                               BitsSmem &sm, unsigned long long &tri)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const Lists ls = lists_of<BATCH>(w, rec);
+    const long long v0 = BATCH ? rec->v0 : 0;
+    const int *list = ls.base + vi.fbeg;
+    const int last = rec->uniform ? list[vi.fdeg - 1] : INT32_MAX;
+    const int nv = BATCH ? rec->nv : (int)w.n, span = nv + rec->core;
+    const MemberBits<PV> tab{sm.bits, sm.below, sm.cnt, BATCH ? (int)v0 - ls.shift : 0, nv,
+                             (unsigned int)span};
+    const int words = (span + 31) >> 5, each = div_up(words, kThreads);
+    const int per = max(4, min(32, vi.fdeg / (4 * kThreads / 32)));
+    __syncthreads();
+    if (threadIdx.x == 0) sm.total = 0;
+    for (int c0 = 0; c0 < vi.fdeg; c0 += kBitMembers) {
+        const int nm = min(vi.fdeg - c0, kBitMembers);
+        for (int k = threadIdx.x; k < words; k += kThreads) sm.bits[k] = 0;
+        if (PV)
+            for (int k = threadIdx.x; k < nm; k += kThreads) sm.cnt[k] = 0;
+        if (threadIdx.x == 0) sm.next = 0;
+        __syncthreads();
+        for (int k = threadIdx.x; k < nm; k += kThreads) {
+            const unsigned int i = tab.index(list[c0 + k]);
+            if (i < tab.span) atomicOr(&sm.bits[i >> 5], 1u << (i & 31));
+        }
+        __syncthreads();
+        if (PV) {
+            const int w0 = (int)threadIdx.x * each;
+            int sum = 0;
+            for (int j = 0; j < each; ++j)
+                if (w0 + j < words) sum += __popc(sm.bits[w0 + j]);
+            const int incl = warp_incl_scan(sum);
+            if (lane == 31) sm.wsum[warp] = (unsigned int)incl;
+            __syncthreads();
+            int first = incl - sum;
+            for (int i = 0; i < warp; ++i) first += (int)sm.wsum[i];
+            for (int j = 0; j < each; ++j)
+                if (w0 + j < words) {
+                    sm.below[w0 + j] = (unsigned short)first;
+                    first += __popc(sm.bits[w0 + j]);
+                }
+            __syncthreads();
+        }
+        unsigned int mine = 0;
+        while (true) {
+            int k = 0;
+            if (lane == 0) k = atomicAdd(&sm.next, per);
+            k = __shfl_sync(0xffffffffu, k, 0);
+            if (k >= vi.fdeg) break;
+            mine += probe_members<PV, Pos>(w, ls, list, k, min(k + per, vi.fdeg), last, tab);
+        }
+        __syncthreads();
+        if (PV)
+            for (int k = threadIdx.x; k < nm; k += kThreads) {
+                const int m = list[c0 + k];
+                const int s = tab.find(m);
+                const unsigned int c = s >= 0 ? sm.cnt[s] : 0u;
+                if (c) credit(w, v0, ls.shift, m, c);
+            }
         const unsigned int ws = warp_sum(mine);
         if (lane == 0 && ws) atomicAdd(&sm.total, (unsigned long long)ws);
         __syncthreads();
@@ -1351,7 +1494,9 @@ __device__ __forceinline__ void table_wide_rows(const Data &w, ListSmem<Pos> &sm
         w, sm.claim, first_block(w.n, gridDim.x / 4), &w.ctr->table_long_next, &w.ctr->table_wide_next, kWarpTable,
         [](const VInfo &vi) { return vi.fdeg >= 2 && vi.fdeg > (vi.dk & INT32_MAX); },
         [&](int v, const VInfo &vi) {
-            table_block_row<PV, BATCH, Pos>(w, v, vi, &w.recs[BATCH ? w.gid[v] : 0], sm.block, tri);
+            const GraphRec *rec = &w.recs[BATCH ? w.gid[v] : 0];
+            if (!in_bitmap<PV, BATCH>(w, vi, rec))
+                table_block_row<PV, BATCH, Pos>(w, v, vi, rec, sm.block, tri);
         },
         [&](int v, const VInfo &vi) {
             table_warp_row<PV, BATCH, Pos>(w, v, vi, &w.recs[BATCH ? w.gid[v] : 0],
@@ -1466,6 +1611,27 @@ list_kernel(const Data w, bool do_wide, bool do_short, int batch)
     if (do_short)
         list_short_rows<PV, BATCH, Pos>(w, batch, sm.tile[threadIdx.x >> 5], tri,
                                         [](long long) {});
+    add_triangles(w.ctr, tri);
+}
+
+// Wide rows that a bitmap holds.  A kernel of its own, launched where rows are
+// long (RowConfig::dense): as a part of list_kernel it cost R-MAT 22 0.8% and a
+// ring of 400K with 100 neighbours each 3%, in registers.
+template <bool PV, bool BATCH, typename Pos>
+__global__ void __launch_bounds__(kThreads, 5)
+bitmap_kernel(const Data w)
+{
+    __shared__ BitsSmem sm;
+    if (gated(w)) return;
+    unsigned long long tri = 0;
+    wide_block_rows(
+        w, sm.claim, blockIdx.x, &w.ctr->bitmap_next, PV ? kBitList : kWarpTable,
+        [](const VInfo &vi) { return vi.fdeg > (vi.dk & INT32_MAX); },
+        [&](int v, const VInfo &vi) {
+            const GraphRec *rec = &w.recs[BATCH ? w.gid[v] : 0];
+            if (in_bitmap<PV, BATCH>(w, vi, rec))
+                bits_block_row<PV, BATCH, Pos>(w, v, vi, rec, sm, tri);
+        });
     add_triangles(w.ctr, tri);
 }
 

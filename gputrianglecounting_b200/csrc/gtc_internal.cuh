@@ -91,6 +91,7 @@ struct Counters {
     unsigned long long place_next;    // dynamic queues:
     unsigned long long core_long_next, core_wide_next, core_short_next;
     unsigned long long table_long_next, table_wide_next, list_short_next;
+    unsigned long long bitmap_next;
     unsigned long long u_words;       // bit-matrix words handed out (batch)
     unsigned int blocks_done;         // degree pass: blocks finished
 };
