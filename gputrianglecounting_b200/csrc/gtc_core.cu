@@ -232,9 +232,12 @@ gtc_status launch(const View<OffT> &w, GraphRec lim, long long *r, long long *t,
         }
         degree_kernel<OffT, BATCH><<<vb < sms * 8 ? vb : sms * 8, kThreads, 0, s>>>(
             w, lim, !cfg.split, !BATCH && !cfg.split);
-        if (BATCH || cfg.split)
-            choose_core_kernel<OffT, BATCH><<<BATCH ? (unsigned)w.graphs : 1u, kThreads, 0, s>>>(
-                w, lim, !cfg.split);
+        if (BATCH || cfg.split) {
+            // one graph per block up to four rounds of blocks
+            const long long per = min((long long)kThreads, max(1ll, w.graphs / (sms * 32)));
+            const unsigned cb = BATCH ? (unsigned)div_up(w.graphs, per) : 1u;
+            choose_core_kernel<OffT, BATCH><<<cb, kThreads, 0, s>>>(w, lim, !cfg.split, (int)per);
+        }
         key_rows_kernel<<<n < sms * 4 * kThreads ? vb : sms * 4, kThreads, 0, s>>>(
             w, !(BATCH && cfg.split));
         if (BATCH && cfg.split) zero_bits_kernel<<<sms * 4, kThreads, 0, s>>>(w);
