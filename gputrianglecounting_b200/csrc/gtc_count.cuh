@@ -1278,7 +1278,7 @@ __device__ __forceinline__ unsigned int probe_members(const Data &w, const Lists
 #pragma unroll
                 for (int j = 0; j < kPer; ++j)
                     x[j] = j0 + 32 * j + lane < n ? ql[j0 + 32 * j + lane] : kNoProbe;
-                if (__shfl_sync(0xffffffffu, x[0], 0) > last) break;
+                if (last != INT32_MAX && __shfl_sync(0xffffffffu, x[0], 0) > last) break;
 #pragma unroll
                 for (int j = 0; j < kPer; ++j) {
                     if (j0 + 32 * j >= n) break;
