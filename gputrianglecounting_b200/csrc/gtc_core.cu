@@ -138,6 +138,7 @@ RowConfig pick_row_config(long long n, long long nnz)
     // so R-MAT 20 takes 1547 us split and 1518 joint.  Smaller ones do not:
     // R-MAT 17 223 us split, 174 joint
     c.split = n >= kSmallGraph && (double)nnz / (double)n > 24.0;
+    c.sparse = n >= kSmallGraph && nnz <= 4 * n;
     c.dense = nnz >= 128 * n && !(n <= kCoreMax && n * n <= 32 * nnz);
     return c;
 }
@@ -169,10 +170,10 @@ int launches_per_count(const RowConfig &cfg, bool per_vertex, long long n)
     // rows, lists and bit matrix for each, per-vertex outputs, global counts;
     // otherwise degrees with the core choice, core keys, placement, lists and
     // bit matrix (one launch below kSmallGraph vertices), outputs; either way
-    // bitmaps for a graph of long rows that they hold
-    const int bitmaps = cfg.dense && n <= kBitSpan ? 1 : 0;
-    if (cfg.split) return (per_vertex ? 11 : 10) + bitmaps;
-    return (n >= kSmallGraph ? 6 : 5) + bitmaps;
+    // bitmaps for a graph of long rows that they hold, pairs for a sparse one
+    const int more = ((cfg.dense && n <= kBitSpan) || cfg.sparse) ? 1 : 0;
+    if (cfg.split) return (per_vertex ? 11 : 10) + more;
+    return (n >= kSmallGraph ? 6 : 5) + more;
 }
 
 namespace {
@@ -259,6 +260,10 @@ gtc_status launch(const View<OffT> &w, GraphRec lim, long long *r, long long *t,
         constexpr auto k = bitmap_kernel<PV, BATCH, Pos>;
         k<<<grid_for<k>(0, dev, n), kThreads, 0, s>>>(w);
     }
+    if (!BATCH && w.pairs) {
+        constexpr auto k = pairs_kernel<PV>;
+        k<<<grid_for<k>(0, dev, vb), kThreads, 0, s>>>(w);
+    }
     if (cfg.split) {
         NvtxRange range("gtc: split count");
         launch_lists<PV, BATCH, Pos>(w, dev, s, true, false);
@@ -314,6 +319,7 @@ gtc_status run_count(const OffT *off, const int *ind, long long n, long long nnz
     w.word = (int)sizeof(unsigned int);
     w.gate = gate;
     w.bitmaps = cfg.dense && (batch || n <= kBitSpan);
+    w.pairs = cfg.sparse && !batch;
     w.status = reinterpret_cast<unsigned int *>(base + p.o_status);
     w.ctr = reinterpret_cast<Counters *>(base + p.o_counters);
     w.recs = reinterpret_cast<GraphRec *>(base + p.o_recs);

@@ -15,6 +15,9 @@ struct RowConfig {
     // Rows so long (mean degree >= 128, the graph not all core) that some are
     // looked up in bitmaps, by a kernel of their own.
     bool dense = false;
+    // Mean degree of at most 4, a large graph: if it is uniform, its short rows'
+    // pairs are looked up one by one, by a kernel of their own.
+    bool sparse = false;
 };
 
 // Kernel launches of one run_count with this configuration (the epilogue
