@@ -83,17 +83,18 @@ class _Workspace:
 
     def get(self, nbytes: int, stream, handle: int | None) -> torch.Tensor:
         """At least nbytes for a call on `stream`, whose handle is given."""
-        if self.buffer is None or self.buffer.numel() < nbytes:
-            self.buffer = None
+        buffer = self.buffer
+        if buffer is None or buffer.numel() < nbytes:
+            self.buffer = buffer = None
             with _allocating_on(stream, self.device):
-                self.buffer = _alloc_workspace(nbytes, self.device)
+                self.buffer = buffer = _alloc_workspace(nbytes, self.device)
             self._owner = handle
         elif handle != self._owner:
             # the block, once dropped, stays taken until this stream is done with it too
             if stream is None:
                 stream = torch.cuda.current_stream()
-            self.buffer.record_stream(_torch_stream(stream, self.device))
-        return self.buffer
+            buffer.record_stream(_torch_stream(stream, self.device))
+        return buffer
 
 
 def _check_csr_tensors(off: torch.Tensor, ind: torch.Tensor) -> int:
@@ -443,7 +444,9 @@ class BatchCounter:
         G, n, nnz = batch.num_graphs, batch.total_n, batch.total_nnz
         handle = _stream_handle(stream)
         ws = self._work.get(self.workspace_bytes(G, n, nnz), stream, handle)
-        if out is None:
+        if out is None and stream is None:
+            out = self.alloc_outputs(batch, outputs)
+        elif out is None:
             with _allocating_on(stream, self.device):
                 out = self.alloc_outputs(batch, outputs)
             _hand_out(stream, out.r, out.t, out.lcc, out.graph_T)

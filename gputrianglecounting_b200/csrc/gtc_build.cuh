@@ -334,8 +334,9 @@ template <typename OffT, bool BATCH>
 __global__ void __launch_bounds__(kThreads)
 choose_core_kernel(const View<OffT> w, GraphRec lim, bool limits, int per)
 {
-    if (!BATCH) {
-        choose_graph_core<OffT, BATCH>(w, 0, lim);
+    auto limits_of = [&](long long g) { return limits ? batch_limits(w, g) : w.recs[g]; };
+    if (!BATCH || per == 1) {
+        choose_graph_core<OffT, BATCH>(w, blockIdx.x, BATCH ? limits_of(blockIdx.x) : lim);
         return;
     }
     __shared__ int s_todo[kThreads], s_n;
@@ -343,11 +344,10 @@ choose_core_kernel(const View<OffT> w, GraphRec lim, bool limits, int per)
     if (threadIdx.x == 0) s_n = 0;
     __syncthreads();
     if (threadIdx.x < per && g0 + threadIdx.x < w.graphs) {
-        const long long g = g0 + threadIdx.x;
-        lim = limits ? batch_limits(w, g) : w.recs[g];
+        lim = limits_of(g0 + threadIdx.x);
         if (lim.nv <= lim.long_min) {
             lim.uniform = 1;
-            w.recs[g] = lim;
+            w.recs[g0 + threadIdx.x] = lim;
         } else {
             s_todo[atomicAdd(&s_n, 1)] = (int)threadIdx.x;
         }
@@ -355,7 +355,7 @@ choose_core_kernel(const View<OffT> w, GraphRec lim, bool limits, int per)
     __syncthreads();
     for (int k = 0; k < s_n; ++k) {
         const long long g = g0 + s_todo[k];
-        choose_graph_core<OffT, BATCH>(w, g, limits ? batch_limits(w, g) : w.recs[g]);
+        choose_graph_core<OffT, BATCH>(w, g, limits_of(g));
         __syncthreads();                          // its shared words are used again
     }
 }
