@@ -169,6 +169,19 @@ class TriangleCounter:
               "gtc_workspace_size")
         return int(out.value)
 
+    def _alloc_outputs(self, dev, n: int, want, stream) -> TriangleCounts:
+        if stream is not None:
+            with _allocating_on(stream, dev):
+                out = self._alloc_outputs(dev, n, want, None)
+            _hand_out(stream, out.r, out.t, out.lcc, out.global_counts)
+            return out
+        return TriangleCounts(
+            r=torch.empty(n, dtype=torch.int64, device=dev) if "r" in want else None,
+            t=torch.empty(n, dtype=torch.int64, device=dev) if "t" in want else None,
+            lcc=torch.empty(n, dtype=torch.float64, device=dev) if "lcc" in want else None,
+            global_counts=torch.empty(3, dtype=torch.int64, device=dev),
+        )
+
     def _workspace(self, nbytes: int, stream=None) -> torch.Tensor:
         return self._work.get(nbytes, stream, _stream_handle(stream))
 
@@ -200,16 +213,7 @@ class TriangleCounter:
             raise ValueError(f"mode must be one of {list(_MODES)}")
         n, nnz = off.numel() - 1, ind.numel()
         if out is None:
-            dev = off.device
-            want = set(outputs) if mode == "plain" else set()
-            with _allocating_on(stream, dev):
-                out = TriangleCounts(
-                    r=torch.empty(n, dtype=torch.int64, device=dev) if "r" in want else None,
-                    t=torch.empty(n, dtype=torch.int64, device=dev) if "t" in want else None,
-                    lcc=torch.empty(n, dtype=torch.float64, device=dev) if "lcc" in want else None,
-                    global_counts=torch.empty(3, dtype=torch.int64, device=dev),
-                )
-            _hand_out(stream, out.r, out.t, out.lcc, out.global_counts)
+            out = self._alloc_outputs(off.device, n, set(outputs) if mode == "plain" else (), stream)
         ws_bytes = self.workspace_bytes(n, nnz, off_bits, mode)
         handle = _stream_handle(stream)
         ws = self._work.get(ws_bytes, stream, handle)

@@ -14,7 +14,7 @@ from oracle import oracle
 
 pytestmark = pytest.mark.gpu
 
-HOLD = 100_000_000                      # clock cycles a stream is held back, some 50 ms
+HOLD = 1_000_000_000                    # clock cycles a stream is held back, half a second
 
 
 class Noting:
