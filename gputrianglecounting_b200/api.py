@@ -52,13 +52,18 @@ def _torch_stream(stream, device) -> torch.cuda.Stream:
             else torch.cuda.default_stream(device))
 
 
+def _is_current(stream, device) -> bool:
+    return (stream is None
+            or stream.cuda_stream == torch.cuda.current_stream(device).cuda_stream)
+
+
 def _allocating_on(stream, device):
     """Context in which torch allocates on the stream that a call launches on.
     The caching allocator hands a block out again in the order of the stream it
     was allocated on: with any other one, memory freed at the call's return
     would be somebody else's while the kernels still use it, and a block could
     be handed to them while earlier work of its own stream is still to come."""
-    if stream is None:
+    if _is_current(stream, device):
         return _AS_IS
     return torch.cuda.stream(_torch_stream(stream, device))
 
@@ -67,10 +72,9 @@ def _hand_out(stream, *tensors) -> None:
     """The tensors, allocated on the launch stream, go to a caller who reads them
     (having waited) on the current one: their blocks stay taken until that is
     done with them too."""
-    if stream is not None:
-        for t in tensors:
-            if t is not None:
-                t.record_stream(torch.cuda.current_stream(t.device))
+    for t in tensors:
+        if t is not None and not _is_current(stream, t.device):
+            t.record_stream(torch.cuda.current_stream(t.device))
 
 
 class _Workspace:
