@@ -76,9 +76,8 @@ def save_cache(path: str | None, cache: dict) -> None:
 
 
 def valid(tuning: dict) -> bool:
-    """Per-row merges need vertex-id labels and use no hash regions, so
-    (rows 2, labels 2) is rejected by the library and (rows 2, region 4)
-    would time (rows 2, region 2) again."""
+    """rows 2 asks for joint launches, so the library rejects (rows 2, labels 2);
+    with region 4 it would be (rows 2, region 2) again."""
     if tuning.get("rows") == 2:
         return tuning.get("labels") != 2 and tuning.get("region", 2) == 2
     return True

@@ -35,9 +35,9 @@ __device__ __forceinline__ int graph_of(const long long *__restrict__ vstart, lo
 // degree and 16 more, which random graphs of equal expected degrees do not have
 // (eight standard deviations at mean 32), so those stay uniform and pay nothing
 // but the empty launches.  At 4 and 8 times the mean the 512-graph batch took
-// 10.64 and 12.31 ms instead of 10.37, R-MAT 17 181 and 200 us instead of 170.  A small graph of mean degree 64 or more, so dense that
-// its whole bit matrix is no larger than its adjacency lists (mean degree >=
-// n / 32), is all core.
+// 10.64 and 12.31 ms instead of 10.37, R-MAT 17 181 and 200 us instead of 170.
+// A small graph of mean degree 64 or more, so dense that its whole bit matrix is
+// no larger than its adjacency lists (mean degree >= n / 32), is all core.
 __host__ __device__ __forceinline__ void core_limits(long long n, long long nnz, long long room,
                                                      int &dmin, int &long_min, int &kcap)
 {

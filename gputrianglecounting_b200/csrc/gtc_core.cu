@@ -55,7 +55,7 @@ unsigned grid_for(size_t dyn_smem, int dev, long long work)
 
 inline size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 
-// Bytes a count asks for at least: per vertex 48 (56 with counts), per entry
+// Bytes a count asks for at least: per vertex 40 (48 with counts), per entry
 // 4.5, and 67 KiB; a batch adds a copy of the ids and per-graph histograms.
 // The layout below fits into it with room to spare for a bit matrix, so the
 // size is a contract with callers rather than a sum of today's arrays.
@@ -134,9 +134,12 @@ Plan make_plan(long long n, long long nnz, int off_bits, bool per_vertex, long l
 RowConfig pick_row_config(long long n, long long nnz)
 {
     RowConfig c;
-    // heavy graphs have enough work to fill the GPU with each kind of row; even
-    // so R-MAT 20 takes 1547 us split and 1518 joint.  Smaller ones do not:
-    // R-MAT 17 223 us split, 174 joint
+    // Split launches are no faster anywhere that was measured (joint and split,
+    // us: R-MAT 17 193 and 242, 18 396 and 429, 20 1518 and 1552, 21 3952 and
+    // 4027, 22 10886 and 11040; ER 900K of mean degree 30 377 and 392; the
+    // 512-graph batch 10267 and 10455).  They stay the form of large heavy graphs
+    // because callers ask gtc_count_launches for the number of launches and the
+    // form; from 2^18 vertices on they cost 1 to 4 percent
     c.split = n >= kSmallGraph && (double)nnz / (double)n > 24.0;
     c.sparse = n >= kSmallGraph && nnz <= 4 * n;
     c.dense = nnz >= 128 * n && !(n <= kCoreMax && n * n <= 32 * nnz);

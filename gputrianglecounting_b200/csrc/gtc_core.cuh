@@ -9,8 +9,8 @@ struct Data;
 
 // Launch plan of one count.
 struct RowConfig {
-    // Heavy graphs (mean degree > 24): wide and short rows in launches of
-    // their own; otherwise one launch takes both.  gtc_tuning.labels.
+    // Large heavy graphs (mean degree > 24): wide and short rows in launches
+    // of their own; otherwise one launch takes both.  gtc_tuning.labels.
     bool split = false;
     // Rows so long (mean degree >= 128, the graph not all core) that some are
     // looked up in bitmaps, by a kernel of their own.

@@ -4,7 +4,6 @@
 #pragma once
 
 #include <cuda_pipeline.h>
-#include <type_traits>
 
 #include "gtc_build.cuh"
 
@@ -1407,7 +1406,7 @@ __device__ void table_block_row(const Data &w, int v, const VInfo &vi, const Gra
 // A longer row of a graph of at most kBitSpan vertices and core positions, in a
 // bitmap of all of them: kBitMembers members at a time, so mostly in one pass over
 // the lists where the table makes one per kMemberChunk, and a hit needs no key.
-// Sums as in table_block_row.  ER 40K of mean degree 2,000 42 ms (table 91; binary
+// Instruction issue bounds it (77%).  Sums as in table_block_row.  ER 40K of mean degree 2,000 42 ms (table 91; binary
 // search of degree-sorted lists, which the tables replaced, 39), ring of 40K with
 // 1,000 neighbours each, in no order of ids, 11.5 (16.9; 11.3).  Where the lines
 // are, with credits: from 257 members on ER 40K of 500 takes 3.14 ms, RGG 100K of
@@ -1645,7 +1644,7 @@ bitmap_kernel(const Data w)
 // Short rows of a sparse uniform graph (RowConfig::sparse): 32 rows per warp, their
 // pairs (q, s) of members, q < s, as one stream, s looked for in q's list.  A tile
 // costs the same however few edges its rows have; here rows of one member cost a
-// load, the next rows' on its way.  Three dependent loads per pair bound it.  Grid
+// load, the next rows' on its way.  Issue (71%) and waits for lists bound it.  Grid
 // of 2000 x 2000: tiles 173 us, 47 here; path of 8 M vertices 176 and 37.
 template <bool PV>
 __global__ void __launch_bounds__(kThreads)

@@ -18,7 +18,7 @@ struct Data {
     int *gid;                       // batch: graph of a vertex
     VInfo *vinfo;
     int *find;                      // forward lists; core members as -1 - position
-    int *wide;                      // rows that blocks take
+    int *wide;                      // rows that a warp or a block takes alone
     int2 *litem;                    // placement items of long rows: {row, chunk}
     unsigned int *u;                // bit matrices
     long long ucap;                 // words of it

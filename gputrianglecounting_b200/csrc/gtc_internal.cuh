@@ -30,7 +30,8 @@ namespace gtc {
 // ------------------------------------------------------------------ tuning
 constexpr int kThreads = 256;               // every pipeline kernel
 // Vertices from which lists and core pairs get a kernel each: R-MAT 17 takes
-// 181 us in one kernel and 201 in two, R-MAT 20 of mean degree 16 697 and 661.
+// 193 us in one kernel and 211 in two, R-MAT 20 of mean degree 16 (global count)
+// 656 and 618; R-MAT 18 and 19 of 16, in between, 228 and 253, 396 and 407.
 constexpr long long kSmallGraph = 1ll << 18;
 constexpr int kShortRow = 64;               // longest row placed with its neighbours
 // Longest forward list of a short row; of a uniform graph.  16 instead of 32:
@@ -55,9 +56,9 @@ enum : unsigned int {
 };
 
 // Per-vertex record: forward-list start, forward degree and the number of
-// core members, in one 16-byte load.  kWideRow in dk marks rows that a block
-// takes (core rows, rows longer than kShortRow, forward lists longer than
-// kShortList); those are the wide list.
+// core members, in one 16-byte load.  kWideRow in dk marks rows that a warp or a
+// block takes alone (core rows, rows longer than kShortRow, forward lists longer
+// than kShortList); those are the wide list.
 constexpr int kWideRow = INT32_MIN;
 struct __align__(16) VInfo {
     long long fbeg;

@@ -10,11 +10,12 @@
 // queues, accumulators) lives in one fixed array compiled into this library.
 //
 // Limits and rules:
-//   * the array holds kStaticScratchBytes (32 MiB); a graph whose workspace
-//     (gtc_workspace_size) is larger is rejected with GTC_ERR_CAPACITY before
-//     any device work -- about 48 bytes per vertex plus 4.5 bytes per
-//     adjacency entry plus 67 KiB, e.g. 100,000 vertices with 4 million
-//     entries fit;
+//   * the array holds kStaticScratchBytes (32 MiB); a graph that a count needs
+//     more for is rejected with GTC_ERR_CAPACITY before any device work: 48
+//     bytes per vertex (40 for the global count alone) plus 4.5 bytes per
+//     adjacency entry plus 67 KiB, e.g. 100,000 vertices with 4 million entries
+//     fit.  gtc_workspace_size may say more: it adds the core's bit matrix at
+//     its full size, which is smaller here;
 //   * every device that loads the library holds the array until the process
 //     exits;
 //   * the array is shared by all calls on a device and keeps the last call's

@@ -118,7 +118,10 @@ gtc_status gtc_count_status(const void *d_workspace, size_t ws_bytes,
  * src/param.cu:2-6).  None of them changes the result.
  *   labels       1 = joint launches: long and short rows in one kernel each
  *                (5 kernels per count, 6 from 2^18 vertices on); 2 = split
- *                launches: a kernel for long and one for short rows (11).
+ *                launches: a kernel for long and one for short rows (11); either
+ *                way one more for dense graphs of up to 2^17 vertices (mean
+ *                degree 128 or more, unless all core) and for sparse ones of 2^18
+ *                or more (mean degree of at most 4).
  *                The library splits above mean degree 24 from 2^18 vertices on
  *   rows         2 asks for joint launches too (rejected with labels = 2);
  *                1 leaves the choice to labels
@@ -180,8 +183,9 @@ gtc_status gtc_count_phase_times(const void *d_off, int off_bits,
  * a plug-in whose host framework owns the device memory, or a caller that must
  * avoid the synchronisation cudaMalloc/cudaFree can cause).  This entry point
  * has no counterpart in the reference.  The pipeline's scratch lives in a
- * fixed 32 MiB array inside the library: graphs whose gtc_workspace_size
- * exceeds it are rejected with GTC_ERR_CAPACITY.  Every device that loads the
+ * fixed 32 MiB array inside the library: graphs that need more (48 bytes per
+ * vertex, 40 in oriented mode, 4.5 per entry and 67 KiB; gtc_workspace_size may
+ * say more than that) are rejected with GTC_ERR_CAPACITY.  Every device that loads the
  * library holds the array until exit.  All calls on a device share it, so
  * calls that overlap on the GPU race and must be serialised.  The first call
  * on each device looks up the array's address; make it before any stream
