@@ -173,8 +173,8 @@ int launches_per_count(const RowConfig &cfg, bool per_vertex, long long n)
     // rows, lists and bit matrix for each, per-vertex outputs, global counts;
     // otherwise degrees with the core choice, core keys, placement, lists and
     // bit matrix (one launch below kSmallGraph vertices), outputs; either way
-    // bitmaps for a graph of long rows that they hold, pairs for a sparse one
-    const int more = ((cfg.dense && n <= kBitSpan) || cfg.sparse) ? 1 : 0;
+    // bitmaps for a graph of long rows that they hold
+    const int more = cfg.dense && n <= kBitSpan ? 1 : 0;
     if (cfg.split) return (per_vertex ? 11 : 10) + more;
     return (n >= kSmallGraph ? 6 : 5) + more;
 }
@@ -193,6 +193,12 @@ int rows_per_batch(unsigned blocks, long long n)
 template <bool PV, bool BATCH>
 void launch_core(const Data &w, int dev, cudaStream_t s, bool wide, bool shrt)
 {
+    if (!BATCH && w.sparse) {
+        constexpr auto k = sparse_core_kernel<PV>;
+        const unsigned blocks = grid_for<k>(0, dev, w.n);
+        k<<<blocks, kThreads, 0, s>>>(w, wide, shrt, rows_per_batch(blocks, w.n));
+        return;
+    }
     constexpr auto k = core_kernel<PV, BATCH>;
     const unsigned blocks = grid_for<k>(0, dev, w.n);
     k<<<blocks, kThreads, 0, s>>>(w, wide, shrt, rows_per_batch(blocks, w.n));
@@ -263,10 +269,6 @@ gtc_status launch(const View<OffT> &w, GraphRec lim, long long *r, long long *t,
         constexpr auto k = bitmap_kernel<PV, BATCH, Pos>;
         k<<<grid_for<k>(0, dev, n), kThreads, 0, s>>>(w);
     }
-    if (!BATCH && w.pairs) {
-        constexpr auto k = pairs_kernel<PV>;
-        k<<<grid_for<k>(0, dev, vb), kThreads, 0, s>>>(w);
-    }
     if (cfg.split) {
         NvtxRange range("gtc: split count");
         launch_lists<PV, BATCH, Pos>(w, dev, s, true, false);
@@ -322,7 +324,7 @@ gtc_status run_count(const OffT *off, const int *ind, long long n, long long nnz
     w.word = (int)sizeof(unsigned int);
     w.gate = gate;
     w.bitmaps = cfg.dense && (batch || n <= kBitSpan);
-    w.pairs = cfg.sparse && !batch;
+    w.sparse = cfg.sparse && !batch;
     w.status = reinterpret_cast<unsigned int *>(base + p.o_status);
     w.ctr = reinterpret_cast<Counters *>(base + p.o_counters);
     w.recs = reinterpret_cast<GraphRec *>(base + p.o_recs);

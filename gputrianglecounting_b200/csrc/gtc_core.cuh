@@ -16,7 +16,7 @@ struct RowConfig {
     // looked up in bitmaps, by a kernel of their own.
     bool dense = false;
     // Mean degree of at most 4, a large graph: if it is uniform, its short rows'
-    // pairs are looked up one by one, by a kernel of their own.
+    // pairs are looked up one by one, by a core kernel of its own.
     bool sparse = false;
 };
 

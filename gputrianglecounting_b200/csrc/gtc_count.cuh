@@ -1554,10 +1554,10 @@ __device__ __forceinline__ void add_triangles(Counters *ctr, unsigned long long 
     if ((threadIdx.x & 31) == 0 && tri) atomicAdd(&ctr->tri_total, tri);
 }
 
-// Whether pairs_kernel takes the short rows.
+// Whether sparse_core_kernel takes the short rows.
 __device__ __forceinline__ bool by_pairs(const Data &w)
 {
-    return w.pairs && w.recs[0].uniform == 1;
+    return w.sparse && w.recs[0].uniform == 1;
 }
 
 // All short rows: rows(u0, ..) of list_rows, then also(u0).  A single graph is
@@ -1602,55 +1602,15 @@ core_kernel(const Data w, bool do_wide, bool do_short, int batch)
     add_triangles(w.ctr, tri);
 }
 
-template <bool PV, bool BATCH, typename Pos>
-__global__ void __launch_bounds__(kThreads, 5)
-list_kernel(const Data w, bool do_wide, bool do_short, int batch)
-{
-    extern __shared__ __align__(16) unsigned char smem[];
-    if (gated(w)) return;
-    ListSmem<Pos> &sm = *reinterpret_cast<ListSmem<Pos> *>(smem);
-    unsigned long long tri = 0;
-    if (do_wide && w.ctr->wide_rows > 0) {
-        table_wide_rows<PV, BATCH, Pos>(w, sm, tri);
-        __syncthreads();
-    }
-    if (do_short)
-        list_short_rows<PV, BATCH, Pos>(w, batch, sm.tile[threadIdx.x >> 5], tri,
-                                        [](long long) {});
-    add_triangles(w.ctr, tri);
-}
-
-// Wide rows that a bitmap holds.  A kernel of its own, launched where rows are
-// long (RowConfig::dense): as a part of list_kernel it cost R-MAT 22 0.8% and a
-// ring of 400K with 100 neighbours each 3%, in registers.
-template <bool PV, bool BATCH, typename Pos>
-__global__ void __launch_bounds__(kThreads, 5)
-bitmap_kernel(const Data w)
-{
-    __shared__ BitsSmem sm;
-    if (gated(w)) return;
-    unsigned long long tri = 0;
-    wide_block_rows(
-        w, sm.claim, blockIdx.x, &w.ctr->bitmap_next, PV ? kBitList : kWarpTable,
-        [](const VInfo &vi) { return vi.fdeg > (vi.dk & INT32_MAX); },
-        [&](int v, const VInfo &vi) {
-            const GraphRec *rec = &w.recs[BATCH ? w.gid[v] : 0];
-            if (in_bitmap<PV, BATCH>(w, vi, rec))
-                bits_block_row<PV, BATCH, Pos>(w, v, vi, rec, sm, tri);
-        });
-    add_triangles(w.ctr, tri);
-}
-
 // Short rows of a sparse uniform graph (RowConfig::sparse): 32 rows per warp, their
 // pairs (q, s) of members, q < s, as one stream, s looked for in q's list.  A tile
 // costs the same however few edges its rows have; here rows of one member cost a
-// load, the next rows' on its way.  Issue (71%) and waits for lists bound it.  Grid
-// of 2000 x 2000: tiles 173 us, 47 here; path of 8 M vertices 176 and 37.
+// load, the next rows' on its way.  Waits for lists bound it, then issue (54%) at 32
+// warps per SM.  Grid of 2000 x 2000: tiles 173 us, 61 here; path of 8 M vertices
+// 176 and 47.
 template <bool PV>
-__global__ void __launch_bounds__(kThreads)
-pairs_kernel(const Data w)
+__device__ __forceinline__ void pair_rows(const Data &w, unsigned long long &tri)
 {
-    if (gated(w) || !by_pairs(w)) return;
     constexpr int kPer = 2;                       // pairs in flight per lane
     const int lane = threadIdx.x & 31;
     const long long step = (long long)gridDim.x * kThreads;
@@ -1658,7 +1618,6 @@ pairs_kernel(const Data w)
     auto row = [&](long long u) {
         return u + lane < w.n ? w.vinfo[u + lane] : VInfo{0, 0, 0};
     };
-    unsigned long long tri = 0;
     for (VInfo vi = row(u0); u0 < w.n; u0 += step) {
         const VInfo next = row(u0 + step);
         const int n = vi.dk >= 0 ? vi.fdeg * (vi.fdeg - 1) / 2 : 0;     // wide rows: none
@@ -1711,6 +1670,66 @@ pairs_kernel(const Data w)
         }
         vi = next;
     }
+}
+
+// core_kernel of a sparse graph: pairs of short rows if the graph is uniform, core
+// pairs if not.  Pairs in a kernel of their own took 47 and 37 us, but a launch more
+// than gtc_count_launches has always said for such a graph.
+template <bool PV>
+__global__ void __launch_bounds__(kThreads, 4)
+sparse_core_kernel(const Data w, bool do_wide, bool do_short, int batch)
+{
+    __shared__ CoreSmem sm;
+    if (gated(w)) return;
+    unsigned long long tri = 0;
+    if (by_pairs(w)) {
+        if (do_short) pair_rows<PV>(w, tri);
+    } else if (has_core<false>(w)) {
+        if (do_wide) core_wide_rows<PV, false>(w, sm, tri);
+        if (do_short)
+            warp_batches(&w.ctr->core_short_next, w.n, batch, [&](long long u0) {
+                core_short_rows<PV, false>(w, u0, batch, tri);
+            });
+    }
+    add_triangles(w.ctr, tri);
+}
+
+template <bool PV, bool BATCH, typename Pos>
+__global__ void __launch_bounds__(kThreads, 5)
+list_kernel(const Data w, bool do_wide, bool do_short, int batch)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    if (gated(w)) return;
+    ListSmem<Pos> &sm = *reinterpret_cast<ListSmem<Pos> *>(smem);
+    unsigned long long tri = 0;
+    if (do_wide && w.ctr->wide_rows > 0) {
+        table_wide_rows<PV, BATCH, Pos>(w, sm, tri);
+        __syncthreads();
+    }
+    if (do_short)
+        list_short_rows<PV, BATCH, Pos>(w, batch, sm.tile[threadIdx.x >> 5], tri,
+                                        [](long long) {});
+    add_triangles(w.ctr, tri);
+}
+
+// Wide rows that a bitmap holds.  A kernel of its own, launched where rows are
+// long (RowConfig::dense): as a part of list_kernel it cost R-MAT 22 0.8% and a
+// ring of 400K with 100 neighbours each 3%, in registers.
+template <bool PV, bool BATCH, typename Pos>
+__global__ void __launch_bounds__(kThreads, 5)
+bitmap_kernel(const Data w)
+{
+    __shared__ BitsSmem sm;
+    if (gated(w)) return;
+    unsigned long long tri = 0;
+    wide_block_rows(
+        w, sm.claim, blockIdx.x, &w.ctr->bitmap_next, PV ? kBitList : kWarpTable,
+        [](const VInfo &vi) { return vi.fdeg > (vi.dk & INT32_MAX); },
+        [&](int v, const VInfo &vi) {
+            const GraphRec *rec = &w.recs[BATCH ? w.gid[v] : 0];
+            if (in_bitmap<PV, BATCH>(w, vi, rec))
+                bits_block_row<PV, BATCH, Pos>(w, v, vi, rec, sm, tri);
+        });
     add_triangles(w.ctr, tri);
 }
 

@@ -29,7 +29,7 @@ struct Data {
     unsigned int *status;
     int word;                       // sizeof(unsigned int)
     const int *gate;                // nullable: while it is 0 the kernels end at once
-    bool bitmaps, pairs;            // bitmap_kernel, pairs_kernel run too
+    bool bitmaps, sparse;           // bitmap_kernel runs too; sparse_core_kernel for core_kernel
 };
 template <typename OffT>
 struct View : Data {

@@ -120,8 +120,7 @@ gtc_status gtc_count_status(const void *d_workspace, size_t ws_bytes,
  *                (5 kernels per count, 6 from 2^18 vertices on); 2 = split
  *                launches: a kernel for long and one for short rows (11); either
  *                way one more for dense graphs of up to 2^17 vertices (mean
- *                degree 128 or more, unless all core) and for sparse ones of 2^18
- *                or more (mean degree of at most 4).
+ *                degree 128 or more, unless all core).
  *                The library splits above mean degree 24 from 2^18 vertices on
  *   rows         2 asks for joint launches too (rejected with labels = 2);
  *                1 leaves the choice to labels
